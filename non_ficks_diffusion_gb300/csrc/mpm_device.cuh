@@ -4,8 +4,8 @@
 // ([field][capacity]): X0..2, V0..2, Fe00..Fe22 (row-major), Jp, m, V0, lambda0, mu0.
 // Two such buffers alternate every substep: the transfer kernel reads particle i of the
 // old buffer through the sort permutation and writes it to slot i of the new one, so the
-// state is always stored in cell order. A per-particle cache of 11 fields (Re, lambda, mu)
-// is written by the same kernel for the CG's Hessian action.
+// state is always stored in cell order. A per-particle cache of the CG's Hessian action
+// (stencil coordinates, left stretch and three coefficients) is written by the same kernel.
 //
 // Grid: 4x4x4 node blocks. Cell (i,j,k) of a scene with counts n is stored at block
 // (b = (i+4)>>2, ...), local (l = (i+4)&3, ...); each scene owns a dense range of
@@ -20,8 +20,11 @@ namespace mpm {
 
 constexpr int NB_FIELDS=20;
 enum { FX=0, FV=3, FF=6, FJP=15, FM=16, FV0=17, FLAM0=18, FMU0=19 };
-constexpr int NC_FIELDS=11;
-enum { CR=0, CLAM=9, CMU=10 };
+// CG cache: V4 vectors per particle ([vector][capacity]), written by P2G in the order of the
+// new buffer and read by every Hessian product: (x0, x1, x2, c1), (Sxx, Sxy, Sxz, Syy),
+// (Syz, Szz, c2, c3) with the stencil coordinates x and the coefficients of HessianData
+// (mpm_math.cuh); FP64 adds the six entries of its K inverse in two more vectors.
+template<class T> __host__ __device__ constexpr int cg_vectors(){return sizeof(T)==8?5:3;}
 constexpr unsigned KEY_SENTINEL=0xFFFFFFFFu;
 constexpr int MAX_BARRIERS=16;
 constexpr int MAX_SCENES=256;
@@ -74,6 +77,13 @@ struct SceneRange { int c0,c1,b0,b1; };
 // scenes' work items and nodes.
 struct ActiveList { int n; int scene[MAX_SCENES]; int cpre[MAX_SCENES+1]; int bpre[MAX_SCENES+1]; };
 
+// Record of a work item, ITEM_WORDS ints, written by P2G for the later transfer kernels: first
+// slot, particles, scene, length of the pair table (FP32), and the active indices of the 27
+// blocks around it (-1: inactive). One 128-byte load replaces a chain of five dependent ones
+// (start, key, scene, bitmap, block map).
+constexpr int ITEM_WORDS=32;
+enum { ITEM_START=0, ITEM_COUNT=1, ITEM_SCENE=2, ITEM_PAIRS=3, ITEM_NBR=4 };
+
 struct Counters {
     unsigned n_valid;          // valid particles after the key pass
     unsigned n_chunks;
@@ -106,12 +116,14 @@ template<class T> struct DevState {
     T* pcur; T* pnxt;               // [NB_FIELDS][pcap]
     int* pid_cur; int* pid_nxt;     // insertion index (global)
     int* scn_cur; int* scn_nxt;     // scene id s, or -(s+1) once removed
-    T* cache;                       // [NC_FIELDS][pcap]
+    V4<T>* cache;                   // [cg_vectors][pcap]
     long long pcap;
     long long n_total;              // particle slots in use (host-known)
     unsigned* keys; int* perm;      // sorted keys and source slots (output of the sort)
     // work items
     int* chunk_start; long long chunk_cap;
+    unsigned* pairs;                // FP32 pair tables, a work item's from its first slot on (see pair_table)
+    int* items;                     // work-item records, written by P2G
     // blocks
     unsigned* bitmap; long long bitmap_words;
     int* blockmap;                  // global block id -> active index (valid where the bitmap bit is set)

@@ -89,18 +89,28 @@ template<class T> struct Stencil {
     int r[3];        // tile coordinate of the particle's cell (1..4)
     T w[3][3],dw[3][3];
 };
-template<class T> __device__ __forceinline__ void make_stencil(const SceneDev<T>& sc,const int* b,unsigned key,const T* X,Stencil<T>& st)
+// Stencil coordinates x = (X - (center(c) - dx))/dx in [0.5, 1.5) of a particle in local cell
+// l of block b, evaluated in the same order as the reference.
+template<class T> __device__ __forceinline__ void stencil_coord(const SceneDev<T>& sc,const int* b,unsigned l,const T* X,T* x)
 {
-    const unsigned l=key&63u;
     const int lc[3]={(int)(l&3u),(int)((l>>2)&3u),(int)(l>>4)};
 #pragma unroll
     for(int a=0;a<3;++a){
-        st.r[a]=lc[a]+1;
         const int cell=4*b[a]+lc[a]-4;
-        // x = (X - (center(c) - dx))/dx, evaluated in the same order as the reference
         const T center=fmul_rn<T>(add_rn<T>((T)cell,(T)0.5),sc.dx[a]);
         const T xe=sub_rn<T>(X[a],sub_rn<T>(center,sc.dx[a]));
-        bspline_weights<T>(fmul_rn<T>(xe,sc.inv_dx[a]),sc.inv_dx[a],st.w[a],st.dw[a]);}
+        x[a]=fmul_rn<T>(xe,sc.inv_dx[a]);}
+}
+template<class T> __device__ __forceinline__ void stencil_from_coord(const SceneDev<T>& sc,unsigned l,const T* x,Stencil<T>& st)
+{
+    st.r[0]=(int)(l&3u)+1;st.r[1]=(int)((l>>2)&3u)+1;st.r[2]=(int)(l>>4)+1;
+#pragma unroll
+    for(int a=0;a<3;++a) bspline_weights<T>(x[a],sc.inv_dx[a],st.w[a],st.dw[a]);
+}
+template<class T> __device__ __forceinline__ void make_stencil(const SceneDev<T>& sc,const int* b,unsigned key,const T* X,Stencil<T>& st)
+{
+    T x[3];stencil_coord(sc,b,key&63u,X,x);
+    stencil_from_coord(sc,key&63u,x,st);
 }
 // Node centre of a grid node.
 template<class T> __device__ __forceinline__ void node_center(const DevState<T>& S,const SceneDev<T>& sc,long long node,int blk,T* x)
@@ -327,53 +337,79 @@ __device__ __forceinline__ void chunk_cell_order(const unsigned* keys,int s,int 
     __syncthreads();
 }
 
-// G[3a+k] = sum_n s_a(n) d_k w(n) over the 27 stencil nodes, for a tile s[3][TILE_N]. The
-// weights are separable, w = wx wy wz: the z sums of wz s_a and dwz s_a come first, then
-// each (x, y) pair adds them with dwx wy, wx dwy and wx wy.
-// FP32: components 0 and 1 of the staged vector as packed pairs, component 2 scalar.
-__device__ __forceinline__ void gather_grad(const Stencil<float>& st,const float (*s)[TILE_S],float* G)
+// A vector over the three components of a node value. FP32 holds components 0 and 1 as a
+// packed pair (one instruction for two fused multiply-adds, each rounded like fmaf).
+template<class T> struct C3 { T x,y,z; };
+template<> struct C3<float> { float2 xy; float z; };
+template<class T> __device__ __forceinline__ C3<T> c3(T x,T y,T z){return C3<T>{x,y,z};}
+template<> __device__ __forceinline__ C3<float> c3<float>(float x,float y,float z){return C3<float>{make_float2(x,y),z};}
+__device__ __forceinline__ C3<float> madd(const C3<float>& a,float s,const C3<float>& c){return C3<float>{pfma(a.xy,pdup(s),c.xy),fmaf(a.z,s,c.z)};}
+__device__ __forceinline__ C3<double> madd(const C3<double>& a,double s,const C3<double>& c){return C3<double>{fma(a.x,s,c.x),fma(a.y,s,c.y),fma(a.z,s,c.z)};}
+__device__ __forceinline__ C3<float> mul(const C3<float>& a,float s){return C3<float>{pmul(a.xy,pdup(s)),a.z*s};}
+__device__ __forceinline__ C3<double> mul(const C3<double>& a,double s){return C3<double>{a.x*s,a.y*s,a.z*s};}
+__device__ __forceinline__ float cx(const C3<float>& a){return a.xy.x;}
+__device__ __forceinline__ float cy(const C3<float>& a){return a.xy.y;}
+__device__ __forceinline__ double cx(const C3<double>& a){return a.x;}
+__device__ __forceinline__ double cy(const C3<double>& a){return a.y;}
+
+// Pair table of a work item, for the kernels that handle two particles of one cell per lane.
+// The particles of a cell are paired in slot order (an odd one stays alone); the pairs are
+// listed level by level, the first pairs of all cells, then the second ones, and so on, the
+// cells of a level with even scatter rank before those with odd rank. 32 consecutive
+// pairs, one warp's pass, therefore lie in distinct cells whose tile addresses fall in
+// distinct banks wherever a level has enough cells. Entry: positions of the two
+// particles in the item (12 bits each), cell (6 bits), PAIR_TWO when there is a second one.
+constexpr unsigned PAIR_TWO=1u<<30;
+__device__ __forceinline__ unsigned pair_entry(int k,bool two,unsigned cell,int stride,const int* run)
 {
-    float2 g03=make_float2(0.f,0.f),g14=g03,g25=g03;
-    float g6=0.f,g7=0.f,g8=0.f;
-    const int tb=tile_addr(st.r[0]-1,st.r[1]-1,st.r[2]-1);
-#pragma unroll
-    for(int ox=0;ox<3;++ox)
-#pragma unroll
-    for(int oy=0;oy<3;++oy){
-        float2 t01=make_float2(0.f,0.f),u01=t01;
-        float t2=0.f,u2=0.f;
-#pragma unroll
-        for(int oz=0;oz<3;++oz){
-            const float wz=st.w[2][oz],dz=st.dw[2][oz];
-            const int n=tb+tile_addr(ox,oy,oz);
-            const float2 s01=make_float2(s[0][n],s[1][n]);
-            const float s2=s[2][n];
-            t01=pfma(pdup(wz),s01,t01);u01=pfma(pdup(dz),s01,u01);
-            t2=fmaf(wz,s2,t2);u2=fmaf(dz,s2,u2);}
-        const float dxy=st.dw[0][ox]*st.w[1][oy],xdy=st.w[0][ox]*st.dw[1][oy],wxy=st.w[0][ox]*st.w[1][oy];
-        g03=pfma(pdup(dxy),t01,g03);g14=pfma(pdup(xdy),t01,g14);g25=pfma(pdup(wxy),u01,g25);
-        g6=fmaf(dxy,t2,g6);g7=fmaf(xdy,t2,g7);g8=fmaf(wxy,u2,g8);}
-    G[0]=g03.x;G[3]=g03.y;G[1]=g14.x;G[4]=g14.y;G[2]=g25.x;G[5]=g25.y;G[6]=g6;G[7]=g7;G[8]=g8;
+    const int L0=k/stride,p0=run[k-L0*stride]+L0;
+    int p1=p0;
+    if(two){const int L1=(k+1)/stride;p1=run[k+1-L1*stride]+L1;}
+    return (unsigned)p0|((unsigned)p1<<12)|(cell<<24)|(two?PAIR_TWO:0u);
 }
-template<class T> __device__ __forceinline__ void gather_grad(const Stencil<T>& st,const T (*s)[TILE_S],T* G)
+// Written by one warp; rank_end[r] is the end of scatter rank r in the item's slot order and
+// cell_of[r] its cell. Returns the number of pairs.
+__device__ __forceinline__ int pair_table(const int* rank_end,const unsigned char* cell_of,int stride,const int* run,unsigned* out)
+{
+    const int lane=threadIdx.x&31;
+    const int e0=rank_end[2*lane],e1=rank_end[2*lane+1];
+    int s0=__shfl_up_sync(0xffffffffu,e1,1);
+    if(lane==0) s0=0;
+    const unsigned below=lane_bits_below();
+    const unsigned c0=cell_of[2*lane],c1=cell_of[2*lane+1];
+    int base=0;
+    for(int j=0;;++j){
+        const int k0=s0+2*j,k1=e0+2*j;
+        const unsigned m0=__ballot_sync(0xffffffffu,k0<e0),m1=__ballot_sync(0xffffffffu,k1<e1);
+        if((m0|m1)==0u) break;
+        if(k0<e0) out[base+__popc(m0&below)]=pair_entry(k0,k0+1<e0,c0,stride,run);
+        base+=__popc(m0);
+        if(k1<e1) out[base+__popc(m1&below)]=pair_entry(k1,k1+1<e1,c1,stride,run);
+        base+=__popc(m1);}
+    return base;
+}
+
+// G[k] = sum_n s(n) d_k w(n) over the 27 stencil nodes, for a tile s[3][TILE_S]. The weights
+// are separable, w = wx wy wz: the z sums of wz s and dwz s come first, then each (x, y)
+// pair adds them with dwx wy, wx dwy and wx wy.
+template<class T> __device__ __forceinline__ void gather_grad(const Stencil<T>& st,const T (*s)[TILE_S],C3<T> (&G)[3])
 {
 #pragma unroll
-    for(int k=0;k<9;++k) G[k]=T(0);
+    for(int k=0;k<3;++k) G[k]=c3<T>(T(0),T(0),T(0));
     const int tb=tile_addr(st.r[0]-1,st.r[1]-1,st.r[2]-1);
 #pragma unroll
     for(int ox=0;ox<3;++ox)
 #pragma unroll
     for(int oy=0;oy<3;++oy){
-        T t[3]={T(0),T(0),T(0)},u[3]={T(0),T(0),T(0)};
+        C3<T> t,u;
 #pragma unroll
         for(int oz=0;oz<3;++oz){
-            const T wz=st.w[2][oz],dz=st.dw[2][oz];
             const int n=tb+tile_addr(ox,oy,oz);
-#pragma unroll
-            for(int a=0;a<3;++a){const T sa=s[a][n];t[a]+=wz*sa;u[a]+=dz*sa;}}
+            const C3<T> v=c3<T>(s[0][n],s[1][n],s[2][n]);
+            t=oz==0?mul(v,st.w[2][oz]):madd(v,st.w[2][oz],t);
+            u=oz==0?mul(v,st.dw[2][oz]):madd(v,st.dw[2][oz],u);}
         const T dxy=st.dw[0][ox]*st.w[1][oy],xdy=st.w[0][ox]*st.dw[1][oy],wxy=st.w[0][ox]*st.w[1][oy];
-#pragma unroll
-        for(int a=0;a<3;++a){G[3*a]+=dxy*t[a];G[3*a+1]+=xdy*t[a];G[3*a+2]+=wxy*u[a];}}
+        G[0]=madd(t,dxy,G[0]);G[1]=madd(t,xdy,G[1]);G[2]=madd(u,wxy,G[2]);}
 }
 
 // Conflict-free rounds for a warp's scatter into its private tile. Lanes whose particles
@@ -427,9 +463,8 @@ template<class P> __device__ __forceinline__ void p2g_pass(const DevState<typena
         T R[9],lam,mu,Je;
         if(sc.eos){
             // EOS fluid (MPM_Example.cpp:737-738): no constitutive update; the
-            // density is the Jp slot. The CG's coefficient V0 k gamma rho^(gamma-1)
-            // goes to the lambda cache slot, the explicit one V0/rho k rho^(gamma-1)
-            // to the mu slot.
+            // density is the Jp slot. lam: the CG's coefficient V0 k gamma rho^(gamma-1);
+            // mu: the explicit one V0/rho k rho^(gamma-1).
             const T pw=tpow(Jp,sc.eos_gamma-T(1));
             lam=V0*sc.bulk*sc.eos_gamma*pw;mu=V0/Jp*sc.bulk*pw;Je=T(1);
 #pragma unroll
@@ -438,15 +473,17 @@ template<class P> __device__ __forceinline__ void p2g_pass(const DevState<typena
 #pragma unroll
         for(int a=0;a<3;++a){Pout[(FX+a)*pc+i]=X[a];Pout[(FV+a)*pc+i]=V[a];}
 #pragma unroll
-        for(int k=0;k<9;++k){Pout[(FF+k)*pc+i]=F[k];S.cache[(CR+k)*pc+i]=R[k];}
+        for(int k=0;k<9;++k) Pout[(FF+k)*pc+i]=F[k];
         Pout[FJP*pc+i]=Jp;Pout[FM*pc+i]=m;Pout[FV0*pc+i]=V0;Pout[FLAM0*pc+i]=lam0;Pout[FMU0*pc+i]=mu0;
-        S.cache[CLAM*pc+i]=lam;S.cache[CMU*pc+i]=mu;
         S.pid_nxt[i]=S.pid_cur[src];S.scn_nxt[i]=S.scn_cur[src];
+        HessianData<T> h;
         if(sc.eos){
             // f += coefficient grad w, i.e. A = -coefficient I
 #pragma unroll
-            for(int k=0;k<9;++k) A[k]=(k%4==0)?-mu:T(0);}
+            for(int k=0;k<9;++k) A[k]=(k%4==0)?-mu:T(0);
+            h=HessianData<T>{{T(1),T(0),T(0),T(1),T(0),T(1)},T(0),lam,T(0)};}
         else{
+            hessian_data(F,R,lam,mu,Je,V0,h);
             // V0 P Fe^T
             T Pk[9];stress_P(F,R,lam,mu,Je,Pk);mat_mul_bt(Pk,F,A);
 #pragma unroll
@@ -454,7 +491,15 @@ template<class P> __device__ __forceinline__ void p2g_pass(const DevState<typena
         cell=cellv[jj];
         const unsigned key=((unsigned)ci.gb<<6)|cell;
         S.keys[i]=key;
-        make_stencil(sc,ci.b,key,X,st);}
+        T x[3];stencil_coord(sc,ci.b,cell,X,x);
+        stencil_from_coord(sc,cell,x,st);
+        S.cache[i]=V4<T>{x[0],x[1],x[2],h.c1};
+        S.cache[pc+i]=V4<T>{h.S[0],h.S[1],h.S[2],h.S[3]};
+        S.cache[2*pc+i]=V4<T>{h.S[4],h.S[5],h.c2,h.c3};
+        if constexpr(sizeof(T)==8){
+            T Ki[6];skew_system_inverse(h.S,Ki);
+            S.cache[3*pc+i]=V4<T>{Ki[0],Ki[1],Ki[2],Ki[3]};
+            S.cache[4*pc+i]=V4<T>{Ki[4],Ki[5],T(0),T(0)};}}
     const ScatterRounds R(valid,cell);
     for(int r=0;r<R.rounds;++r){
         const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
@@ -536,8 +581,10 @@ template<class P,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) 
     int (*ocnt)[64]=reinterpret_cast<int (*)[64]>(smem_raw+p2g_tile_bytes<T>());
     unsigned short* inv=reinterpret_cast<unsigned short*>(smem_raw+p2g_tile_bytes<T>()+NW*64*4);
     unsigned char* cellv=reinterpret_cast<unsigned char*>(inv+S.chunk);
-    __shared__ unsigned char crank[64];
-    if(threadIdx.x<64) crank[threadIdx.x]=cell_rank_of(threadIdx.x);   // read after the next barrier
+    __shared__ unsigned char crank[64],cell_of[64];
+    if(threadIdx.x<64){                                                // read after the next barrier
+        const unsigned char r=cell_rank_of(threadIdx.x);
+        crank[threadIdx.x]=r;cell_of[r]=(unsigned char)threadIdx.x;}
     __shared__ int nbr[27];
     __shared__ int run[129];
     const int warp=threadIdx.x>>5;
@@ -546,10 +593,24 @@ template<class P,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) 
         ChunkInfo<T> ci;
         load_chunk(S,c,nc,nv,ci,nbr);
         const int np=ci.e-ci.s,stride=(np+31)>>5;
-        if(np>S.chunk){if(threadIdx.x==0) atomicOr(&S.ctr->error,ERR_CAPACITY);continue;}   // uniform
+        // a work item longer than `chunk` only arises when the work-item capacity was exceeded;
+        // an empty record keeps the later kernels off it
+        const bool over=np>S.chunk;
+        if(warp==0){
+            __syncwarp();                              // nbr was written by this warp
+            const int lane=threadIdx.x&31;
+            if(lane<ITEM_PAIRS||(lane==ITEM_PAIRS&&over)||lane>=ITEM_NBR)
+                S.items[c*ITEM_WORDS+lane]=lane==ITEM_START?ci.s:lane==ITEM_COUNT?(over?0:np):lane==ITEM_SCENE?ci.scene:
+                                           lane==ITEM_PAIRS?0:lane-ITEM_NBR<27?nbr[lane-ITEM_NBR]:-1;}
+        if(over){if(threadIdx.x==0) atomicOr(&S.ctr->error,ERR_CAPACITY);continue;}   // uniform
         if(warp==0) chunk_runs(np,stride,run);        // read after the barriers in chunk_cell_order
         for(int t=threadIdx.x;t<NW*7*TILE_S;t+=blockDim.x) (&acc[0][0][0])[t]=T(0);
         chunk_cell_order(S.keys,ci.s,np,crank,ocnt,inv,cellv);
+        // the last warp has the fewest passes; its counts now hold the ends of the ranks
+        if constexpr(sizeof(T)==4){
+            if(warp==NW-1){
+                const int m=pair_table(ocnt[NW-1],cell_of,stride,run,S.pairs+ci.s);
+                if((threadIdx.x&31)==0) S.items[c*ITEM_WORDS+ITEM_PAIRS]=m;}}
         const SceneDev<T>& sc=S.scenes[ci.scene];
         for(int qi=warp;qi<stride;qi+=NW) p2g_pass<P>(S,sc,ci,run,inv,cellv,qi,stride,np,acc[warp]);
         __syncthreads();
@@ -724,63 +785,50 @@ template<class T> __global__ void __launch_bounds__(NODE_THREADS) k_grid_update(
 // (V0 Fe dP^T)^T grad w_i. The gathered vector is x (FROM_X, for r = b - A x) or the new
 // search direction s = r + beta s_old, formed on the fly from r and the old s.
 // =====================================================================================
-// One pass of a work item's particles through the Hessian product: pass qi gives lane L the
-// cell-ordered particle L*stride + qi (stored by P2G at position run[qi] + L). It gathers
-// G = sum_n s(n) grad w(n)^T from the staged vector tile sv, forms
-// A = V0 Fe dP(dF = G Fe)^T, and scatters A^T grad w into the warp's private tile in rounds
-// of lanes in distinct cells. Called by every lane of the warp.
-// Requests into L2 the fields the Hessian reads for particle position i (its pass runs
-// next), so that those loads wait on L2 rather than on DRAM.
-template<class T> __device__ __forceinline__ void prefetch_hessian_particle(const DevState<T>& S,int i)
+// B = V0 dP Fe^T from G, by columns (HessianData in mpm_math.cuh). FP32 solves the 3x3 system
+// of the rotation part here; FP64, whose arithmetic is 64 times slower against the same
+// memory, reads the inverse that P2G stored.
+template<class T> __device__ __forceinline__ void hessian_stress(const C3<T> (&G)[3],const T* Sm,T c1,T c2,T cc3,const T* Ki,C3<T> (&B)[3])
 {
-    const long long pc=S.pcap;
-    auto pf=[](const void* p){asm volatile("prefetch.global.L2 [%0];"::"l"(p));};
+    const T S[3][3]={{Sm[0],Sm[1],Sm[2]},{Sm[1],Sm[3],Sm[4]},{Sm[2],Sm[4],Sm[5]}};
+    C3<T> M[3];
 #pragma unroll
-    for(int a=0;a<3;++a) pf(S.pcur+(FX+a)*pc+i);
+    for(int j=0;j<3;++j) M[j]=madd(G[2],S[2][j],madd(G[1],S[1][j],mul(G[0],S[0][j])));
+    const T L0=cy(M[0])-cx(M[1]),L1=M[0].z-cx(M[2]),L2=M[1].z-cy(M[2]);
+    const T a=Ki[0]*L0+Ki[1]*L1+Ki[2]*L2,b=Ki[1]*L0+Ki[3]*L1+Ki[4]*L2,c=Ki[2]*L0+Ki[4]*L1+Ki[5]*L2;
+    const C3<T> N[3]={c3<T>(cx(M[0]),cy(M[0])-a,M[0].z-b),c3<T>(cx(M[1])+a,cy(M[1]),M[1].z-c),c3<T>(cx(M[2])+b,cy(M[2])+c,M[2].z)};
+    const T tr=c2*(cx(G[0])+cy(G[1])+G[2].z);
+    // columns j of -c3 G^T (rows j of G), then c1 N S and the trace on the diagonal
+    const C3<T> gt[3]={c3<T>(cx(G[0]),cx(G[1]),cx(G[2])),c3<T>(cy(G[0]),cy(G[1]),cy(G[2])),c3<T>(G[0].z,G[1].z,G[2].z)};
 #pragma unroll
-    for(int k=0;k<9;++k){pf(S.pcur+(FF+k)*pc+i);pf(S.cache+(CR+k)*pc+i);}
-    pf(S.pcur+FV0*pc+i);pf(S.cache+CLAM*pc+i);pf(S.cache+CMU*pc+i);pf(S.keys+i);
+    for(int j=0;j<3;++j)
+        B[j]=madd(N[2],c1*S[2][j],madd(N[1],c1*S[1][j],madd(N[0],c1*S[0][j],mul(gt[j],-cc3))));
+    B[0]=c3<T>(cx(B[0])+tr,cy(B[0]),B[0].z);B[1]=c3<T>(cx(B[1]),cy(B[1])+tr,B[1].z);B[2]=c3<T>(cx(B[2]),cy(B[2]),B[2].z+tr);
 }
-template<class P> __device__ __forceinline__ void hessian_pass(const DevState<typename P::T>& S,const SceneDev<typename P::T>& sc,
-    const ChunkInfo<typename P::T>& ci,const int* run,int qi,int stride,int np,const typename P::T (*sv)[TILE_S],
-    typename P::T (*tile)[TILE_S],int qn=-1)
+
+// FP64: one pass of a work item gives lane L the cell-ordered particle L*stride + qi (stored
+// by P2G at position run[qi] + L). It gathers G = sum_n s(n) grad w(n)^T from the staged
+// vector tile sv, forms B and scatters B grad w into the warp's private tile in rounds of
+// lanes in distinct cells. Called by every lane of the warp.
+__device__ __forceinline__ void hessian_pass(const DevState<double>& S,const SceneDev<double>& sc,int s,const int* run,int qi,int stride,int np,
+    const double (*sv)[TILE_S],double (*tile)[TILE_S])
 {
-    using T=typename P::T;
+    using T=double;
     const int j=(int)(threadIdx.x&31)*stride+qi;
     const bool valid=j<np;
-    const int i=ci.s+run[qi]+(int)(threadIdx.x&31);   // the position P2G stored slot j at
-    if(qn>=0&&(int)(threadIdx.x&31)*stride+qn<np) prefetch_hessian_particle(S,ci.s+run[qn]+(int)(threadIdx.x&31));
-    T A[9];
+    const int i=s+run[qi]+(int)(threadIdx.x&31);
+    C3<T> B[3];
     Stencil<T> st;
     unsigned cell=0;
     if(valid){
         const long long pc=S.pcap;
-        T X[3];
-#pragma unroll
-        for(int a=0;a<3;++a) X[a]=S.pcur[(FX+a)*pc+i];
-        const unsigned key=S.keys[i];
-        make_stencil(sc,ci.b,key,X,st);
-        cell=key&63u;
-        // G[3a+k] = sum_n s_a grad_k w_n, contracted over z first (separable weights)
-        T G[9];
+        const V4<T> q0=S.cache[i],q1=S.cache[pc+i],q2=S.cache[2*pc+i],q3=S.cache[3*pc+i],q4=S.cache[4*pc+i];
+        cell=S.keys[i]&63u;
+        const T Sm[6]={q1.x,q1.y,q1.z,q1.w,q2.x,q2.y},Ki[6]={q3.x,q3.y,q3.z,q3.w,q4.x,q4.y},x[3]={q0.x,q0.y,q0.z};
+        stencil_from_coord(sc,cell,x,st);
+        C3<T> G[3];
         gather_grad(st,sv,G);
-        if(sc.eos){
-            // EOS fluid (MPM_CG_System.h:102-107, 138-140): coefficient times
-            // sum_i grad w_i . s_i on the diagonal, scattered as eos_scp grad w
-            const T e=S.cache[CLAM*pc+i]*(G[0]+G[4]+G[8]);
-#pragma unroll
-            for(int k=0;k<9;++k) A[k]=(k%4==0)?e:T(0);}
-        else{
-            T F[9],Rm[9];
-#pragma unroll
-            for(int k=0;k<9;++k){F[k]=S.pcur[(FF+k)*pc+i];Rm[k]=S.cache[(CR+k)*pc+i];}
-            const T lam=S.cache[CLAM*pc+i],mu=S.cache[CMU*pc+i],V0=S.pcur[FV0*pc+i];
-            T dF[9],dP[9];
-            mat_mul(G,F,dF);
-            dP_dF(F,Rm,lam,mu,dF,dP);
-            mat_mul_bt(F,dP,A);        // Fe dP^T
-#pragma unroll
-            for(int k=0;k<9;++k) A[k]*=V0;}}
+        hessian_stress<T>(G,Sm,q0.w,q2.z,q2.w,Ki,B);}
     const ScatterRounds R(valid,cell);
     for(int r=0;r<R.rounds;++r){
         const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
@@ -790,35 +838,115 @@ template<class P> __device__ __forceinline__ void hessian_pass(const DevState<ty
             for(int ox=0;ox<3;++ox)
 #pragma unroll
             for(int oy=0;oy<3;++oy){
-                // q_a = sum_k A[3k+a] grad_k w = al_a wz + be_a dwz at this (x, y)
-                const T dxy=st.dw[0][ox]*st.w[1][oy],xdy=st.w[0][ox]*st.dw[1][oy],wxy=st.w[0][ox]*st.w[1][oy];
-                if constexpr(sizeof(T)==4){
-                    // channels 0 and 1 as packed pairs, channel 2 scalar
-                    const float2 al01=pfma(make_float2(A[0],A[1]),pdup(dxy),pmul(make_float2(A[3],A[4]),pdup(xdy)));
-                    const float2 be01=pmul(make_float2(A[6],A[7]),pdup(wxy));
-                    const T al2=tfma(A[2],dxy,A[5]*xdy),be2=A[8]*wxy;
+                // q = sum_k B_k grad_k w = al wz + be dwz at this (x, y)
+                const C3<T> al=madd(B[1],st.w[0][ox]*st.dw[1][oy],mul(B[0],st.dw[0][ox]*st.w[1][oy]));
+                const C3<T> be=mul(B[2],st.w[0][ox]*st.w[1][oy]);
 #pragma unroll
-                    for(int oz=0;oz<3;++oz){
-                        const T wz=st.w[2][oz],dz=st.dw[2][oz];
-                        const int t=tb+tile_addr(ox,oy,oz);
-                        float2 q01=make_float2(tile[0][t],tile[1][t]);
-                        q01=pfma(be01,pdup(dz),pfma(al01,pdup(wz),q01));
-                        tile[0][t]=q01.x;tile[1][t]=q01.y;
-                        tile[2][t]=tfma(be2,dz,tfma(al2,wz,tile[2][t]));
-                        __syncwarp(rmask);}}
-                else{
-                    const T al0=A[0]*dxy+A[3]*xdy,al1=A[1]*dxy+A[4]*xdy,al2=A[2]*dxy+A[5]*xdy;
-                    const T be0=A[6]*wxy,be1=A[7]*wxy,be2=A[8]*wxy;
-#pragma unroll
-                    for(int oz=0;oz<3;++oz){
-                        const T wz=st.w[2][oz],dz=st.dw[2][oz];
-                        const int t=tb+tile_addr(ox,oy,oz);
-                        // two fused multiply-adds per channel: tile + al wz + be dz
-                        tile[0][t]=tfma(be0,dz,tfma(al0,wz,tile[0][t]));
-                        tile[1][t]=tfma(be1,dz,tfma(al1,wz,tile[1][t]));
-                        tile[2][t]=tfma(be2,dz,tfma(al2,wz,tile[2][t]));
-                        __syncwarp(rmask);}}}}
+                for(int oz=0;oz<3;++oz){
+                    const int t=tb+tile_addr(ox,oy,oz);
+                    const C3<T> q=madd(be,st.dw[2][oz],madd(al,st.w[2][oz],c3<T>(tile[0][t],tile[1][t],tile[2][t])));
+                    tile[0][t]=cx(q);tile[1][t]=cy(q);tile[2][t]=q.z;
+                    __syncwarp(rmask);}}}
         __syncwarp();}
+}
+
+// FP32: two particles of one cell per lane (the pair table). The 81 node values of the cell's
+// stencil are read once for both, and both particles' forces are added to the tile in one
+// read and one write per node. The particles' vectors arrive in shared memory by
+// asynchronous copies issued one pass ahead (slots[k][lane], read only by the lane that
+// copied them), so that no load latency is left in a pass and the coefficients take no
+// registers during the gather.
+__device__ __forceinline__ void copy_pair(const DevState<float>& S,int s,unsigned entry,V4<float> (*slots)[32])
+{
+    const int lane=threadIdx.x&31;
+#pragma unroll
+    for(int h=0;h<2;++h){
+        const V4<float>* p=S.cache+s+((entry>>(12*h))&4095u);
+#pragma unroll
+        for(int k=0;k<3;++k){
+            const unsigned d=(unsigned)__cvta_generic_to_shared(&slots[3*h+k][lane]);
+            asm volatile("cp.async.cg.shared.global [%0],[%1],16;"::"r"(d),"l"(p+k*S.pcap):"memory");}}
+}
+// The passes m0, m0 + dm, ... (pair index of the pass's first lane) of a work item of M pairs.
+__device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const SceneDev<float>& sc,int s,int M,int m0,int dm,
+    const float (*sv)[TILE_S],float (*tile)[TILE_S],V4<float> (*slots)[32])
+{
+    constexpr int NP=2;
+    const unsigned* tab=S.pairs+s;
+    const int lane=threadIdx.x&31;
+    unsigned entry=0,next=0;
+    if(m0+lane<M){entry=tab[m0+lane];copy_pair(S,s,entry,slots);}
+    if(m0+dm+lane<M) next=tab[m0+dm+lane];
+    for(int m=m0;m<M;m+=dm){
+        const bool valid=m+lane<M;
+        const unsigned cell=(entry>>24)&63u;
+        C3<float> B[NP][3];
+        Stencil<float> st[NP];
+        int tb=0;
+        asm volatile("cp.async.wait_all;":::"memory");
+        if(valid){
+#pragma unroll
+            for(int h=0;h<NP;++h){
+                const V4<float> q0=slots[3*h][lane];
+                const float x[3]={q0.x,q0.y,q0.z};
+                stencil_from_coord(sc,cell,x,st[h]);}
+            tb=tile_addr(st[0].r[0]-1,st[0].r[1]-1,st[0].r[2]-1);
+            C3<float> G[NP][3];
+#pragma unroll
+            for(int h=0;h<NP;++h)
+#pragma unroll
+                for(int k=0;k<3;++k) G[h][k]=c3<float>(0.f,0.f,0.f);
+#pragma unroll
+            for(int ox=0;ox<3;++ox)
+#pragma unroll
+            for(int oy=0;oy<3;++oy){
+                C3<float> t[NP],u[NP];
+#pragma unroll
+                for(int oz=0;oz<3;++oz){
+                    const int n=tb+tile_addr(ox,oy,oz);
+                    const C3<float> v=c3<float>(sv[0][n],sv[1][n],sv[2][n]);
+#pragma unroll
+                    for(int h=0;h<NP;++h){
+                        t[h]=oz==0?mul(v,st[h].w[2][oz]):madd(v,st[h].w[2][oz],t[h]);
+                        u[h]=oz==0?mul(v,st[h].dw[2][oz]):madd(v,st[h].dw[2][oz],u[h]);}}
+#pragma unroll
+                for(int h=0;h<NP;++h){
+                    G[h][0]=madd(t[h],st[h].dw[0][ox]*st[h].w[1][oy],G[h][0]);
+                    G[h][1]=madd(t[h],st[h].w[0][ox]*st[h].dw[1][oy],G[h][1]);
+                    G[h][2]=madd(u[h],st[h].w[0][ox]*st[h].w[1][oy],G[h][2]);}}
+#pragma unroll
+            for(int h=0;h<NP;++h){
+                const V4<float> q0=slots[3*h][lane],q1=slots[3*h+1][lane],q2=slots[3*h+2][lane];
+                const float Sm[6]={q1.x,q1.y,q1.z,q1.w,q2.x,q2.y};
+                const float on=h==0||(entry&PAIR_TWO)?1.f:0.f;      // no second particle: no force
+                float Ki[6];skew_system_inverse(Sm,Ki);
+                hessian_stress<float>(G[h],Sm,on*q0.w,on*q2.z,on*q2.w,Ki,B[h]);}}
+        entry=next;
+        if(m+dm+lane<M) copy_pair(S,s,entry,slots);
+        if(m+2*dm+lane<M) next=tab[m+2*dm+lane];
+        const ScatterRounds R(valid,cell);
+        for(int r=0;r<R.rounds;++r){
+            const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
+            if(valid&&R.rank==r){
+#pragma unroll
+                for(int ox=0;ox<3;++ox)
+#pragma unroll
+                for(int oy=0;oy<3;++oy){
+                    C3<float> al[NP],be[NP];
+#pragma unroll
+                    for(int h=0;h<NP;++h){
+                        al[h]=madd(B[h][1],st[h].w[0][ox]*st[h].dw[1][oy],mul(B[h][0],st[h].dw[0][ox]*st[h].w[1][oy]));
+                        be[h]=mul(B[h][2],st[h].w[0][ox]*st[h].w[1][oy]);}
+#pragma unroll
+                    for(int oz=0;oz<3;++oz){
+                        const int t=tb+tile_addr(ox,oy,oz);
+                        C3<float> v=c3<float>(tile[0][t],tile[1][t],tile[2][t]);
+#pragma unroll
+                        for(int h=0;h<NP;++h) v=madd(be[h],st[h].dw[2][oz],madd(al[h],st[h].w[2][oz],v));
+                        tile[0][t]=cx(v);tile[1][t]=cy(v);tile[2][t]=v.z;
+                        __syncwarp(rmask);}}}
+            __syncwarp();}
+    }
 }
 
 // The Hessian's two ways of taking work items, one kernel (the form is a launch argument,
@@ -836,19 +964,43 @@ template<class P> __device__ __forceinline__ void hessian_pass(const DevState<ty
 //   occupancy variant), else a CTA per item (the count is known on the device: all items
 //   for the first product, the iterating scenes' items for a loop trip).
 constexpr int HESS_CTA=0, HESS_WARP=1, HESS_AUTO=2;
-template<class T> constexpr int hess_kernel_smem_bytes(){return hess_smem_bytes<T>()>hess_warp_smem_bytes<T>()?hess_smem_bytes<T>():hess_warp_smem_bytes<T>();}
-template<class P,bool FROM_X> __device__ __forceinline__ void stage_vector(const DevState<typename P::T>& S,const int* nbr,typename P::T beta,
-    typename P::T (*sv)[TILE_S],int t0,int dt)
+// Shared memory of one warp: accumulated tile, staged tile and, in FP32, the copied pairs.
+template<class T> __host__ __device__ constexpr int hess_warp_bytes(){return 6*TILE_S*(int)sizeof(T)+(sizeof(T)==4?6*32*16:0);}
+template<class T> constexpr int hess_kernel_smem_bytes(){return (XFER_THREADS/32)*hess_warp_bytes<T>();}
+// Tile node t packed as neighbour index (5 bits), local node (6 bits), tile address.
+__device__ __forceinline__ unsigned tile_map_entry(int t)
+{
+    const int tx=t%TILE,ty=(t/TILE)%TILE,tz=t/(TILE*TILE);
+    const int idx=(tx+3)/4+3*((ty+3)/4)+9*((tz+3)/4),l=((tx+3)&3)|(((ty+3)&3)<<2)|(((tz+3)&3)<<4);
+    return (unsigned)idx|((unsigned)l<<5)|((unsigned)tile_addr(t)<<11);
+}
+// The gathered vector at the item's tile nodes, by NT threads: the loads of a batch of nodes
+// are all issued before one is used (a node's address needs only the item record).
+template<class P,bool FROM_X,int NT> __device__ __forceinline__ void stage_vector(const DevState<typename P::T>& S,const int* nbr,const unsigned* tmap,
+    typename P::T beta,typename P::T (*sv)[TILE_S],int tid)
 {
     using T=typename P::T;
-    for(int t=t0;t<TILE_N;t+=dt){
-        const long long node=tile_node(nbr,t);
-        T a=T(0),b=T(0),d=T(0);
-        if(node>=0){
-            if(FROM_X){const V4<T> x=S.gx[node];a=x.x;b=x.y;d=x.z;}
-            else{const V4<T> r=S.gr[node],so=S.gs[node];a=r.x+beta*so.x;b=r.y+beta*so.y;d=r.z+beta*so.z;}}
-        const int ta=tile_addr(t);
-        sv[0][ta]=a;sv[1][ta]=b;sv[2][ta]=d;}
+    constexpr int IT=(TILE_N+NT-1)/NT,BATCH=sizeof(T)==8?1:IT;
+#pragma unroll
+    for(int i0=0;i0<IT;i0+=BATCH){
+        V4<T> a[BATCH],b[BATCH];unsigned ta[BATCH];
+#pragma unroll
+        for(int i=0;i<BATCH;++i){
+            const int t=tid+(i0+i)*NT;
+            a[i]=b[i]=V4<T>{T(0),T(0),T(0),T(0)};ta[i]=~0u;
+            if(t<TILE_N){
+                const unsigned e=tmap[t];
+                ta[i]=e>>11;
+                const int blk=nbr[e&31u];
+                if(blk>=0){
+                    const long long node=(long long)blk*64+((e>>5)&63u);
+                    if(FROM_X) a[i]=S.gx[node];
+                    else{a[i]=S.gr[node];b[i]=S.gs[node];}}}}
+#pragma unroll
+        for(int i=0;i<BATCH;++i) if(ta[i]!=~0u){
+            sv[0][ta[i]]=FROM_X?a[i].x:a[i].x+beta*b[i].x;
+            sv[1][ta[i]]=FROM_X?a[i].y:a[i].y+beta*b[i].y;
+            sv[2][ta[i]]=FROM_X?a[i].z:a[i].z+beta*b[i].z;}}
 }
 template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) k_hessian(DevState<typename P::T> S,int form,long long warp_min)
 {
@@ -856,79 +1008,83 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
     using T=typename P::T;
     constexpr int NW=XFER_THREADS/32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ int nbr_s[NW][27];
-    __shared__ int run_s[NW][129];
+    __shared__ int rec_s[NW][ITEM_WORDS];
+    __shared__ int run_s[sizeof(T)==8?NW:1][129];
+    __shared__ unsigned tmap[TILE_N];
     __shared__ ListSmem lsm;
     const int warp=threadIdx.x>>5,lane=threadIdx.x&31;
-    const unsigned nc=min(S.ctr->n_chunks,(unsigned)S.chunk_cap),nv=S.ctr->n_valid;
+    const unsigned nc=min(S.ctr->n_chunks,(unsigned)S.chunk_cap);
+    auto tile_of=[&](int w){return reinterpret_cast<T (*)[TILE_S]>(smem_raw+w*hess_warp_bytes<T>());};   // [component][node]
+    T (*q)[TILE_S]=tile_of(warp);                  // accumulated
+    V4<float> (*slots)[32]=reinterpret_cast<V4<float> (*)[32]>(smem_raw+warp*hess_warp_bytes<T>()+6*TILE_S*sizeof(T));
+    for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x) tmap[t]=tile_map_entry(t);
+    for(int t=lane;t<3*TILE_S;t+=32) (&q[0][0])[t]=T(0);
     // the first product (FROM_X) covers every work item; a loop trip only the work items of
     // the scenes still iterating (the list the previous convergence check wrote)
     long long nwork=nc;
     if(!FROM_X){load_active_list(S.alist,lsm,false);nwork=lsm.pre[lsm.n];}
+    __syncthreads();
     auto item=[&](long long w){
         if(FROM_X) return w;
         const int j=list_find(lsm,(int)w);return S.srange[lsm.scene[j]].c0+(w-lsm.pre[j]);};
     if(form==HESS_AUTO) form=nwork>=warp_min?HESS_WARP:HESS_CTA;
+    // the passes of an item: pairs (FP32) or cell-ordered particles (FP64), `first` of every `of`
+    auto passes=[&](const SceneDev<T>& sc,const int* rec,const T (*sv)[TILE_S],int* run,int first,int of){
+        if constexpr(sizeof(T)==4) hessian_pairs(S,sc,rec[ITEM_START],rec[ITEM_PAIRS],first*32,of*32,sv,q,slots);
+        else{
+            const int np=rec[ITEM_COUNT],stride=(np+31)>>5;
+            for(int qi=first;qi<stride;qi+=of) hessian_pass(S,sc,rec[ITEM_START],run,qi,stride,np,sv,q);}};
+    auto flush=[&](const int* rec,unsigned e,T v0,T v1,T v2){
+        if(v0==T(0)&&v1==T(0)&&v2==T(0)) return;
+        const int blk=rec[ITEM_NBR+(e&31u)];
+        if(blk>=0) atomic_add_v3(S.gf+(long long)blk*64+((e>>5)&63u),v0,v1,v2,T(0));};
     if(form==HESS_CTA){
-        T (*q)[3][TILE_S]=reinterpret_cast<T (*)[3][TILE_S]>(smem_raw);                 // [warp][component][node]
-        T (*sv)[TILE_S]=reinterpret_cast<T (*)[TILE_S]>(smem_raw+NW*3*TILE_S*sizeof(T)); // [component][node]
-        int* nbr=nbr_s[0];int* run=run_s[0];
+        T (*sv)[TILE_S]=tile_of(0)+3;
+        int* rec=rec_s[0];int* run=run_s[0];
+        int mine=blockIdx.x<nwork?S.items[item(blockIdx.x)*ITEM_WORDS+lane]:0;
         for(long long w=blockIdx.x;w<nwork;w+=gridDim.x){
-            ChunkInfo<T> ci;load_chunk(S,item(w),nc,nv,ci,nbr);
-            if(S.cg[ci.scene].done) continue;    // uniform over the CTA
-            // a work item longer than `chunk` only arises when the work-item capacity was
-            // exceeded (ERR_CAPACITY is set); its run table would not fit: skip it (uniform)
-            if(ci.e-ci.s>S.chunk) continue;
-            const T beta=(T)S.cg[ci.scene].beta;
-            if(warp==0) chunk_runs(ci.e-ci.s,(ci.e-ci.s+31)>>5,run);
+            if(warp==0) rec[lane]=mine;
             __syncthreads();
-            stage_vector<P,FROM_X>(S,nbr,beta,sv,threadIdx.x,blockDim.x);
-            for(int t=threadIdx.x;t<NW*3*TILE_S;t+=blockDim.x) (&q[0][0][0])[t]=T(0);
+            if(w+gridDim.x<nwork) mine=S.items[item(w+gridDim.x)*ITEM_WORDS+lane];
+            const int scene=rec[ITEM_SCENE];
+            stage_vector<P,FROM_X,XFER_THREADS>(S,rec+ITEM_NBR,tmap,FROM_X?T(0):(T)S.cg[scene].beta,sv,threadIdx.x);
+            if constexpr(sizeof(T)==8) if(warp==0) chunk_runs(rec[ITEM_COUNT],(rec[ITEM_COUNT]+31)>>5,run);
             __syncthreads();
-            const SceneDev<T>& sc=S.scenes[ci.scene];
-            const int np=ci.e-ci.s,stride=(np+31)>>5;
-            for(int qi=warp;qi<stride;qi+=NW) hessian_pass<P>(S,sc,ci,run,qi,stride,np,sv,q[warp],qi+NW<stride?qi+NW:-1);
+            passes(S.scenes[scene],rec,sv,run,warp,NW);
             __syncthreads();
             for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x){
-                const int ta=tile_addr(t);
+                const unsigned e=tmap[t];
                 T v[3];
 #pragma unroll
                 for(int ch=0;ch<3;++ch){T a=T(0);
 #pragma unroll
-                    for(int w2=0;w2<NW;++w2) a+=q[w2][ch][ta];
+                    for(int w2=0;w2<NW;++w2){T* p=&tile_of(w2)[ch][e>>11];a+=*p;*p=T(0);}
                     v[ch]=a;}
-                if(v[0]==T(0)&&v[1]==T(0)&&v[2]==T(0)) continue;
-                const long long node=tile_node(nbr,t);
-                if(node<0) continue;
-                atomic_add_v3(S.gf+node,v[0],v[1],v[2],T(0));}
+                flush(rec,e,v[0],v[1],v[2]);}
             __syncthreads();
         }
     }
     else{
-        T (*q)[TILE_S]=reinterpret_cast<T (*)[TILE_S]>(smem_raw)+6*warp;   // [component][node], accumulated
-        T (*sv)[TILE_S]=q+3;                                                 // [component][node], gathered
-        int* nbr=nbr_s[warp];int* run=run_s[warp];
-        for(long long w=(long long)blockIdx.x*NW+warp;w<nwork;w+=(long long)gridDim.x*NW){
-            ChunkInfo<T> ci;load_chunk(S,item(w),nc,nv,ci,nbr,lane);
-            if(S.cg[ci.scene].done) continue;    // uniform over the warp
-            if(ci.e-ci.s>S.chunk) continue;       // capacity exceeded (see above)
-            const T beta=(T)S.cg[ci.scene].beta;
-            chunk_runs(ci.e-ci.s,(ci.e-ci.s+31)>>5,run);
+        T (*sv)[TILE_S]=q+3;
+        int* rec=rec_s[warp];int* run=run_s[sizeof(T)==8?warp:0];
+        const long long w0=(long long)blockIdx.x*NW+warp,dw=(long long)gridDim.x*NW;
+        int mine=w0<nwork?S.items[item(w0)*ITEM_WORDS+lane]:0;
+        for(long long w=w0;w<nwork;w+=dw){
+            rec[lane]=mine;
             __syncwarp();
-            stage_vector<P,FROM_X>(S,nbr,beta,sv,lane,32);
-            for(int t=lane;t<3*TILE_S;t+=32) (&q[0][0])[t]=T(0);
+            if(w+dw<nwork) mine=S.items[item(w+dw)*ITEM_WORDS+lane];
+            const int scene=rec[ITEM_SCENE];
+            stage_vector<P,FROM_X,32>(S,rec+ITEM_NBR,tmap,FROM_X?T(0):(T)S.cg[scene].beta,sv,lane);
+            if constexpr(sizeof(T)==8) chunk_runs(rec[ITEM_COUNT],(rec[ITEM_COUNT]+31)>>5,run);
             __syncwarp();
-            const SceneDev<T>& sc=S.scenes[ci.scene];
-            const int np=ci.e-ci.s,stride=(np+31)>>5;
-            for(int qi=0;qi<stride;++qi) hessian_pass<P>(S,sc,ci,run,qi,stride,np,sv,q,qi+1<stride?qi+1:-1);
+            passes(S.scenes[scene],rec,sv,run,0,1);
             __syncwarp();
             for(int t=lane;t<TILE_N;t+=32){
-                const int ta=tile_addr(t);
-                const T v0=q[0][ta],v1=q[1][ta],v2=q[2][ta];
-                if(v0==T(0)&&v1==T(0)&&v2==T(0)) continue;
-                const long long node=tile_node(nbr,t);
-                if(node<0) continue;
-                atomic_add_v3(S.gf+node,v0,v1,v2,T(0));}
+                const unsigned e=tmap[t];
+                T* p=&q[0][e>>11];
+                const T v0=p[0],v1=p[TILE_S],v2=p[2*TILE_S];
+                p[0]=p[TILE_S]=p[2*TILE_S]=T(0);
+                flush(rec,e,v0,v1,v2);}
             __syncwarp();
         }
     }
