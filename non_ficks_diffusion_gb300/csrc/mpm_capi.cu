@@ -56,7 +56,7 @@ struct mpm_context {
     // key-pass status words from inc_status_off, sort status words from sort_status_off.
     unsigned* sortws=nullptr; long long sortws_len=0,bin_heads_off=0,bin_blocks_off=0,inc_status_off=0,sort_status_off=0;
     int* chunk_start=nullptr; long long chunk_cap=0;
-    unsigned* pairs=nullptr; int* items=nullptr;   // FP32 pair tables and records of the work items
+    int* items=nullptr;                       // records of the work items
     // blocks and nodes
     unsigned* bitmap=nullptr; long long bitmap_words=0;
     int* blockmap=nullptr; int* active_gb=nullptr; int* active_scene=nullptr; long long block_cap=0;
@@ -157,7 +157,8 @@ template<class P> DevState<TT<P>> make_state(mpm_context* c,int parity,double dt
     S.cache=(V4<T>*)c->cache;S.pcap=c->cfg.max_particles;S.n_total=c->n_total;
     const int fin=c->sort_passes&1;   // the sort's final ping-pong buffer
     S.keys=c->keys[fin];S.perm=c->vals[fin];
-    S.chunk_start=c->chunk_start;S.chunk_cap=c->chunk_cap;S.pairs=c->pairs;S.items=c->items;
+    S.chunk_start=c->chunk_start;S.chunk_cap=c->chunk_cap;S.items=c->items;
+    S.pairs=c->mkeys[0];                      // free between the binning and the next substep's
     S.bitmap=c->bitmap;S.bitmap_words=c->bitmap_words;
     S.blockmap=c->blockmap;S.active_gb=c->active_gb;S.active_scene=c->active_scene;S.block_cap=c->block_cap;
     S.gv=(V4<T>*)c->gv;S.gf=(V4<T>*)c->gf;S.gx=(V4<T>*)c->gx;S.gr=(V4<T>*)c->gr;S.gs=(V4<T>*)c->gs;S.gm=(T*)c->gm;S.gproj=c->gproj;
@@ -705,7 +706,6 @@ template<class P> mpm_status alloc_buffers(mpm_context* c)
         c->sortws_len=c->sort_status_off+4LL*((pc+(long long)RS_THREADS*RS_ITEMS_SMALL-1)/((long long)RS_THREADS*RS_ITEMS_SMALL))*256;}
     CUDA_TRY(c,M((void**)&c->sortws,sizeof(unsigned)*c->sortws_len));
     CUDA_TRY(c,M((void**)&c->chunk_start,sizeof(int)*c->chunk_cap));
-    CUDA_TRY(c,M((void**)&c->pairs,sizeof(unsigned)*pc));
     CUDA_TRY(c,M((void**)&c->items,sizeof(int)*ITEM_WORDS*c->chunk_cap));
     CUDA_TRY(c,M((void**)&c->bitmap,sizeof(unsigned)*c->bitmap_words));
     CUDA_TRY(c,M((void**)&c->blockmap,sizeof(int)*base));
@@ -875,7 +875,7 @@ mpm_status mpm_destroy(mpm_context* c)
     if(c->stream) cudaStreamSynchronize(c->stream);
     for(int p=0;p<2;++p){if(c->gexec[p]) cudaGraphExecDestroy(c->gexec[p]);if(c->fgexec[p]) cudaGraphExecDestroy(c->fgexec[p]);}
     void* bufs[]={c->pstate[0],c->pstate[1],c->pid[0],c->pid[1],c->scn[0],c->scn[1],c->cache,c->keys[0],c->keys[1],c->vals[0],c->vals[1],
-                  c->sortws,c->chunk_start,c->pairs,c->items,c->bitmap,c->blockmap,c->active_gb,c->active_scene,c->gv,c->gf,c->gx,c->gr,c->gs,c->gm,c->gproj,
+                  c->sortws,c->chunk_start,c->items,c->bitmap,c->blockmap,c->active_gb,c->active_scene,c->gv,c->gf,c->gx,c->gr,c->gs,c->gm,c->gproj,
                   c->scenes_dev,c->scene_block_base,c->cg,c->acc,c->acc2,c->ctr,c->staging,c->d_dt,c->frame,c->inv,
                   c->srange,c->alist,c->mkeys[0],c->mkeys[1],c->mvals[0],c->mvals[1],c->mwords,c->manchor};
     for(void* p:bufs) if(p) cudaFree(p);

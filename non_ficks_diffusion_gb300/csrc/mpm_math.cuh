@@ -475,7 +475,7 @@ template<class T> MPM_HD void dP_dF(const T* Fe,const T* Re,const T lambda,const
     for(int k=0;k<9;++k) dP[k]=m2*(dF[k]-dR[k])+lh*H[k]+lj*dH[k];
 }
 
-// The elastic Hessian of one particle in the rotated-free form the CG products use. With the
+// The elastic Hessian of one particle in the rotation-free form the CG products use. With the
 // left polar form F = S R (S = R F^T symmetric), J = det F and dF = G F:
 //   dF F^T = G S^2,  cof(F) F^T = J I,  cof(F):dF = J tr G,  d(cof F) F^T = J (tr G I - G^T),
 // and R W R^T = W' solves W' S + S W' = M - M^T for M = G S, so that dP of dP_dF becomes

@@ -50,6 +50,13 @@ __device__ __forceinline__ void atomic_add_v3(V4<float>* p,float x,float y,float
 __device__ __forceinline__ void atomic_add_v3(V4<double>* p,double x,double y,double z,double w)
 {atomicAdd(&p->x,x);atomicAdd(&p->y,y);atomicAdd(&p->z,z);if(w!=0.) atomicAdd(&p->w,w);}
 
+// Hides a value from the compiler's loop-invariant motion: the scatters' rounds loop mostly
+// runs once, and the coefficients of all nine (x, y) columns hoisted out of it would take more
+// registers than a thread has.
+__device__ __forceinline__ void opaque(float& x){asm volatile("":"+f"(x));}
+__device__ __forceinline__ void opaque(float2& x){asm volatile("":"+f"(x.x),"+f"(x.y));}
+__device__ __forceinline__ void opaque(double& x){asm volatile("":"+d"(x));}
+
 // Chunk geometry: particle range, block, scene and the 27 neighbour active indices.
 template<class T> struct ChunkInfo {
     int s,e,scene;
@@ -367,25 +374,28 @@ __device__ __forceinline__ unsigned pair_entry(int k,bool two,unsigned cell,int 
     if(two){const int L1=(k+1)/stride;p1=run[k+1-L1*stride]+L1;}
     return (unsigned)p0|((unsigned)p1<<12)|(cell<<24)|(two?PAIR_TWO:0u);
 }
-// Written by one warp; rank_end[r] is the end of scatter rank r in the item's slot order and
-// cell_of[r] its cell. Returns the number of pairs.
+// Called by every warp of the CTA, which writes the levels warp, warp + nw, ...; rank_end[r] is
+// the end of scatter rank r in the item's slot order and cell_of[r] its cell. Returns the
+// number of pairs.
 __device__ __forceinline__ int pair_table(const int* rank_end,const unsigned char* cell_of,int stride,const int* run,unsigned* out)
 {
-    const int lane=threadIdx.x&31;
+    const int lane=threadIdx.x&31,warp=threadIdx.x>>5,nw=blockDim.x>>5;
     const int e0=rank_end[2*lane],e1=rank_end[2*lane+1];
     int s0=__shfl_up_sync(0xffffffffu,e1,1);
     if(lane==0) s0=0;
     const unsigned below=lane_bits_below();
     const unsigned c0=cell_of[2*lane],c1=cell_of[2*lane+1];
     int base=0;
-    for(int j=0;;++j){
+    for(int j=0,mine=warp;;++j){
         const int k0=s0+2*j,k1=e0+2*j;
         const unsigned m0=__ballot_sync(0xffffffffu,k0<e0),m1=__ballot_sync(0xffffffffu,k1<e1);
         if((m0|m1)==0u) break;
-        if(k0<e0) out[base+__popc(m0&below)]=pair_entry(k0,k0+1<e0,c0,stride,run);
-        base+=__popc(m0);
-        if(k1<e1) out[base+__popc(m1&below)]=pair_entry(k1,k1+1<e1,c1,stride,run);
-        base+=__popc(m1);}
+        const int b1=base+__popc(m0);
+        if(j==mine){                                   // uniform over the warp
+            mine+=nw;
+            if(k0<e0) out[base+__popc(m0&below)]=pair_entry(k0,k0+1<e0,c0,stride,run);
+            if(k1<e1) out[b1+__popc(m1&below)]=pair_entry(k1,k1+1<e1,c1,stride,run);}
+        base=b1+__popc(m1);}
     return base;
 }
 
@@ -505,6 +515,8 @@ template<class P> __device__ __forceinline__ void p2g_pass(const DevState<typena
         const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
         if(valid&&R.rank==r){
             const int tb=tile_addr(st.r[0]-1,st.r[1]-1,st.r[2]-1);
+#pragma unroll
+            for(int k=0;k<3;++k){opaque(st.w[0][k]);opaque(st.dw[0][k]);}
             const T mv0=m*V[0],mv1=m*V[1],mv2=m*V[2];
             const T mg0=sc.gravity[0]*m,mg1=sc.gravity[1]*m,mg2=sc.gravity[2]*m;
 #pragma unroll
@@ -606,11 +618,9 @@ template<class P,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) 
         if(warp==0) chunk_runs(np,stride,run);        // read after the barriers in chunk_cell_order
         for(int t=threadIdx.x;t<NW*7*TILE_S;t+=blockDim.x) (&acc[0][0][0])[t]=T(0);
         chunk_cell_order(S.keys,ci.s,np,crank,ocnt,inv,cellv);
-        // the last warp has the fewest passes; its counts now hold the ends of the ranks
-        if constexpr(sizeof(T)==4){
-            if(warp==NW-1){
-                const int m=pair_table(ocnt[NW-1],cell_of,stride,run,S.pairs+ci.s);
-                if((threadIdx.x&31)==0) S.items[c*ITEM_WORDS+ITEM_PAIRS]=m;}}
+        if constexpr(sizeof(T)==4){                   // the last warp's counts now hold the ends of the ranks
+            const int m=pair_table(ocnt[NW-1],cell_of,stride,run,S.pairs+ci.s);
+            if(threadIdx.x==0) S.items[c*ITEM_WORDS+ITEM_PAIRS]=m;}
         const SceneDev<T>& sc=S.scenes[ci.scene];
         for(int qi=warp;qi<stride;qi+=NW) p2g_pass<P>(S,sc,ci,run,inv,cellv,qi,stride,np,acc[warp]);
         __syncthreads();
@@ -850,12 +860,64 @@ __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const Sce
         __syncwarp();}
 }
 
-// FP32: two particles of one cell per lane (the pair table). The 81 node values of the cell's
-// stencil are read once for both, and both particles' forces are added to the tile in one
-// read and one write per node. The particles' vectors arrive in shared memory by
-// asynchronous copies issued one pass ahead (slots[k][lane], read only by the lane that
-// copied them), so that no load latency is left in a pass and the coefficients take no
-// registers during the gather.
+// FP32: two particles of one cell per lane (the pair table), every operation on both as a
+// packed pair: (p, q) of the two particles in one register pair, each half rounded like the
+// scalar operation. The 81 node values of the cell's stencil are read once for both, and
+// both particles' forces are added to the tile in one read and one write per node. The
+// particles' vectors arrive in shared memory by asynchronous copies issued one pass ahead
+// (slots[k][lane], read only by the lane that copied them), so that no load latency is
+// left in a pass and the coefficients take no registers during the gather.
+// Bound by the FMA pipe and issue (53 % each busy, 4 CTAs per SM): per product 0.158 ->
+// 0.107 ms on 1.94M particles, 1.32 -> 0.83 ms on 21.5M, against one particle per lane with
+// its Fe, Re, lambda, mu and V0 read as 25 separate words. Of that the stress form of
+// HessianData gives 1.32 -> 1.08, pairs, item records and copies ahead the rest.
+__device__ __forceinline__ float2 padd(float2 a,float2 b){return __fadd2_rn(a,b);}
+__device__ __forceinline__ float2 psub(float2 a,float2 b){return __ffma2_rn(b,make_float2(-1.f,-1.f),a);}   // exact product: rounds like a - b
+__device__ __forceinline__ float2 pabs(float2 a){return make_float2(fabsf(a.x),fabsf(a.y));}
+// bspline_weights of two coordinates, operation for operation.
+__device__ __forceinline__ void bspline_weights2(float2 x,float2 inv_dx,float2 (&w)[3],float2 (&dw)[3])
+{
+    const float2 half=pdup(.5f),th=pdup(1.5f);
+    w[0]=pabs(padd(psub(pmul(pmul(half,x),x),pmul(th,x)),pdup(1.125f)));
+    dw[0]=pmul(psub(x,th),inv_dx);
+    float2 y=psub(x,pdup(1.f));
+    w[1]=pabs(psub(pdup(.75f),pmul(y,y)));
+    dw[1]=pmul(pmul(pdup(-2.f),y),inv_dx);
+    y=psub(y,pdup(1.f));
+    w[2]=pabs(padd(padd(pmul(pmul(half,y),y),pmul(th,y)),pdup(1.125f)));
+    dw[2]=pmul(padd(y,th),inv_dx);
+}
+// B = V0 dP Fe^T from G for two particles (hessian_stress).
+__device__ __forceinline__ void hessian_stress2(const float2 (&G)[3][3],const float2 (&Sm)[6],float2 c1,float2 c2,float2 cc3,float2 (&B)[3][3])
+{
+    const int ix[3][3]={{0,1,2},{1,3,4},{2,4,5}};
+    float2 M[3][3];
+#pragma unroll
+    for(int i=0;i<3;++i)
+#pragma unroll
+        for(int j=0;j<3;++j) M[i][j]=pfma(G[i][2],Sm[ix[2][j]],pfma(G[i][1],Sm[ix[1][j]],pmul(G[i][0],Sm[ix[0][j]])));
+    // K a = L for the axial vector (a, b, c) of W' (skew_system_inverse)
+    const float2 k00=padd(Sm[3],Sm[0]),k01=Sm[4],k02=pmul(Sm[2],pdup(-1.f)),k11=padd(Sm[5],Sm[0]),k12=Sm[1],k22=padd(Sm[5],Sm[3]);
+    auto det2=[](float2 p,float2 q,float2 r,float2 s){return psub(pmul(p,q),pmul(r,s));};
+    const float2 i00=det2(k11,k22,k12,k12),i01=det2(k02,k12,k01,k22),i02=det2(k01,k12,k02,k11);
+    const float2 i11=det2(k00,k22,k02,k02),i12=det2(k01,k02,k00,k12),i22=det2(k00,k11,k01,k01);
+    const float2 det=pfma(k02,i02,pfma(k01,i01,pmul(k00,i00)));
+    const float2 inv=make_float2(1.f/det.x,1.f/det.y);
+    const float2 L0=pmul(psub(M[1][0],M[0][1]),inv),L1=pmul(psub(M[2][0],M[0][2]),inv),L2=pmul(psub(M[2][1],M[1][2]),inv);
+    const float2 a=pfma(i02,L2,pfma(i01,L1,pmul(i00,L0))),b=pfma(i12,L2,pfma(i11,L1,pmul(i01,L0))),c=pfma(i22,L2,pfma(i12,L1,pmul(i02,L0)));
+    M[0][1]=padd(M[0][1],a);M[0][2]=padd(M[0][2],b);M[1][2]=padd(M[1][2],c);
+    M[1][0]=psub(M[1][0],a);M[2][0]=psub(M[2][0],b);M[2][1]=psub(M[2][1],c);
+    const float2 tr=pmul(c2,padd(padd(G[0][0],G[1][1]),G[2][2])),n3=pmul(cc3,pdup(-1.f));
+    float2 cS[6];
+#pragma unroll
+    for(int k=0;k<6;++k) cS[k]=pmul(c1,Sm[k]);
+#pragma unroll
+    for(int i=0;i<3;++i)
+#pragma unroll
+        for(int j=0;j<3;++j){
+            const float2 g=i==j?pfma(n3,G[j][i],tr):pmul(n3,G[j][i]);
+            B[i][j]=pfma(M[i][2],cS[ix[2][j]],pfma(M[i][1],cS[ix[1][j]],pfma(M[i][0],cS[ix[0][j]],g)));}
+}
 __device__ __forceinline__ void copy_pair(const DevState<float>& S,int s,unsigned entry,V4<float> (*slots)[32])
 {
     const int lane=threadIdx.x&31;
@@ -871,7 +933,6 @@ __device__ __forceinline__ void copy_pair(const DevState<float>& S,int s,unsigne
 __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const SceneDev<float>& sc,int s,int M,int m0,int dm,
     const float (*sv)[TILE_S],float (*tile)[TILE_S],V4<float> (*slots)[32])
 {
-    constexpr int NP=2;
     const unsigned* tab=S.pairs+s;
     const int lane=threadIdx.x&31;
     unsigned entry=0,next=0;
@@ -880,47 +941,43 @@ __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const Sce
     for(int m=m0;m<M;m+=dm){
         const bool valid=m+lane<M;
         const unsigned cell=(entry>>24)&63u;
-        C3<float> B[NP][3];
-        Stencil<float> st[NP];
-        int tb=0;
+        const int tb=tile_addr((int)(cell&3u),(int)((cell>>2)&3u),(int)(cell>>4));
+        float2 B[3][3],w[3][3],dw[3][3];      // B[component][direction], w[axis][node]
         asm volatile("cp.async.wait_all;":::"memory");
+        // formed before the gather and again before the scatter: kept across the stress the
+        // 36 registers would cost a resident CTA
+        auto weights=[&](float2 (&w)[3][3],float2 (&dw)[3][3]){
+            const volatile V4<float>* p=&slots[0][lane];const volatile V4<float>* q=&slots[3][lane];
+            bspline_weights2(make_float2(p->x,q->x),pdup(sc.inv_dx[0]),w[0],dw[0]);
+            bspline_weights2(make_float2(p->y,q->y),pdup(sc.inv_dx[1]),w[1],dw[1]);
+            bspline_weights2(make_float2(p->z,q->z),pdup(sc.inv_dx[2]),w[2],dw[2]);};
         if(valid){
-#pragma unroll
-            for(int h=0;h<NP;++h){
-                const V4<float> q0=slots[3*h][lane];
-                const float x[3]={q0.x,q0.y,q0.z};
-                stencil_from_coord(sc,cell,x,st[h]);}
-            tb=tile_addr(st[0].r[0]-1,st[0].r[1]-1,st[0].r[2]-1);
-            C3<float> G[NP][3];
-#pragma unroll
-            for(int h=0;h<NP;++h)
-#pragma unroll
-                for(int k=0;k<3;++k) G[h][k]=c3<float>(0.f,0.f,0.f);
+            weights(w,dw);
+            float2 G[3][3];
 #pragma unroll
             for(int ox=0;ox<3;++ox)
 #pragma unroll
             for(int oy=0;oy<3;++oy){
-                C3<float> t[NP],u[NP];
+                const float2 dxy=pmul(dw[0][ox],w[1][oy]),xdy=pmul(w[0][ox],dw[1][oy]),wxy=pmul(w[0][ox],w[1][oy]);
 #pragma unroll
-                for(int oz=0;oz<3;++oz){
-                    const int n=tb+tile_addr(ox,oy,oz);
-                    const C3<float> v=c3<float>(sv[0][n],sv[1][n],sv[2][n]);
+                for(int a=0;a<3;++a){
+                    float2 t,u;
 #pragma unroll
-                    for(int h=0;h<NP;++h){
-                        t[h]=oz==0?mul(v,st[h].w[2][oz]):madd(v,st[h].w[2][oz],t[h]);
-                        u[h]=oz==0?mul(v,st[h].dw[2][oz]):madd(v,st[h].dw[2][oz],u[h]);}}
-#pragma unroll
-                for(int h=0;h<NP;++h){
-                    G[h][0]=madd(t[h],st[h].dw[0][ox]*st[h].w[1][oy],G[h][0]);
-                    G[h][1]=madd(t[h],st[h].w[0][ox]*st[h].dw[1][oy],G[h][1]);
-                    G[h][2]=madd(u[h],st[h].w[0][ox]*st[h].w[1][oy],G[h][2]);}}
-#pragma unroll
-            for(int h=0;h<NP;++h){
-                const V4<float> q0=slots[3*h][lane],q1=slots[3*h+1][lane],q2=slots[3*h+2][lane];
-                const float Sm[6]={q1.x,q1.y,q1.z,q1.w,q2.x,q2.y};
-                const float on=h==0||(entry&PAIR_TWO)?1.f:0.f;      // no second particle: no force
-                float Ki[6];skew_system_inverse(Sm,Ki);
-                hessian_stress<float>(G[h],Sm,on*q0.w,on*q2.z,on*q2.w,Ki,B[h]);}}
+                    for(int oz=0;oz<3;++oz){
+                        const float2 v=pdup(sv[a][tb+tile_addr(ox,oy,oz)]);
+                        t=oz==0?pmul(v,w[2][oz]):pfma(v,w[2][oz],t);
+                        u=oz==0?pmul(v,dw[2][oz]):pfma(v,dw[2][oz],u);}
+                    const bool first=ox==0&&oy==0;
+                    G[a][0]=first?pmul(t,dxy):pfma(t,dxy,G[a][0]);
+                    G[a][1]=first?pmul(t,xdy):pfma(t,xdy,G[a][1]);
+                    G[a][2]=first?pmul(u,wxy):pfma(u,wxy,G[a][2]);}}
+            const V4<float> p1=slots[1][lane],q1=slots[4][lane],p2=slots[2][lane],q2=slots[5][lane];
+            const float2 Sm[6]={make_float2(p1.x,q1.x),make_float2(p1.y,q1.y),make_float2(p1.z,q1.z),
+                                make_float2(p1.w,q1.w),make_float2(p2.x,q2.x),make_float2(p2.y,q2.y)};
+            const bool two=(entry&PAIR_TWO)!=0u;                    // no second particle: no force
+            hessian_stress2(G,Sm,make_float2(slots[0][lane].w,two?slots[3][lane].w:0.f),make_float2(p2.z,two?q2.z:0.f),
+                            make_float2(p2.w,two?q2.w:0.f),B);
+            weights(w,dw);}
         entry=next;
         if(m+dm+lane<M) copy_pair(S,s,entry,slots);
         if(m+2*dm+lane<M) next=tab[m+2*dm+lane];
@@ -929,21 +986,28 @@ __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const Sce
             const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
             if(valid&&R.rank==r){
 #pragma unroll
+                for(int k=0;k<3;++k){
+                    opaque(w[0][k]);opaque(dw[0][k]);
+#pragma unroll
+                    for(int a=0;a<3;++a) opaque(B[a][k]);}
+#pragma unroll
                 for(int ox=0;ox<3;++ox)
 #pragma unroll
                 for(int oy=0;oy<3;++oy){
-                    C3<float> al[NP],be[NP];
+                    const float2 dxy=pmul(dw[0][ox],w[1][oy]),xdy=pmul(w[0][ox],dw[1][oy]),wxy=pmul(w[0][ox],w[1][oy]);
+                    float2 al[3],be[3];
 #pragma unroll
-                    for(int h=0;h<NP;++h){
-                        al[h]=madd(B[h][1],st[h].w[0][ox]*st[h].dw[1][oy],mul(B[h][0],st[h].dw[0][ox]*st[h].w[1][oy]));
-                        be[h]=mul(B[h][2],st[h].w[0][ox]*st[h].w[1][oy]);}
+                    for(int a=0;a<3;++a){al[a]=pfma(B[a][1],xdy,pmul(B[a][0],dxy));be[a]=pmul(B[a][2],wxy);}
 #pragma unroll
                     for(int oz=0;oz<3;++oz){
                         const int t=tb+tile_addr(ox,oy,oz);
-                        C3<float> v=c3<float>(tile[0][t],tile[1][t],tile[2][t]);
+                        float v[3];
 #pragma unroll
-                        for(int h=0;h<NP;++h) v=madd(be[h],st[h].dw[2][oz],madd(al[h],st[h].w[2][oz],v));
-                        tile[0][t]=cx(v);tile[1][t]=cy(v);tile[2][t]=v.z;
+                        for(int a=0;a<3;++a){
+                            const float2 f=pfma(be[a],dw[2][oz],pfma(al[a],w[2][oz],make_float2(tile[a][t],0.f)));
+                            v[a]=f.x+f.y;}
+#pragma unroll
+                        for(int a=0;a<3;++a) tile[a][t]=v[a];
                         __syncwarp(rmask);}}}
             __syncwarp();}
     }
