@@ -350,6 +350,196 @@ MPM_HD void polar_refine_mixed(const float* F,float* R)
     for(int k=0;k<9;++k) R[k]=Rn[k];
 }
 
+// ---- FP32 pairs ----
+// An unevaluated sum h + l of two FP32 numbers. Products and sums that the error terms depend
+// on are rounded one by one (never contracted into a fused multiply-add).
+struct F2x { float h,l; };
+MPM_HD float ff_mul(float a,float b)
+{
+#ifdef __CUDA_ARCH__
+    return __fmul_rn(a,b);
+#else
+    return a*b;
+#endif
+}
+MPM_HD float ff_add(float a,float b)
+{
+#ifdef __CUDA_ARCH__
+    return __fadd_rn(a,b);
+#else
+    return a+b;
+#endif
+}
+// a0 b0 + a1 b1 + a2 b2 + c: the products split exactly by one FMA each, their sum by TwoSum,
+// the error terms and c (small) added up in l (Dot2, as in dot2_skew3). h + l has an error
+// below 2^-44 sum |terms|.
+MPM_HD F2x ff_dot3(float a0,float b0,float a1,float b1,float a2,float b2,float c=0.f)
+{
+    const float p0=ff_mul(a0,b0),p1=ff_mul(a1,b1),p2=ff_mul(a2,b2);
+    const float s=ff_add(p0,p1),z=ff_add(s,-p0),q=ff_add(ff_add(p0,-ff_add(s,-z)),ff_add(p1,-z));
+    const float t=ff_add(s,p2),y=ff_add(t,-s),r=ff_add(ff_add(s,-ff_add(t,-y)),ff_add(p2,-y));
+    return F2x{t,(fmaf(a0,b0,-p0)+fmaf(a1,b1,-p1))+(fmaf(a2,b2,-p2)+c)+(q+r)};
+}
+MPM_HD F2x ff_norm(F2x a){const float h=ff_add(a.h,a.l);return F2x{h,ff_add(a.l,-ff_add(h,-a.h))};}
+MPM_HD F2x ff_prod(F2x a,F2x b){const float p=ff_mul(a.h,b.h);return ff_norm(F2x{p,fmaf(a.h,b.h,-p)+(a.h*b.l+a.l*b.h)});}
+
+// The clamped plasticity update of the mixed variant from the FP32 SVD F ~ U diag(s) V^T
+// (s2 well above 0), to FP32 rounding of the exact result, without FP64 operations: the FP64
+// pipe runs at 1/64 of the FP32 rate, and the FP64 Jacobi this replaces took four fifths
+// of P2G once most particles yield (1.94M particles, nearly all clamped: P2G 1.79 -> 0.65 ms).
+// One step of first-order correction, its inputs evaluated to twice FP32 precision:
+//   dU = U^T U - I, dV = V^T V - I   (the orthonormal factors are U (I - dU/2), V (I - dV/2)),
+//   M = U^T F V - (dU D + D dV)/2 = D + E with D diagonal and E ~ 1e-7.
+// A function f of the singular values changes along E by the divided differences of f (Daleckii
+// and Krein; for singular values, Noferini, "A formula for the Frechet derivative of a
+// generalized matrix function", SIAM J. Matrix Anal. Appl. 38, 2017):
+//   N_ij = (f_i - f_j)/(d_i - d_j) (E_ij + E_ji)/2 + (f_i + f_j)/(d_i + d_j) (E_ij - E_ji)/2,
+// bounded for the clamp (its first quotient lies in [0, 1]); f = 1 gives the rotation. The
+// neglected terms are of order E^2. Fe, Re = U (f + N - (dU f + f dV)/2) V^T, the leading
+// product to twice FP32 precision.
+MPM_HD void clamp_refined(float* Fe,float& Jp,const float* U,const float* V,const float cy,const float sy,float* Re,float& Je)
+{
+    float dU[9],dV[9];               // symmetric
+#pragma unroll
+    for(int i=0;i<3;++i)
+#pragma unroll
+        for(int j=i;j<3;++j){
+            const F2x u=ff_dot3(U[i],U[j],U[3+i],U[3+j],U[6+i],U[6+j]),v=ff_dot3(V[i],V[j],V[3+i],V[3+j],V[6+i],V[6+j]);
+            dU[3*i+j]=dU[3*j+i]=(i==j?u.h-1.f:u.h)+u.l;
+            dV[3*i+j]=dV[3*j+i]=(i==j?v.h-1.f:v.h)+v.l;}
+    F2x D[3];float E[9];
+#pragma unroll
+    for(int j=0;j<3;++j){
+        F2x t[3];                     // column j of F V
+#pragma unroll
+        for(int k=0;k<3;++k) t[k]=ff_dot3(Fe[3*k],V[j],Fe[3*k+1],V[3+j],Fe[3*k+2],V[6+j]);
+#pragma unroll
+        for(int i=0;i<3;++i){
+            const F2x m=ff_dot3(U[i],t[0].h,U[3+i],t[1].h,U[6+i],t[2].h,U[i]*t[0].l+U[3+i]*t[1].l+U[6+i]*t[2].l);
+            if(i==j) D[i]=m; else E[3*i+j]=m.h+m.l;}}
+#pragma unroll
+    for(int i=0;i<3;++i){D[i].l-=0.5f*D[i].h*(dU[4*i]+dV[4*i]);D[i]=ff_norm(D[i]);}
+    // e[i][j] of the sum above, of which the symmetric part S enters with f's quotient
+    float S01,S02,S12,w01,w02,w12;
+    auto split=[&](int i,int j,float& sym,float& w){
+        const float di=D[i].h,dj=D[j].h,u=0.5f*dU[3*i+j],v=0.5f*dV[3*i+j];
+        const float e1=E[3*i+j]-(u*dj+di*v),e2=E[3*j+i]-(u*di+dj*v);
+        sym=0.5f*(e1+e2);w=(e1-e2)/(di+dj);};
+    split(0,1,S01,w01);split(0,2,S02,w02);split(1,2,S12,w12);
+    // The first order is not enough where singular values lie on both sides of one limit and
+    // about E or less apart. Those within 1e-4 of a limit (where E^2 over the gap is far below
+    // the rounding) have their small block, D - limit and S, diagonalised: Q, lam.
+    F2x f[3],q=F2x{1.f,0.f},jf=F2x{1.f,0.f};
+    const float rlo=0.f-cy,rhi=0.f-sy;
+    auto off=[&](int i,float r){return ff_add(D[i].h,r)+D[i].l;};
+    auto count=[&](float r){return (mpm_abs(off(0,r))<1e-4f)+(mpm_abs(off(1,r))<1e-4f)+(mpm_abs(off(2,r))<1e-4f);};
+    const float k=count(rlo)>=2?cy:count(rhi)>=2?sy:0.f;
+    bool near[3]={false,false,false};
+    float P01=0.f,P02=0.f,P12=0.f;
+    if(k!=0.f){
+        float a[3];
+#pragma unroll
+        for(int i=0;i<3;++i){a[i]=off(i,-k);near[i]=mpm_abs(a[i])<1e-4f;}
+        float a01=near[0]&&near[1]?S01:0.f,a02=near[0]&&near[2]?S02:0.f,a12=near[1]&&near[2]?S12:0.f;
+        float Q[9]={1.f,0.f,0.f,0.f,1.f,0.f,0.f,0.f,1.f};
+        auto rotate=[&](float& app,float& aqq,float& apq,float& arp,float& arq,int p,int r){
+            if(apq==0.f) return;
+            const float th=(aqq-app)/(2.f*apq);
+            const float t=(th>=0.f?1.f:-1.f)/(mpm_abs(th)+mpm_sqrt(th*th+1.f)),c=1.f/mpm_sqrt(t*t+1.f),sn=t*c;
+            app-=t*apq;aqq+=t*apq;apq=0.f;
+            const float rp=arp,rq=arq;arp=c*rp-sn*rq;arq=sn*rp+c*rq;
+#pragma unroll
+            for(int m=0;m<3;++m){const float vp=Q[3*m+p],vq=Q[3*m+r];Q[3*m+p]=c*vp-sn*vq;Q[3*m+r]=sn*vp+c*vq;}};
+#pragma unroll 1
+        for(int sweep=0;sweep<3;++sweep){
+            rotate(a[0],a[1],a01,a02,a12,0,1);rotate(a[0],a[2],a02,a01,a12,0,2);rotate(a[1],a[2],a12,a01,a02,1,2);}
+        float ph[3];
+#pragma unroll
+        for(int m=0;m<3;++m){
+            ph[m]=near[m]?fminf(fmaxf(a[m],cy-k),sy-k):0.f;        // f(k + lam) - k
+            if(near[m]){q=ff_prod(q,F2x{1.f,(a[m]-ph[m])/(k+ph[m])});jf=ff_prod(jf,F2x{k,ph[m]});}}
+        auto back=[&](int i,int j){return Q[3*i]*ph[0]*Q[3*j]+Q[3*i+1]*ph[1]*Q[3*j+1]+Q[3*i+2]*ph[2]*Q[3*j+2];};
+        P01=back(0,1);P02=back(0,2);P12=back(1,2);
+#pragma unroll
+        for(int i=0;i<3;++i) if(near[i]) f[i]=F2x{k,back(i,i)};}
+#pragma unroll
+    for(int i=0;i<3;++i) if(!near[i]){
+        // the sign of D - limit decides, as one rounding of the exact value would
+        const bool up=off(i,rhi)>0.f,lo=off(i,rlo)<0.f;
+        f[i]=up?F2x{sy,0.f}:lo?F2x{cy,0.f}:D[i];
+        jf=ff_prod(jf,f[i]);
+        if(up||lo){                  // q *= D / f
+            const float r=1.f/f[i].h,qh=D[i].h*r;
+            q=ff_prod(q,F2x{qh,(fmaf(-qh,f[i].h,D[i].h)+D[i].l)*r});}}
+    const float jh=ff_mul(Jp,q.h);
+    Jp=jh+(fmaf(Jp,q.h,-jh)+Jp*q.l);
+    Je=jf.h+jf.l;
+    float C[9],W[9];                 // corrections of Fe and of Re inside U (.) V^T
+#pragma unroll
+    for(int i=0;i<3;++i){
+        C[4*i]=f[i].l-0.5f*f[i].h*(dU[4*i]+dV[4*i]);
+        W[4*i]=-0.5f*(dU[4*i]+dV[4*i]);}
+    auto couple=[&](int i,int j,float sym,float w,float P){
+        const float fi=f[i].h+f[i].l,fj=f[j].h+f[j].l,u=0.5f*dU[3*i+j],v=0.5f*dV[3*i+j];
+        const float gap=ff_add(D[i].h,-D[j].h)+(D[i].l-D[j].l),num=ff_add(f[i].h,-f[j].h)+(f[i].l-f[j].l);
+        // equal singular values: the clamp's slope there (0 beyond a limit, else 1)
+        const float a=gap!=0.f?fminf(fmaxf(num/gap,0.f),1.f):(fi==sy||fi==cy?0.f:1.f);
+        const float sm=near[i]&&near[j]?P:a*sym,sk=0.5f*(fi+fj)*w;
+        C[3*i+j]=sm+sk-(u*fj+fi*v);C[3*j+i]=sm-sk-(u*fi+fj*v);
+        W[3*i+j]=w-(u+v);W[3*j+i]=-w-(u+v);};
+    couple(0,1,S01,w01,P01);couple(0,2,S02,w02,P02);couple(1,2,S12,w12,P12);
+#pragma unroll
+    for(int i=0;i<3;++i){
+        float ph[3],pl[3],cf[3],cr[3];      // row i of U f (split exactly), U C, U W
+#pragma unroll
+        for(int k=0;k<3;++k){
+            ph[k]=ff_mul(U[3*i+k],f[k].h);pl[k]=fmaf(U[3*i+k],f[k].h,-ph[k]);
+            cf[k]=U[3*i]*C[k]+U[3*i+1]*C[3+k]+U[3*i+2]*C[6+k];
+            cr[k]=U[3*i]*W[k]+U[3*i+1]*W[3+k]+U[3*i+2]*W[6+k];}
+#pragma unroll
+        for(int j=0;j<3;++j){
+            const float v0=V[3*j],v1=V[3*j+1],v2=V[3*j+2];
+            const F2x x=ff_dot3(ph[0],v0,ph[1],v1,ph[2],v2,(pl[0]+cf[0])*v0+(pl[1]+cf[1])*v1+(pl[2]+cf[2])*v2);
+            Fe[3*i+j]=x.h+x.l;
+            const F2x y=ff_dot3(U[3*i],v0,U[3*i+1],v1,U[3*i+2],v2,cr[0]*v0+cr[1]*v1+cr[2]*v2);
+            Re[3*i+j]=y.h+y.l;}}
+}
+
+// The clamp by the FP64 Jacobi SVD (to `rel`, see svd3) warm-started from the FP32 V.
+template<class T> MPM_HD void clamp_fp64(T* Fe,T& Jp,const float* V32,const int plastic,const T cy,const T sy,const double rel,T* Re,T& Je)
+{
+    double F[9],U[9],s[3],V[9],V0[9];
+#pragma unroll
+    for(int k=0;k<9;++k){F[k]=(double)Fe[k];V0[k]=(double)V32[k];}
+    orthonormalize3(V0);
+    svd3<double,4>(F,U,s,V,V0,rel);
+    const double prod_s=s[0]*s[1]*s[2];
+    if(plastic){
+#pragma unroll
+        for(int i=0;i<3;++i){if(s[i]>(double)sy) s[i]=(double)sy;if(s[i]<(double)cy) s[i]=(double)cy;}
+        Jp=(T)((double)Jp*(prod_s/(s[0]*s[1]*s[2])));
+#pragma unroll
+        for(int i=0;i<3;++i)
+#pragma unroll
+            for(int j=0;j<3;++j) Fe[3*i+j]=(T)(U[3*i]*s[0]*V[3*j]+U[3*i+1]*s[1]*V[3*j+1]+U[3*i+2]*s[2]*V[3*j+2]);}
+    Je=(T)(s[0]*s[1]*s[2]);
+    double R[9];mat_mul_bt(U,V,R);
+#pragma unroll
+    for(int k=0;k<9;++k) Re[k]=(T)R[k];
+}
+// The same out of line, for the mixed variant, where it is rare: inlined, its code would push
+// P2G's loop out of the instruction cache. An FP64 SVD to 1e-12 relative (one sweep from
+// the FP32 start, as a rule) is four orders below the FP32 rounding of Fe, Jp and Re.
+struct ClampArgs { float Fe[9],V32[9],Jp,cy,sy; };
+struct ClampResult { float Fe[9],Re[9],Jp,Je; };
+static __host__ __device__ __noinline__ ClampResult clamp_fp64_cold(ClampArgs a)
+{
+    ClampResult r;r.Jp=a.Jp;
+    for(int k=0;k<9;++k) r.Fe[k]=a.Fe[k];
+    clamp_fp64<float>(r.Fe,r.Jp,a.V32,1,a.cy,a.sy,1e-12,r.Re,r.Je);
+    return r;
+}
+
 // Precompute: SVD of Fe, clamp of the singular values to [cy, sy], Jp update (det of the
 // reference's Fp <- V S^-1 U^T Fe Fp), Fe <- U S_hat V^T, hardened Lame parameters,
 // Re = U V^T. Writes Fe, Jp in place (rounded to T).
@@ -358,8 +548,10 @@ MPM_HD void polar_refine_mixed(const float* F,float* R)
 // first done in FP32. If those singular values lie inside [cy, sy] by a margin far above
 // the FP32 error, no clamp happens in exact arithmetic, so Fe and Jp are unchanged and
 // only the polar rotation Re is needed, refined in FP64 from the FP32 U V^T by
-// polar_refine3. Otherwise the FP64 Jacobi SVD runs, warm-started from the FP32 V, and the
-// clamp and reconstruction are done in FP64.
+// polar_refine3 or polar_refine_mixed. Otherwise the mixed variant corrects the FP32 SVD to
+// FP32 rounding of the exact clamp (clamp_refined); for singular values far from 1, where the
+// correction's quotients are not well conditioned, and in the FP64 variant the FP64 Jacobi
+// SVD runs, warm-started from the FP32 V, and clamp and reconstruction are done in FP64.
 template<class T,class TS> MPM_HD void precompute(T* Fe,T& Jp,const T lambda0,const T mu0,
     const int plastic,const T hardening,const T cy,const T sy,const T hardening_max,
     T* Re,T& lambda,T& mu,T& Je)
@@ -368,41 +560,32 @@ template<class T,class TS> MPM_HD void precompute(T* Fe,T& Jp,const T lambda0,co
 #pragma unroll
     for(int k=0;k<9;++k) F32[k]=(float)Fe[k];
     svd3<float>(F32,U32,s32,V32);
-    const bool fp32_only=sizeof(TS)==4;
     const float margin=1e-5f;
     const bool inside=s32[0]<(float)sy-margin&&s32[2]>(float)cy+margin;
-    if(fp32_only||(plastic&&!inside)){
-        TS F[9],U[9],s[3],V[9];
-#pragma unroll
-        for(int k=0;k<9;++k) F[k]=(TS)Fe[k];
-        if(fp32_only){
-#pragma unroll
-            for(int k=0;k<9;++k){U[k]=(TS)U32[k];V[k]=(TS)V32[k];}
-#pragma unroll
-            for(int k=0;k<3;++k) s[k]=(TS)s32[k];}
-        else{
-            TS V0[9];
-#pragma unroll
-            for(int k=0;k<9;++k) V0[k]=(TS)V32[k];
-            orthonormalize3(V0);
-            // the mixed variant stores Fe, Jp and Re in FP32: an FP64 SVD to 1e-12 relative
-            // (one sweep from the FP32 start, as a rule) is four orders below that rounding
-            svd3<TS,4>(F,U,s,V,V0,sizeof(T)==4?TS(1e-12):TS(0));}
-        const TS prod_s=s[0]*s[1]*s[2];
+    if constexpr(sizeof(TS)==4){
         if(plastic){
-            const TS tsy=(TS)sy,tcy=(TS)cy;
+            const T prod_s=s32[0]*s32[1]*s32[2];
 #pragma unroll
-            for(int i=0;i<3;++i){if(s[i]>tsy) s[i]=tsy;if(s[i]<tcy) s[i]=tcy;}
-            const TS prod_hat=s[0]*s[1]*s[2];
-            Jp=(T)((TS)Jp*(prod_s/prod_hat));
+            for(int i=0;i<3;++i){if(s32[i]>sy) s32[i]=sy;if(s32[i]<cy) s32[i]=cy;}
+            const T prod_hat=s32[0]*s32[1]*s32[2];
+            Jp=Jp*(prod_s/prod_hat);
 #pragma unroll
             for(int i=0;i<3;++i)
 #pragma unroll
-                for(int j=0;j<3;++j) Fe[3*i+j]=(T)(U[3*i]*s[0]*V[3*j]+U[3*i+1]*s[1]*V[3*j+1]+U[3*i+2]*s[2]*V[3*j+2]);}
-        Je=(T)(s[0]*s[1]*s[2]);
-        TS R[9];mat_mul_bt(U,V,R);
+                for(int j=0;j<3;++j) Fe[3*i+j]=U32[3*i]*s32[0]*V32[3*j]+U32[3*i+1]*s32[1]*V32[3*j+1]+U32[3*i+2]*s32[2]*V32[3*j+2];}
+        Je=s32[0]*s32[1]*s32[2];
+        mat_mul_bt(U32,V32,Re);}
+    else if(plastic&&!inside){
+        if constexpr(sizeof(T)==8) clamp_fp64<T>(Fe,Jp,V32,plastic,cy,sy,0.,Re,Je);
+        else if(s32[2]>0.25f&&s32[0]<4.f) clamp_refined(Fe,Jp,U32,V32,cy,sy,Re,Je);
+        else{
+            ClampArgs a;a.Jp=Jp;a.cy=cy;a.sy=sy;
 #pragma unroll
-        for(int k=0;k<9;++k) Re[k]=(T)R[k];}
+            for(int k=0;k<9;++k){a.Fe[k]=Fe[k];a.V32[k]=V32[k];}
+            const ClampResult r=clamp_fp64_cold(a);
+#pragma unroll
+            for(int k=0;k<9;++k){Fe[k]=r.Fe[k];Re[k]=r.Re[k];}
+            Jp=r.Jp;Je=r.Je;}}
     else{
         float R32[9];mat_mul_bt(U32,V32,R32);
         if constexpr(sizeof(T)==8){
