@@ -259,7 +259,6 @@ template<class P> void enqueue_cg_body(mpm_context* c,cudaStream_t st,const DevS
     {PhaseScope ps(c,PH_HESS,st);
         launch_hessian<P,false>(c,st,S2);counted(c,PH_HESS);}
     {PhaseScope ps(c,PH_CGNODE,st);
-        launch_dep(c,k_cg_q<P>,grid_for(c,c->node_grid),NODE_THREADS,0,st,S2);counted(c,PH_CGNODE);
         launch_dep(c,k_cg_update<P>,grid_for(c,c->node_grid),NODE_THREADS,0,st,S2,cond,use_cond,max_cg_iters(c)+1);counted(c,PH_CGNODE);}
 }
 

@@ -52,7 +52,8 @@ template<class T> struct SceneDev {
 // Per-scene solver state, written only by the last CTA of a reduction kernel.
 struct CGState {
     double rho;                // <r,r>_M of the current residual
-    double alpha,beta;
+    double beta;
+    double msq;                // <s,s>_M of the search direction r + beta s of the next trip
     double tol;                // absolute tolerance of this substep
     double residual;           // max-norm of the residual at the last check
     int iters;                 // completed CG iterations
@@ -61,7 +62,8 @@ struct CGState {
 };
 // Per-scene accumulators, zeroed by the consumer after use.
 struct SceneAcc {
-    double sum0,sum1;          // dot products
+    double sum[3];             // dot products of a node kernel
+    double sks;                // s^T K s, added up by the Hessian product of a loop trip
     unsigned long long max0;   // bit pattern of a non-negative double max
     unsigned long long count0;
 };

@@ -143,51 +143,129 @@ template<class T> __device__ __forceinline__ bool inside_barrier(const SceneDev<
 
 // ---------- per-scene reductions inside node kernels ----------
 struct SceneRed {
-    double sum[MAX_SCENES];
     unsigned long long mx[MAX_SCENES];
     unsigned long long cnt[MAX_SCENES];
 };
 __device__ __forceinline__ void red_init(SceneRed& R,int ns)
-{for(int i=threadIdx.x;i<ns;i+=blockDim.x){R.sum[i]=0.;R.mx[i]=0ull;R.cnt[i]=0ull;}}
+{for(int i=threadIdx.x;i<ns;i+=blockDim.x){R.mx[i]=0ull;R.cnt[i]=0ull;}}
 template<class TR> __device__ __forceinline__ TR warp_sum(TR v){for(int o=16;o>0;o>>=1) v+=__shfl_xor_sync(0xffffffffu,v,o);return v;}
 template<class TR> __device__ __forceinline__ TR warp_max(TR v){for(int o=16;o>0;o>>=1){TR u=__shfl_xor_sync(0xffffffffu,v,o);v=u>v?u:v;}return v;}
 __device__ __forceinline__ unsigned long long dbits(double x){return (unsigned long long)__double_as_longlong(x);}
 __device__ __forceinline__ double bitsd(unsigned long long b){return __longlong_as_double((long long)b);}
-// Flush the CTA's per-scene partials to the global accumulators, then let the last CTA
-// (ticket) run `fin` for every scene; fin sees complete sums. Returns true in every
-// thread of the last CTA.
-template<class F> __device__ __forceinline__ bool red_finish(SceneRed& R,int ns,SceneAcc* acc,unsigned* ticket,F fin,bool use_sum,bool use_max,bool use_cnt)
+// Flush the CTA's per-scene partials (maximum, and the count when asked for) to the global
+// accumulators, then let the last of the `parts` CTAs that take part (ticket) run `fin` for
+// every scene; fin sees complete values. Returns true in every thread of that CTA.
+template<bool USE_CNT,class F> __device__ __forceinline__ bool red_finish(SceneRed& R,int ns,SceneAcc* acc,unsigned* ticket,unsigned parts,F fin)
 {
     __syncthreads();
     for(int i=threadIdx.x;i<ns;i+=blockDim.x){
-        if(use_sum&&R.sum[i]!=0.) atomicAdd(&acc[i].sum0,R.sum[i]);
-        if(use_max&&R.mx[i]) atomicMax(&acc[i].max0,R.mx[i]);
-        if(use_cnt&&R.cnt[i]) atomicAdd(&acc[i].count0,R.cnt[i]);}
+        if(R.mx[i]) atomicMax(&acc[i].max0,R.mx[i]);
+        if(USE_CNT&&R.cnt[i]) atomicAdd(&acc[i].count0,R.cnt[i]);}
     __threadfence();
     __shared__ bool last;
     __syncthreads();
-    if(threadIdx.x==0) last=(atomicAdd(ticket,1u)==gridDim.x-1);
+    if(threadIdx.x==0) last=(atomicAdd(ticket,1u)==parts-1u);
     __syncthreads();
     if(!last) return false;
     __threadfence();
     for(int i=threadIdx.x;i<ns;i+=blockDim.x){
         volatile SceneAcc* a=acc+i;
-        const double s=a->sum0;const unsigned long long m=a->max0,c=a->count0;
-        a->sum0=0.;a->max0=0ull;a->count0=0ull;
-        fin(i,s,bitsd(m),c);}
+        const unsigned long long m=a->max0,c=a->count0;
+        a->max0=0ull;a->count0=0ull;
+        fin(i,bitsd(m),c);}
     __syncthreads();
     if(threadIdx.x==0) *ticket=0u;
+    return true;
+}
+// CTAs of the grid that get any of `work` items when each takes `per` at least; at least one
+// (it runs the reduction's end). The others return at once: with a small scene's few dozen
+// blocks, hundreds of CTAs would otherwise pass through the one ticket.
+__device__ __forceinline__ unsigned taking_part(long long work,long long per)
+{
+    const long long n=(work+per-1)/per;
+    return (unsigned)(n<1?1:n<(long long)gridDim.x?n:(long long)gridDim.x);
+}
+
+// A running sum per lane for the node kernels. FP32 terms go into an unevaluated pair by TwoSum
+// (48 bits): an FP64 addition and its conversion take the FP64 pipe, at 1/64 of the FP32
+// rate, longer than the node's memory traffic takes.
+template<class T> struct NodeSum { T h=T(0);
+    __device__ __forceinline__ void add(T x){h+=x;}
+    __device__ __forceinline__ double value() const {return h;} };
+template<> struct NodeSum<float> { float h=0.f,l=0.f;
+    __device__ __forceinline__ void add(float x)
+    {const float s=__fadd_rn(h,x),z=__fadd_rn(s,-h);l+=__fadd_rn(__fadd_rn(h,-__fadd_rn(s,-z)),__fadd_rn(x,-z));h=s;}
+    __device__ __forceinline__ double value() const {return (double)h+(double)l;} };
+// The reduction of kernels whose warps walk contiguous block ranges: a warp's last scene goes
+// into its slot here, an earlier one (rare) straight to the accumulators; one warp joins the
+// slots (mostly one scene) and adds them. Against per-scene shared arrays this spares a
+// small scene the shared FP64 atomics and the loops over all scenes.
+struct WarpParts { int scene[NODE_THREADS/32]; double sum[NODE_THREADS/32][3]; double mx[NODE_THREADS/32]; };
+template<int NS> __device__ __forceinline__ void add_scene(SceneAcc* acc,int sc,const double* s,double mx)
+{
+#pragma unroll
+    for(int k=0;k<NS;++k) if(s[k]!=0.) atomicAdd(&acc[sc].sum[k],s[k]);
+    if(mx>0.) atomicMax(&acc[sc].max0,dbits(mx));
+}
+template<int NS> __device__ __forceinline__ void flush_scene(WarpParts& W,SceneAcc* acc,int sc,bool last,double a,double b,double c,double mx)
+{
+    const double s[3]={warp_sum<double>(a),NS>1?warp_sum<double>(b):0.,NS>2?warp_sum<double>(c):0.},m=warp_max<double>(mx);
+    if((threadIdx.x&31)!=0) return;
+    if(!last){add_scene<NS>(acc,sc,s,m);return;}
+    const int w=threadIdx.x>>5;
+    W.scene[w]=sc;W.mx[w]=m;
+#pragma unroll
+    for(int k=0;k<NS;++k) W.sum[w][k]=s[k];
+}
+// As red_finish. Every warp has flushed its last scene (-1: none) into W.
+template<int NS,class F> __device__ __forceinline__ bool parts_finish(const WarpParts& W,int ns,SceneAcc* acc,unsigned* ticket,unsigned parts,F fin)
+{
+    __shared__ bool last;
+    __syncthreads();
+    if(threadIdx.x<32){
+        const int w=threadIdx.x,nw=blockDim.x>>5;
+        const int sc=w<nw?W.scene[w]:-1;
+        double s[3]={0.,0.,0.},m=0.;
+        if(sc>=0){
+#pragma unroll
+            for(int k=0;k<NS;++k) s[k]=W.sum[w][k];
+            m=W.mx[w];}
+        const unsigned any=__ballot_sync(0xffffffffu,sc>=0);
+        const int sc0=__shfl_sync(0xffffffffu,sc,any?__ffs(any)-1:0);
+        if(__all_sync(0xffffffffu,sc<0||sc==sc0)){
+            for(int o=NODE_THREADS/64;o>0;o>>=1){
+#pragma unroll
+                for(int k=0;k<NS;++k) s[k]+=__shfl_xor_sync(0xffffffffu,s[k],o);
+                m=fmax(m,__shfl_xor_sync(0xffffffffu,m,o));}
+            if(w==0&&any) add_scene<NS>(acc,sc0,s,m);}
+        else if(sc>=0) add_scene<NS>(acc,sc,s,m);
+        __threadfence();
+        __syncwarp();
+        if(w==0){last=(atomicAdd(ticket,1u)==parts-1u);if(last) *ticket=0u;}}
+    __syncthreads();
+    if(!last) return false;
+    __threadfence();
+    for(int i=threadIdx.x;i<ns;i+=blockDim.x){
+        volatile SceneAcc* a=acc+i;
+        double s[3]={0.,0.,0.};
+#pragma unroll
+        for(int k=0;k<NS;++k){s[k]=a->sum[k];a->sum[k]=0.;}
+        const unsigned long long m=a->max0;
+        a->max0=0ull;
+        fin(i,s,bitsd(m));}
     return true;
 }
 
 // A warp's contiguous share [b, b1) of nb node blocks.
 struct WarpRange {
     int b,b1;
+    unsigned parts;          // CTAs with a block
     __device__ __forceinline__ explicit WarpRange(int nb)
     {
         const int nw=(int)(gridDim.x*(blockDim.x>>5)),gw=(int)(blockIdx.x*(blockDim.x>>5)+(threadIdx.x>>5));
         const int per=(nb+nw-1)/nw;
         b=gw*per<nb?gw*per:nb;b1=b+per<nb?b+per:nb;
+        parts=taking_part(nb,(long long)max(per,1)*(blockDim.x>>5));
     }
 };
 // Exclusive prefix sum of one int per thread over the CTA (any blockDim up to 1024);
@@ -220,6 +298,12 @@ template<class T> __device__ __forceinline__ void build_active_list(const DevSta
     const int i=threadIdx.x;
     int act=0,nc=0,nb=0;
     if(i<S.n_scenes&&!S.cg[i].done){const SceneRange r=S.srange[i];act=1;nc=r.c1-r.c0;nb=r.b1-r.b0;}
+    if(S.n_scenes==1){                               // no scans for a single scene
+        if(i==0){
+            ActiveList* L=S.alist;
+            L->scene[0]=0;L->cpre[0]=L->bpre[0]=0;L->n=act;
+            if(act){L->cpre[1]=nc;L->bpre[1]=nb;}}
+        return;}
     int na,ct,bt;
     const int pos=cta_scan_int(act,&na),cp=cta_scan_int(nc,&ct),bp=cta_scan_int(nb,&bt);
     ActiveList* L=S.alist;
@@ -267,13 +351,18 @@ template<class T> constexpr int hess_warp_smem_bytes(){return (XFER_THREADS/32)*
 // sit about two cells apart in this order (a full block has 8 particles per cell and the
 // lanes are chunk/32 particles apart), so their tile addresses, and for every stencil
 // offset the addresses of their nodes, fall in distinct banks.
-__device__ __forceinline__ unsigned char cell_rank_of(int l)
+struct CellRank { unsigned char rank[64],cell[64]; };     // rank of a cell, cell of a rank
+constexpr CellRank make_cell_rank()
 {
-    const int b=tile_addr(l&3,(l>>2)&3,l>>4)&31;
-    int k=0;
-    for(int m=0;m<64;++m){const int bm=tile_addr(m&3,(m>>2)&3,m>>4)&31;k+=(bm<b||(bm==b&&m<l));}
-    return (unsigned char)k;
+    CellRank r{};
+    for(int l=0;l<64;++l){
+        const int b=(l%4+TSY*((l/4)%4)+TSZ*(l/16))%32;
+        int k=0;
+        for(int m=0;m<64;++m){const int bm=(m%4+TSY*((m/4)%4)+TSZ*(m/16))%32;k+=(bm<b||(bm==b&&m<l))?1:0;}
+        r.rank[l]=(unsigned char)k;r.cell[k]=(unsigned char)l;}
+    return r;
 }
+static __device__ const CellRank cell_ranks=make_cell_rank();
 
 // Storage order of a work item. Pass q of a warp gives lane L the cell-ordered slot
 // k = L*stride + q (stride = ceil(np/32)), so the lanes of a warp sit about two cells
@@ -594,13 +683,11 @@ template<class P,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) 
     unsigned short* inv=reinterpret_cast<unsigned short*>(smem_raw+p2g_tile_bytes<T>()+NW*64*4);
     unsigned char* cellv=reinterpret_cast<unsigned char*>(inv+S.chunk);
     __shared__ unsigned char crank[64],cell_of[64];
-    if(threadIdx.x<64){                                                // read after the next barrier
-        const unsigned char r=cell_rank_of(threadIdx.x);
-        crank[threadIdx.x]=r;cell_of[r]=(unsigned char)threadIdx.x;}
     __shared__ int nbr[27];
     __shared__ int run[129];
     const int warp=threadIdx.x>>5;
     const unsigned nc=min(S.ctr->n_chunks,(unsigned)S.chunk_cap),nv=S.ctr->n_valid;
+    if(threadIdx.x<64){crank[threadIdx.x]=cell_ranks.rank[threadIdx.x];cell_of[threadIdx.x]=cell_ranks.cell[threadIdx.x];}   // read after the next barrier
     for(long long c=blockIdx.x;c<nc;c+=gridDim.x){
         ChunkInfo<T> ci;
         load_chunk(S,c,nc,nv,ci,nbr);
@@ -740,9 +827,11 @@ template<class T> __global__ void __launch_bounds__(NODE_THREADS) k_grid_update(
 {
     pdl_enter();
     __shared__ SceneRed R;
+    const long long nn=(long long)min(S.ctr->n_active,(unsigned)S.block_cap)*64;
+    const unsigned parts=taking_part(nn,blockDim.x);
+    if(blockIdx.x>=parts) return;
     red_init(R,S.n_scenes);
     __syncthreads();
-    const long long nn=(long long)min(S.ctr->n_active,(unsigned)S.block_cap)*64;
     const V4<T> z={T(0),T(0),T(0),T(0)};
     for(long long n=blockIdx.x*(long long)blockDim.x+threadIdx.x;n<nn;n+=(long long)gridDim.x*blockDim.x){
         const int blk=(int)(n>>6);
@@ -782,11 +871,11 @@ template<class T> __global__ void __launch_bounds__(NODE_THREADS) k_grid_update(
         const unsigned wc=warp_sum<unsigned>(cnt);
         if((threadIdx.x&31)==0){if(wmax>0.) atomicMax(&R.mx[scene],dbits(wmax));if(wc) atomicAdd(&R.cnt[scene],(unsigned long long)wc);}
     }
-    red_finish(R,S.n_scenes,S.acc2,&S.ctr->ticket[0],[&](int i,double,double mx,unsigned long long cnt){
+    red_finish<true>(R,S.n_scenes,S.acc2,&S.ctr->ticket[0],parts,[&](int i,double mx,unsigned long long cnt){
         const SceneDev<T>& sc=S.scenes[i];CGState& st=S.cg[i];
         st.tol=fmax(sc.cg_abs_tol,sc.cg_rel_tol*sqrt(mx));
-        st.rho=0.;st.alpha=0.;st.beta=0.;st.residual=0.;st.iters=0;st.done=0;st.converged=0;st.n_interior=(int)cnt;
-    },false,true,true);
+        st.rho=0.;st.beta=0.;st.msq=0.;st.residual=0.;st.iters=0;st.done=0;st.converged=0;st.n_interior=(int)cnt;
+    });
 }
 
 // =====================================================================================
@@ -795,10 +884,11 @@ template<class T> __global__ void __launch_bounds__(NODE_THREADS) k_grid_update(
 // (V0 Fe dP^T)^T grad w_i. The gathered vector is x (FROM_X, for r = b - A x) or the new
 // search direction s = r + beta s_old, formed on the fly from r and the old s.
 // =====================================================================================
-// B = V0 dP Fe^T from G, by columns (HessianData in mpm_math.cuh). FP32 solves the 3x3 system
+// B = V0 dP Fe^T from G, by columns (HessianData in mpm_math.cuh), and bg = B:G, the particle's
+// part of s^T K s. FP32 solves the 3x3 system
 // of the rotation part here; FP64, whose arithmetic is 64 times slower against the same
 // memory, reads the inverse that P2G stored.
-template<class T> __device__ __forceinline__ void hessian_stress(const C3<T> (&G)[3],const T* Sm,T c1,T c2,T cc3,const T* Ki,C3<T> (&B)[3])
+template<class T> __device__ __forceinline__ void hessian_stress(const C3<T> (&G)[3],const T* Sm,T c1,T c2,T cc3,const T* Ki,C3<T> (&B)[3],T& bg)
 {
     const T S[3][3]={{Sm[0],Sm[1],Sm[2]},{Sm[1],Sm[3],Sm[4]},{Sm[2],Sm[4],Sm[5]}};
     C3<T> M[3];
@@ -814,6 +904,9 @@ template<class T> __device__ __forceinline__ void hessian_stress(const C3<T> (&G
     for(int j=0;j<3;++j)
         B[j]=madd(N[2],c1*S[2][j],madd(N[1],c1*S[1][j],madd(N[0],c1*S[0][j],mul(gt[j],-cc3))));
     B[0]=c3<T>(cx(B[0])+tr,cy(B[0]),B[0].z);B[1]=c3<T>(cx(B[1]),cy(B[1])+tr,B[1].z);B[2]=c3<T>(cx(B[2]),cy(B[2]),B[2].z+tr);
+    bg=T(0);
+#pragma unroll
+    for(int j=0;j<3;++j) bg+=cx(B[j])*cx(G[j])+cy(B[j])*cy(G[j])+B[j].z*G[j].z;
 }
 
 // FP64: one pass of a work item gives lane L the cell-ordered particle L*stride + qi (stored
@@ -821,7 +914,7 @@ template<class T> __device__ __forceinline__ void hessian_stress(const C3<T> (&G
 // vector tile sv, forms B and scatters B grad w into the warp's private tile in rounds of
 // lanes in distinct cells. Called by every lane of the warp.
 __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const SceneDev<double>& sc,int s,const int* run,int qi,int stride,int np,
-    const double (*sv)[TILE_S],double (*tile)[TILE_S])
+    const double (*sv)[TILE_S],double (*tile)[TILE_S],double& sks)
 {
     using T=double;
     const int j=(int)(threadIdx.x&31)*stride+qi;
@@ -838,7 +931,8 @@ __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const Sce
         stencil_from_coord(sc,cell,x,st);
         C3<T> G[3];
         gather_grad(st,sv,G);
-        hessian_stress<T>(G,Sm,q0.w,q2.z,q2.w,Ki,B);}
+        T bg;hessian_stress<T>(G,Sm,q0.w,q2.z,q2.w,Ki,B,bg);
+        sks+=bg;}
     const ScatterRounds R(valid,cell);
     for(int r=0;r<R.rounds;++r){
         const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
@@ -888,7 +982,7 @@ __device__ __forceinline__ void bspline_weights2(float2 x,float2 inv_dx,float2 (
     dw[2]=pmul(padd(y,th),inv_dx);
 }
 // B = V0 dP Fe^T from G for two particles (hessian_stress).
-__device__ __forceinline__ void hessian_stress2(const float2 (&G)[3][3],const float2 (&Sm)[6],float2 c1,float2 c2,float2 cc3,float2 (&B)[3][3])
+__device__ __forceinline__ void hessian_stress2(const float2 (&G)[3][3],const float2 (&Sm)[6],float2 c1,float2 c2,float2 cc3,float2 (&B)[3][3],float2& bg)
 {
     const int ix[3][3]={{0,1,2},{1,3,4},{2,4,5}};
     float2 M[3][3];
@@ -916,7 +1010,8 @@ __device__ __forceinline__ void hessian_stress2(const float2 (&G)[3][3],const fl
 #pragma unroll
         for(int j=0;j<3;++j){
             const float2 g=i==j?pfma(n3,G[j][i],tr):pmul(n3,G[j][i]);
-            B[i][j]=pfma(M[i][2],cS[ix[2][j]],pfma(M[i][1],cS[ix[1][j]],pfma(M[i][0],cS[ix[0][j]],g)));}
+            B[i][j]=pfma(M[i][2],cS[ix[2][j]],pfma(M[i][1],cS[ix[1][j]],pfma(M[i][0],cS[ix[0][j]],g)));
+            bg=i==0&&j==0?pmul(B[i][j],G[i][j]):pfma(B[i][j],G[i][j],bg);}
 }
 __device__ __forceinline__ void copy_pair(const DevState<float>& S,int s,unsigned entry,V4<float> (*slots)[32])
 {
@@ -931,7 +1026,7 @@ __device__ __forceinline__ void copy_pair(const DevState<float>& S,int s,unsigne
 }
 // The passes m0, m0 + dm, ... (pair index of the pass's first lane) of a work item of M pairs.
 __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const SceneDev<float>& sc,int s,int M,int m0,int dm,
-    const float (*sv)[TILE_S],float (*tile)[TILE_S],V4<float> (*slots)[32])
+    const float (*sv)[TILE_S],float (*tile)[TILE_S],V4<float> (*slots)[32],double& sks)
 {
     const unsigned* tab=S.pairs+s;
     const int lane=threadIdx.x&31;
@@ -975,8 +1070,10 @@ __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const Sce
             const float2 Sm[6]={make_float2(p1.x,q1.x),make_float2(p1.y,q1.y),make_float2(p1.z,q1.z),
                                 make_float2(p1.w,q1.w),make_float2(p2.x,q2.x),make_float2(p2.y,q2.y)};
             const bool two=(entry&PAIR_TWO)!=0u;                    // no second particle: no force
+            float2 bg;
             hessian_stress2(G,Sm,make_float2(slots[0][lane].w,two?slots[3][lane].w:0.f),make_float2(p2.z,two?q2.z:0.f),
-                            make_float2(p2.w,two?q2.w:0.f),B);
+                            make_float2(p2.w,two?q2.w:0.f),B,bg);
+            sks+=(double)(bg.x+bg.y);
             weights(w,dw);}
         entry=next;
         if(m+dm+lane<M) copy_pair(S,s,entry,slots);
@@ -1077,27 +1174,35 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
     __shared__ unsigned tmap[TILE_N];
     __shared__ ListSmem lsm;
     const int warp=threadIdx.x>>5,lane=threadIdx.x&31;
-    const unsigned nc=min(S.ctr->n_chunks,(unsigned)S.chunk_cap);
+    // the first product (FROM_X) covers every work item; a loop trip only the work items of
+    // the scenes still iterating (the list the previous convergence check wrote)
+    const long long nwork=FROM_X?(long long)min(S.ctr->n_chunks,(unsigned)S.chunk_cap):S.alist->cpre[S.alist->n];
+    if(form==HESS_AUTO) form=nwork>=warp_min?HESS_WARP:HESS_CTA;
+    if((form==HESS_CTA?(long long)blockIdx.x:(long long)blockIdx.x*NW)>=nwork) return;     // no item for this CTA
     auto tile_of=[&](int w){return reinterpret_cast<T (*)[TILE_S]>(smem_raw+w*hess_warp_bytes<T>());};   // [component][node]
     T (*q)[TILE_S]=tile_of(warp);                  // accumulated
     V4<float> (*slots)[32]=reinterpret_cast<V4<float> (*)[32]>(smem_raw+warp*hess_warp_bytes<T>()+6*TILE_S*sizeof(T));
     for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x) tmap[t]=tile_map_entry(t);
     for(int t=lane;t<3*TILE_S;t+=32) (&q[0][0])[t]=T(0);
-    // the first product (FROM_X) covers every work item; a loop trip only the work items of
-    // the scenes still iterating (the list the previous convergence check wrote)
-    long long nwork=nc;
-    if(!FROM_X){load_active_list(S.alist,lsm,false);nwork=lsm.pre[lsm.n];}
+    if(!FROM_X) load_active_list(S.alist,lsm,false);
     __syncthreads();
     auto item=[&](long long w){
         if(FROM_X) return w;
         const int j=list_find(lsm,(int)w);return S.srange[lsm.scene[j]].c0+(w-lsm.pre[j]);};
-    if(form==HESS_AUTO) form=nwork>=warp_min?HESS_WARP:HESS_CTA;
+    // s^T K s of a loop trip (k_cg_update), per lane until the warp's scene changes
+    double sks=0.;int sks_scene=-1;
+    auto add_sks=[&](int next){
+        if(!FROM_X&&sks_scene>=0&&sks_scene!=next){
+            const double v=warp_sum<double>(sks);
+            if(lane==0&&v!=0.) atomicAdd(&S.acc[sks_scene].sks,v);
+            sks=0.;}
+        sks_scene=next;};
     // the passes of an item: pairs (FP32) or cell-ordered particles (FP64), `first` of every `of`
     auto passes=[&](const SceneDev<T>& sc,const int* rec,const T (*sv)[TILE_S],int* run,int first,int of){
-        if constexpr(sizeof(T)==4) hessian_pairs(S,sc,rec[ITEM_START],rec[ITEM_PAIRS],first*32,of*32,sv,q,slots);
+        if constexpr(sizeof(T)==4) hessian_pairs(S,sc,rec[ITEM_START],rec[ITEM_PAIRS],first*32,of*32,sv,q,slots,sks);
         else{
             const int np=rec[ITEM_COUNT],stride=(np+31)>>5;
-            for(int qi=first;qi<stride;qi+=of) hessian_pass(S,sc,rec[ITEM_START],run,qi,stride,np,sv,q);}};
+            for(int qi=first;qi<stride;qi+=of) hessian_pass(S,sc,rec[ITEM_START],run,qi,stride,np,sv,q,sks);}};
     auto flush=[&](const int* rec,unsigned e,T v0,T v1,T v2){
         if(v0==T(0)&&v1==T(0)&&v2==T(0)) return;
         const int blk=rec[ITEM_NBR+(e&31u)];
@@ -1114,6 +1219,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
             stage_vector<P,FROM_X,XFER_THREADS>(S,rec+ITEM_NBR,tmap,FROM_X?T(0):(T)S.cg[scene].beta,sv,threadIdx.x);
             if constexpr(sizeof(T)==8) if(warp==0) chunk_runs(rec[ITEM_COUNT],(rec[ITEM_COUNT]+31)>>5,run);
             __syncthreads();
+            add_sks(scene);
             passes(S.scenes[scene],rec,sv,run,warp,NW);
             __syncthreads();
             for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x){
@@ -1141,6 +1247,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
             stage_vector<P,FROM_X,32>(S,rec+ITEM_NBR,tmap,FROM_X?T(0):(T)S.cg[scene].beta,sv,lane);
             if constexpr(sizeof(T)==8) chunk_runs(rec[ITEM_COUNT],(rec[ITEM_COUNT]+31)>>5,run);
             __syncwarp();
+            add_sks(scene);
             passes(S.scenes[scene],rec,sv,run,0,1);
             __syncwarp();
             for(int t=lane;t<TILE_N;t+=32){
@@ -1152,37 +1259,27 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
             __syncwarp();
         }
     }
+    add_sks(-1);
 }
 
-// Project (MPM_CG_System.h:220-225, intended semantics of Project_Helper.h:30-45).
-template<class T> __device__ __forceinline__ bool projected(const DevState<T>& S,const SceneDev<T>& sc,long long n,int blk)
-{
-    if(!sc.project||sc.n_barriers==0) return false;
-    T x[3];node_center(S,sc,n,blk,x);
-    for(int b=0;b<sc.n_barriers;++b) if(inside_barrier(sc,b,x)) return true;
-    return false;
-}
-
-// CG start: r = b - (x + dt^2/m K x), Project(r), then the first convergence check of the
+// CG start: r = b - (x + dt^2/m K x), Project(r) (MPM_CG_System.h:220-225, intended semantics of
+// Project_Helper.h:30-45; the grid update flagged the nodes), then the first convergence check of the
 // restated CG loop (iteration 0).
 template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_start(DevState<typename P::T> S,unsigned long long cond,int use_cond)
 {
     pdl_enter();
-    using T=typename P::T; using TR=typename P::TR;
-    __shared__ SceneRed R;
-    red_init(R,S.n_scenes);
-    __syncthreads();
+    using T=typename P::T;
+    __shared__ WarpParts W;
     const int na=(int)min(S.ctr->n_active,(unsigned)S.block_cap);
     const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
     const WarpRange wr(na);
-    int scene=-1;double acc=0.,amax=0.;
-    auto flush=[&](int sc){
-        const double ws=warp_sum<double>(acc),wm=warp_max<double>(amax);
-        if((threadIdx.x&31)==0){if(ws!=0.) atomicAdd(&R.sum[sc],ws);if(wm>0.) atomicMax(&R.mx[sc],dbits(wm));}
-        acc=0.;amax=0.;};
+    if(blockIdx.x>=wr.parts) return;
+    if((threadIdx.x&31)==0) W.scene[threadIdx.x>>5]=-1;
+    int scene=-1;NodeSum<T> rr;T amax=T(0);
+    auto flush=[&](int sc,bool last){flush_scene<1>(W,S.acc,sc,last,rr.value(),0.,0.,(double)amax);rr=NodeSum<T>();amax=T(0);};
     for(int blk=wr.b;blk<wr.b1;++blk){
         const int sb=S.active_scene[blk];
-        if(sb!=scene){if(scene>=0) flush(scene);scene=sb;}
+        if(sb!=scene){if(scene>=0) flush(scene,false);scene=sb;}
         T m[2];V4<T> x[2],b[2],k[2];unsigned char pj[2];
 #pragma unroll
         for(int h=0;h<2;++h){const long long n=((long long)blk<<6)+h*32+(threadIdx.x&31);m[h]=S.gm[n];x[h]=S.gx[n];b[h]=S.gr[n];k[h]=S.gf[n];pj[h]=S.gproj[n];}
@@ -1194,38 +1291,36 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_start(Dev
                 T r[3]={b[h].x-(c*k[h].x+x[h].x),b[h].y-(c*k[h].y+x[h].y),b[h].z-(c*k[h].z+x[h].z)};
                 if(pj[h]) r[0]=r[1]=r[2]=T(0);       // Project, flagged by the grid update
                 S.gr[n]=V4<T>{r[0],r[1],r[2],T(0)};
-                acc+=(double)(TR)(r[0]*(r[0]*m[h])+r[1]*(r[1]*m[h])+r[2]*(r[2]*m[h]));
-                const double cn=(double)(TR)(r[0]*r[0]+r[1]*r[1]+r[2]*r[2]);
+                rr.add(r[0]*(r[0]*m[h])+r[1]*(r[1]*m[h])+r[2]*(r[2]*m[h]));
+                const T cn=r[0]*r[0]+r[1]*r[1]+r[2]*r[2];
                 amax=cn>amax?cn:amax;}
             S.gf[n]=V4<T>{T(0),T(0),T(0),T(0)};}
     }
-    if(scene>=0) flush(scene);
+    if(scene>=0) flush(scene,true);
     __shared__ int any;
     if(threadIdx.x==0) any=0;
-    const bool last=red_finish(R,S.n_scenes,S.acc,&S.ctr->ticket[1],[&](int i,double rr,double mx,unsigned long long){
+    const bool last=parts_finish<1>(W,S.n_scenes,S.acc,&S.ctr->ticket[1],wr.parts,[&](int i,const double* sum,double mx){
         const SceneDev<T>& sc=S.scenes[i];CGState& st=S.cg[i];
-        const double cn=sqrt(mx);
+        const double cn=sqrt(mx),rr=sum[0];
         const double eps=sizeof(T)==4?1.1920928955078125e-07:2.220446049250313e-16;
         st.residual=cn;
         if(cn<=st.tol&&(0>=sc.cg_min_iters||cn<eps)){st.done=1;st.converged=1;}
         else if(sc.cg_max_iters<=0){st.done=1;st.converged=0;atomicOr(&S.ctr->error,ERR_CG_NOT_CONVERGED);}
-        else{st.rho=rr;st.beta=0.;atomicOr(&any,1);}
-    },true,true,false);
+        else{st.rho=rr;st.beta=0.;st.msq=rr;atomicOr(&any,1);}    // the first direction is r
+    });
     if(last) build_active_list(S);
     if(last&&threadIdx.x==0){
         S.ctr->any_active=any;S.ctr->loop_iters=0;
         if(use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond,any?1u:0u);}
 }
 
-// CG part 1: s = r + beta s_old (stored), q = s + dt^2/m K s, Project(q), <s,q>_M; the last
-// CTA forms alpha = rho/<s,q>.
 // A warp's share of the node blocks of the scenes in the list: a contiguous range of list
 // blocks, so that the warp meets each scene once and streams whole blocks (64 nodes, two
 // per lane). next() moves to list block bw (non-decreasing) and tells whether the scene
 // changed; node(h) is the lane's h-th node (h = 0, 1) of that block.
 struct WarpBlocks {
     int b,b1,j=0,scene=-1;long long base=0;
-    __device__ __forceinline__ explicit WarpBlocks(const ListSmem& sm){const WarpRange r(sm.pre[sm.n]);b=r.b;b1=r.b1;}
+    __device__ __forceinline__ explicit WarpBlocks(const WarpRange& r):b(r.b),b1(r.b1){}
     __device__ __forceinline__ bool next(const ListSmem& sm,const SceneRange* sr,int bw)
     {
         if(scene>=0&&bw<sm.pre[j+1]) return false;
@@ -1235,93 +1330,78 @@ struct WarpBlocks {
     }
     __device__ __forceinline__ long long node(int bw,int h) const {return ((base+bw)<<6)+h*32+(threadIdx.x&31);}
 };
-template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_q(DevState<typename P::T> S)
-{
-    pdl_enter();
-    using T=typename P::T; using TR=typename P::TR;
-    __shared__ SceneRed R;
-    __shared__ ListSmem lsm;
-    red_init(R,S.n_scenes);
-    load_active_list(S.alist,lsm,true);     // the scenes still iterating (its barrier orders red_init)
-    const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
-    WarpBlocks wb(lsm);
-    double acc=0.;T beta=T(0);
-    auto flush=[&](int sc){const double ws=warp_sum<double>(acc);if((threadIdx.x&31)==0&&ws!=0.) atomicAdd(&R.sum[sc],ws);acc=0.;};
-    for(int bw=wb.b;bw<wb.b1;++bw){
-        const int prev=wb.scene;
-        if(wb.next(lsm,S.srange,bw)){if(prev>=0) flush(prev);beta=(T)S.cg[wb.scene].beta;}
-        T m[2];V4<T> r[2],so[2],k[2];unsigned char pj[2];
-#pragma unroll
-        for(int h=0;h<2;++h){const long long n=wb.node(bw,h);m[h]=S.gm[n];r[h]=S.gr[n];so[h]=S.gs[n];k[h]=S.gf[n];pj[h]=S.gproj[n];}
-#pragma unroll
-        for(int h=0;h<2;++h){
-            if(!(m[h]>T(0))) continue;
-            const long long n=wb.node(bw,h);
-            const T s[3]={r[h].x+beta*so[h].x,r[h].y+beta*so[h].y,r[h].z+beta*so[h].z};
-            const T c=dt2/m[h];
-            T qv[3]={c*k[h].x+s[0],c*k[h].y+s[1],c*k[h].z+s[2]};
-            if(pj[h]) qv[0]=qv[1]=qv[2]=T(0);
-            S.gs[n]=V4<T>{s[0],s[1],s[2],T(0)};
-            S.gf[n]=V4<T>{qv[0],qv[1],qv[2],T(0)};
-            acc+=(double)(TR)(s[0]*(qv[0]*m[h])+s[1]*(qv[1]*m[h])+s[2]*(qv[2]*m[h]));}
-    }
-    if(wb.scene>=0) flush(wb.scene);
-    red_finish(R,S.n_scenes,S.acc,&S.ctr->ticket[2],[&](int i,double sq,double,unsigned long long){
-        CGState& st=S.cg[i];
-        if(st.done) return;
-        st.alpha=sq!=0.?st.rho/sq:(double)FLT_MAX;
-    },true,false,false);
-}
-
-// CG part 2: x += alpha s, r -= alpha q (Interior only), clear q for the next Hessian
-// action, then the convergence check: stop when max|r| <= tol (and iters >= min, or the
-// norm is below epsilon) or at cg_max_iters; else beta = <r,r>/rho, rho = <r,r>.
+// The vector update of a loop trip, one pass over the nodes: s = r + beta s_old, q = s +
+// dt^2/m K s, Project(q), x += alpha s, r -= alpha q (Interior only), K s cleared for the next
+// product. alpha = <r,r>_M / <s,q>_M needs no pass of its own over the nodes: <s,q>_M =
+// dt^2 s^T K s + <s,s>_M, of which the Hessian product adds up s^T K s over the particles
+// (sum of B:G) and the previous update <s,s>_M = <r,r> + 2 beta <r,s_old> + beta^2
+// <s_old,s_old> (s vanishes at projected nodes). Then the convergence check: stop when
+// max|r| <= tol (and iters >= min, or the norm is below epsilon) or at cg_max_iters; else beta
+// = <r,r>/rho, rho = <r,r>. Bound by memory on large scenes (133 bytes a node against 200 with a
+// separate q pass: 114 -> 85 us a trip on the 21.5M slab), by the latency of its chain of
+// reductions on small ones (22 -> 15 us).
 template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(DevState<typename P::T> S,unsigned long long cond,int use_cond,int max_trips)
 {
     pdl_enter();
-    using T=typename P::T; using TR=typename P::TR;
-    __shared__ SceneRed R;
+    using T=typename P::T;
+    __shared__ WarpParts W;
     __shared__ ListSmem lsm;
-    red_init(R,S.n_scenes);
-    load_active_list(S.alist,lsm,true);
-    WarpBlocks wb(lsm);
-    double acc=0.,amax=0.;T alpha=T(0);
-    auto flush=[&](int sc){
-        const double ws=warp_sum<double>(acc),wm=warp_max<double>(amax);
-        if((threadIdx.x&31)==0){if(ws!=0.) atomicAdd(&R.sum[sc],ws);if(wm>0.) atomicMax(&R.mx[sc],dbits(wm));}
-        acc=0.;amax=0.;};
+    const WarpRange wr(S.alist->bpre[S.alist->n]);
+    if(blockIdx.x>=wr.parts) return;
+    if((threadIdx.x&31)==0) W.scene[threadIdx.x>>5]=-1;
+    load_active_list(S.alist,lsm,true);     // the scenes still iterating
+    WarpBlocks wb(wr);
+    const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
+    NodeSum<T> rr,rs,ss;T amax=T(0),alpha=T(0),beta=T(0);
+    auto flush=[&](int sc,bool last){
+        flush_scene<3>(W,S.acc,sc,last,rr.value(),rs.value(),ss.value(),(double)amax);
+        rr=rs=ss=NodeSum<T>();amax=T(0);};
     for(int bw=wb.b;bw<wb.b1;++bw){
         const int prev=wb.scene;
-        if(wb.next(lsm,S.srange,bw)){if(prev>=0) flush(prev);alpha=(T)S.cg[wb.scene].alpha;}
-        T m[2];V4<T> s[2],qv[2],x[2],r[2];
+        if(wb.next(lsm,S.srange,bw)){
+            if(prev>=0) flush(prev,false);
+            const CGState& st=S.cg[wb.scene];
+            const double sq=(double)dt2*S.acc[wb.scene].sks+st.msq;
+            alpha=(T)(sq!=0.?st.rho/sq:(double)FLT_MAX);beta=(T)st.beta;}
+        T m[2];V4<T> s[2],k[2],x[2],r[2];unsigned char pj[2];
 #pragma unroll
-        for(int h=0;h<2;++h){const long long n=wb.node(bw,h);m[h]=S.gm[n];s[h]=S.gs[n];qv[h]=S.gf[n];x[h]=S.gx[n];r[h]=S.gr[n];}
+        for(int h=0;h<2;++h){const long long n=wb.node(bw,h);m[h]=S.gm[n];s[h]=S.gs[n];k[h]=S.gf[n];x[h]=S.gx[n];r[h]=S.gr[n];pj[h]=S.gproj[n];}
 #pragma unroll
         for(int h=0;h<2;++h){
             const long long n=wb.node(bw,h);
             if(m[h]>T(0)){
+                const T c=dt2/m[h];
+                s[h].x=r[h].x+beta*s[h].x;s[h].y=r[h].y+beta*s[h].y;s[h].z=r[h].z+beta*s[h].z;
+                T q[3]={c*k[h].x+s[h].x,c*k[h].y+s[h].y,c*k[h].z+s[h].z};
+                if(pj[h]) q[0]=q[1]=q[2]=T(0);
                 x[h].x=alpha*s[h].x+x[h].x;x[h].y=alpha*s[h].y+x[h].y;x[h].z=alpha*s[h].z+x[h].z;
-                r[h].x=-alpha*qv[h].x+r[h].x;r[h].y=-alpha*qv[h].y+r[h].y;r[h].z=-alpha*qv[h].z+r[h].z;
-                S.gx[n]=x[h];S.gr[n]=r[h];
-                acc+=(double)(TR)(r[h].x*(r[h].x*m[h])+r[h].y*(r[h].y*m[h])+r[h].z*(r[h].z*m[h]));
-                const double cn=(double)(TR)(r[h].x*r[h].x+r[h].y*r[h].y+r[h].z*r[h].z);
+                r[h].x=-alpha*q[0]+r[h].x;r[h].y=-alpha*q[1]+r[h].y;r[h].z=-alpha*q[2]+r[h].z;
+                S.gs[n]=s[h];S.gx[n]=x[h];S.gr[n]=r[h];
+                rr.add(r[h].x*(r[h].x*m[h])+r[h].y*(r[h].y*m[h])+r[h].z*(r[h].z*m[h]));
+                rs.add(r[h].x*(s[h].x*m[h])+r[h].y*(s[h].y*m[h])+r[h].z*(s[h].z*m[h]));
+                ss.add(s[h].x*(s[h].x*m[h])+s[h].y*(s[h].y*m[h])+s[h].z*(s[h].z*m[h]));
+                const T cn=(r[h].x*r[h].x+r[h].y*r[h].y+r[h].z*r[h].z);
                 amax=cn>amax?cn:amax;}
             S.gf[n]=V4<T>{T(0),T(0),T(0),T(0)};}
     }
-    if(wb.scene>=0) flush(wb.scene);
+    if(wb.scene>=0) flush(wb.scene,true);
     __shared__ int any;
     if(threadIdx.x==0) any=0;
-    const bool last=red_finish(R,S.n_scenes,S.acc,&S.ctr->ticket[3],[&](int i,double rr,double mx,unsigned long long){
+    const bool last=parts_finish<3>(W,S.n_scenes,S.acc,&S.ctr->ticket[3],wr.parts,[&](int i,const double* sum,double mx){
         const SceneDev<T>& sc=S.scenes[i];CGState& st=S.cg[i];
         if(st.done) return;
+        S.acc[i].sks=0.;
         st.iters+=1;
         const double cn=sqrt(mx);
         const double eps=sizeof(T)==4?1.1920928955078125e-07:2.220446049250313e-16;
         st.residual=cn;
         if(cn<=st.tol&&(st.iters>=sc.cg_min_iters||cn<eps)){st.done=1;st.converged=1;}
         else if(st.iters>=sc.cg_max_iters){st.done=1;st.converged=0;atomicOr(&S.ctr->error,ERR_CG_NOT_CONVERGED);}
-        else{st.beta=rr/st.rho;st.rho=rr;atomicOr(&any,1);}
-    },true,true,false);
+        else{
+            st.beta=sum[0]/st.rho;st.rho=sum[0];
+            st.msq=sum[0]+st.beta*(2.*sum[1]+st.beta*sum[2]);
+            atomicOr(&any,1);}
+    });
     if(last) build_active_list(S);
     if(last&&threadIdx.x==0){
         S.ctr->loop_iters+=1;S.ctr->total_trips+=1;
@@ -1467,6 +1547,8 @@ template<class T> __global__ void __launch_bounds__(NODE_THREADS) k_cfl(DevState
 {
     __shared__ SceneRed R;
     __shared__ unsigned long long dtbits;
+    const unsigned parts=taking_part(S.n_total,blockDim.x);
+    if(blockIdx.x>=parts) return;
     red_init(R,S.n_scenes);
     if(threadIdx.x==0) dtbits=dbits(F->dt_max);
     __syncthreads();
@@ -1479,11 +1561,11 @@ template<class T> __global__ void __launch_bounds__(NODE_THREADS) k_cfl(DevState
         for(int k=0;k<3;++k){const T v=S.pcur[(FV+k)*pc+i];a+=v*v;}
         const double v2=(double)a;
         if(v2>0.) atomicMax(&R.mx[s],dbits(v2));}
-    const bool last=red_finish(R,S.n_scenes,S.acc2,&S.ctr->ticket[4],[&](int i,double,double mx,unsigned long long){
+    const bool last=red_finish<false>(R,S.n_scenes,S.acc2,&S.ctr->ticket[4],parts,[&](int i,double mx,unsigned long long){
         const double vmax=sqrt(mx);
         const double dt=fmax(F->dt_min,fmin(F->dt_max,F->cfl*(double)S.scenes[i].dx[0]/fmax(vmax,1e-2)));
         atomicMin(&dtbits,dbits(dt));
-    },false,true,false);
+    });
     if(last&&threadIdx.x==0){
         double dt=bitsd(dtbits);
         const double rem=F->target-F->time;
