@@ -86,6 +86,7 @@ struct mpm_context {
     int xfer_grid=12;                        // transfer-kernel CTAs per SM (grid-stride over work items)
     int node_grid=4;                         // node-kernel (grid update, CG vectors) CTAs per SM
     int hess_warp=HESS_AUTO;                 // Hessian work items per CTA (0), per warp (1), or chosen per launch (2)
+    bool coop=false;                          // the device takes cooperative launches
     bool use_pdl=true;                       // substep kernels as programmatic dependents
     // timing
     bool timing=false;
@@ -262,7 +263,36 @@ template<class P> void enqueue_cg_body(mpm_context* c,cudaStream_t st,const DevS
         launch_dep(c,k_cg_update<P>,grid_for(c,c->node_grid),NODE_THREADS,0,st,S2,cond,use_cond,max_cg_iters(c)+1);counted(c,PH_CGNODE);}
 }
 
-// Everything of one substep before the CG loop. Returns the state with swapped buffers.
+// Whether a graph's substep solves in one cooperative kernel (k_cg_solve): one scene in FP32
+// storage, the Hessian's form left to the library, at most SOLVE_MAX particles. Substeps
+// measured as a loop of kernels -> one kernel: 3K particles 158 -> 128 us, 20K 295 -> 222,
+// 61K 345 -> 281, 237K 342 -> 328, 400K 499 -> 454, 1.2M 1,218 -> 1,174; from 2M on the
+// loop with a warp per work item is faster (1,820 against 1,905, at 4M 3,454 against 3,910).
+constexpr long long SOLVE_MAX=1LL<<20;
+template<class P> bool solve_in_one(const mpm_context* c)
+{
+    return sizeof(TT<P>)==4&&c->coop&&c->scenes.size()==1&&c->hess_warp==HESS_AUTO&&c->n_total<=SOLVE_MAX;
+}
+// CTAs of k_cg_solve: at most those that fit the GPU at once (the launch is cooperative); fewer
+// for few particles, where more would only take part in the barriers.
+template<class P> cudaError_t launch_solve(mpm_context* c,cudaStream_t st,const DevState<TT<P>>& S2)
+{
+    if constexpr(sizeof(TT<P>)==4){
+        const size_t smem=hess_kernel_smem_bytes<TT<P>>();
+        int per_sm=0;
+        cudaError_t e=cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,k_cg_solve<P>,XFER_THREADS,smem);
+        if(e!=cudaSuccess) return e;
+        cudaLaunchAttribute at[1];
+        at[0].id=cudaLaunchAttributeCooperative;at[0].val.cooperative=1;
+        cudaLaunchConfig_t cfg={};
+        cfg.gridDim=dim3((unsigned)std::min<long long>((long long)c->num_sms*std::max(per_sm,1),std::max<long long>(c->num_sms,c->n_total/128)));
+        cfg.blockDim=dim3(XFER_THREADS);cfg.dynamicSmemBytes=smem;cfg.stream=st;cfg.attrs=at;cfg.numAttrs=1;
+        return cudaLaunchKernelEx(&cfg,k_cg_solve<P>,S2,max_cg_iters(c)+1);}
+    else return cudaErrorNotSupported;
+}
+
+// Everything of one substep before the CG loop, up to the grid update with stop_after 1 or 2.
+// Returns the state with swapped buffers.
 template<class P> DevState<TT<P>> enqueue_pre(mpm_context* c,cudaStream_t st,int parity,double dt,unsigned long long cond,int use_cond,int stop_after)
 {
     DevState<TT<P>> S=make_state<P>(c,parity,dt);
@@ -353,6 +383,14 @@ mpm_status end_body_capture(mpm_context* c,cudaStream_t st_body)
 // body is captured on `st_body`. Kernel counts go to *outside and *body.
 template<class P> mpm_status capture_substep(mpm_context* c,cudaStream_t st,cudaStream_t st_body,int parity,double dt,long long* outside,long long* body)
 {
+    if(solve_in_one<P>(c)){
+        c->count_into=outside;
+        const DevState<TT<P>> S2=enqueue_pre<P>(c,st,parity,dt,0,0,2);
+        const cudaError_t e=launch_solve<P>(c,st,S2);
+        counted(c,PH_HESS);
+        if(e==cudaSuccess) enqueue_post<P>(c,st,S2);
+        c->count_into=nullptr;
+        return e==cudaSuccess?MPM_OK:fail(c,MPM_CUDA_ERROR,std::string("cooperative launch: ")+cudaGetErrorString(e));}
     cudaGraphConditionalHandle h;
     mpm_status s=capture_handle(c,st,0,&h);if(s!=MPM_OK) return s;
     c->count_into=outside;
@@ -467,6 +505,7 @@ mpm_status collect_status(mpm_context* c)
                     (b?" (highest scene index with one: "+std::to_string((int)b-1)+")":std::string()));}
     if(e&ERR_OUT_OF_GRID) return fail(c,MPM_BAD_ARG,"particle outside the grid; it was removed");
     if(e&ERR_SORT_WAIT) return fail(c,MPM_CUDA_ERROR,"sort look-back wait exceeded its limit");
+    if(e&ERR_GRID_WAIT) return fail(c,MPM_CUDA_ERROR,"CG grid barrier wait exceeded its limit");
     if(e&ERR_CG_NOT_CONVERGED) return MPM_CG_NOT_CONVERGED;
     return MPM_OK;
 }
@@ -820,6 +859,7 @@ mpm_status mpm_create(const mpm_config* cfg,mpm_context** out)
     cudaDeviceProp prop;
     if(cudaGetDeviceProperties(&prop,c0.device)!=cudaSuccess) return bail(MPM_CUDA_ERROR);
     c->num_sms=prop.multiProcessorCount;
+    {int v=0;if(cudaDeviceGetAttribute(&v,cudaDevAttrCooperativeLaunch,c0.device)==cudaSuccess) c->coop=v!=0;}
     {int v=0;if(cudaDeviceGetAttribute(&v,cudaDevAttrPageableMemoryAccess,c0.device)==cudaSuccess) c->pageable_access=v!=0;}
     if(const char* v=std::getenv("MPM_HOST_DIRECT")) c->host_direct=std::strcmp(v,"0")!=0;   // "0": always stage host arrays
     if(const char* v=std::getenv("MPM_PDL")) c->use_pdl=std::strcmp(v,"0")!=0;               // "0": plain stream order

@@ -86,7 +86,12 @@ struct ActiveList { int n; int scene[MAX_SCENES]; int cpre[MAX_SCENES+1]; int bp
 constexpr int ITEM_WORDS=32;
 enum { ITEM_START=0, ITEM_COUNT=1, ITEM_SCENE=2, ITEM_PAIRS=3, ITEM_NBR=4 };
 
+// Sums of one phase of k_cg_solve.
+struct SolveSlot { double sum[3]; unsigned long long max0; };
 struct Counters {
+    // zeroed before every substep (up to `error`)
+    SolveSlot solve[4];        // k_cg_solve, by phase mod 4
+    unsigned solve_arrived;    // its grid barrier: arrivals so far
     unsigned n_valid;          // valid particles after the key pass
     unsigned n_chunks;
     unsigned n_active;         // active node blocks
@@ -97,7 +102,7 @@ struct Counters {
     int loop_iters;            // CG loop trips this substep
     unsigned long long total_trips;   // CG loop trips since the context was created
 };
-enum { ERR_CAPACITY=1u, ERR_NONFINITE=2u, ERR_OUT_OF_GRID=4u, ERR_CG_NOT_CONVERGED=8u, ERR_SORT_WAIT=16u };
+enum { ERR_CAPACITY=1u, ERR_NONFINITE=2u, ERR_OUT_OF_GRID=4u, ERR_CG_NOT_CONVERGED=8u, ERR_SORT_WAIT=16u, ERR_GRID_WAIT=32u };
 
 // Device-side time stepping of mpm_advance_to_time: the reference's CFL rule and
 // end-of-frame split (MPM_Driver.cpp:55-80), evaluated on the device before every substep.

@@ -1024,14 +1024,19 @@ __device__ __forceinline__ void copy_pair(const DevState<float>& S,int s,unsigne
             const unsigned d=(unsigned)__cvta_generic_to_shared(&slots[3*h+k][lane]);
             asm volatile("cp.async.cg.shared.global [%0],[%1],16;"::"r"(d),"l"(p+k*S.pcap):"memory");}}
 }
+// A single pass that a warp runs again and again (k_cg_solve): once copied, its pairs stay in
+// the warp's slots and its entry here.
+struct PairPass { unsigned entry=0u; bool ready=false; };
 // The passes m0, m0 + dm, ... (pair index of the pass's first lane) of a work item of M pairs.
 __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const SceneDev<float>& sc,int s,int M,int m0,int dm,
-    const float (*sv)[TILE_S],float (*tile)[TILE_S],V4<float> (*slots)[32],double& sks)
+    const float (*sv)[TILE_S],float (*tile)[TILE_S],V4<float> (*slots)[32],double& sks,
+    PairPass& pass)
 {
     const unsigned* tab=S.pairs+s;
     const int lane=threadIdx.x&31;
-    unsigned entry=0,next=0;
-    if(m0+lane<M){entry=tab[m0+lane];copy_pair(S,s,entry,slots);}
+    unsigned entry=pass.entry,next=0;
+    if(!pass.ready&&m0+lane<M){entry=tab[m0+lane];copy_pair(S,s,entry,slots);}
+    pass.entry=entry;pass.ready=m0+dm>=M;
     if(m0+dm+lane<M) next=tab[m0+dm+lane];
     for(int m=m0;m<M;m+=dm){
         const bool valid=m+lane<M;
@@ -1137,10 +1142,9 @@ __device__ __forceinline__ unsigned tile_map_entry(int t)
 }
 // The gathered vector at the item's tile nodes, by NT threads: the loads of a batch of nodes
 // are all issued before one is used (a node's address needs only the item record).
-template<class P,bool FROM_X,int NT> __device__ __forceinline__ void stage_vector(const DevState<typename P::T>& S,const int* nbr,const unsigned* tmap,
-    typename P::T beta,typename P::T (*sv)[TILE_S],int tid)
+template<class T,int NT> __device__ __forceinline__ void stage_vector(const DevState<T>& S,const int* nbr,const unsigned* tmap,bool from_x,
+    T beta,T (*sv)[TILE_S],int tid)
 {
-    using T=typename P::T;
     constexpr int IT=(TILE_N+NT-1)/NT,BATCH=sizeof(T)==8?1:IT;
 #pragma unroll
     for(int i0=0;i0<IT;i0+=BATCH){
@@ -1155,13 +1159,20 @@ template<class P,bool FROM_X,int NT> __device__ __forceinline__ void stage_vecto
                 const int blk=nbr[e&31u];
                 if(blk>=0){
                     const long long node=(long long)blk*64+((e>>5)&63u);
-                    if(FROM_X) a[i]=S.gx[node];
+                    if(from_x) a[i]=S.gx[node];
                     else{a[i]=S.gr[node];b[i]=S.gs[node];}}}}
 #pragma unroll
         for(int i=0;i<BATCH;++i) if(ta[i]!=~0u){
-            sv[0][ta[i]]=FROM_X?a[i].x:a[i].x+beta*b[i].x;
-            sv[1][ta[i]]=FROM_X?a[i].y:a[i].y+beta*b[i].y;
-            sv[2][ta[i]]=FROM_X?a[i].z:a[i].z+beta*b[i].z;}}
+            sv[0][ta[i]]=from_x?a[i].x:a[i].x+beta*b[i].x;
+            sv[1][ta[i]]=from_x?a[i].y:a[i].y+beta*b[i].y;
+            sv[2][ta[i]]=from_x?a[i].z:a[i].z+beta*b[i].z;}}
+}
+// Adds an item's sum at a tile node to the grid.
+template<class T> __device__ __forceinline__ void add_tile_node(const DevState<T>& S,const int* rec,unsigned e,T v0,T v1,T v2)
+{
+    if(v0==T(0)&&v1==T(0)&&v2==T(0)) return;
+    const int blk=rec[ITEM_NBR+(e&31u)];
+    if(blk>=0) atomic_add_v3(S.gf+(long long)blk*64+((e>>5)&63u),v0,v1,v2,T(0));
 }
 template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) k_hessian(DevState<typename P::T> S,int form,long long warp_min)
 {
@@ -1199,14 +1210,10 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
         sks_scene=next;};
     // the passes of an item: pairs (FP32) or cell-ordered particles (FP64), `first` of every `of`
     auto passes=[&](const SceneDev<T>& sc,const int* rec,const T (*sv)[TILE_S],int* run,int first,int of){
-        if constexpr(sizeof(T)==4) hessian_pairs(S,sc,rec[ITEM_START],rec[ITEM_PAIRS],first*32,of*32,sv,q,slots,sks);
+        if constexpr(sizeof(T)==4){PairPass pass;hessian_pairs(S,sc,rec[ITEM_START],rec[ITEM_PAIRS],first*32,of*32,sv,q,slots,sks,pass);}
         else{
             const int np=rec[ITEM_COUNT],stride=(np+31)>>5;
             for(int qi=first;qi<stride;qi+=of) hessian_pass(S,sc,rec[ITEM_START],run,qi,stride,np,sv,q,sks);}};
-    auto flush=[&](const int* rec,unsigned e,T v0,T v1,T v2){
-        if(v0==T(0)&&v1==T(0)&&v2==T(0)) return;
-        const int blk=rec[ITEM_NBR+(e&31u)];
-        if(blk>=0) atomic_add_v3(S.gf+(long long)blk*64+((e>>5)&63u),v0,v1,v2,T(0));};
     if(form==HESS_CTA){
         T (*sv)[TILE_S]=tile_of(0)+3;
         int* rec=rec_s[0];int* run=run_s[0];
@@ -1216,7 +1223,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
             __syncthreads();
             if(w+gridDim.x<nwork) mine=S.items[item(w+gridDim.x)*ITEM_WORDS+lane];
             const int scene=rec[ITEM_SCENE];
-            stage_vector<P,FROM_X,XFER_THREADS>(S,rec+ITEM_NBR,tmap,FROM_X?T(0):(T)S.cg[scene].beta,sv,threadIdx.x);
+            stage_vector<T,XFER_THREADS>(S,rec+ITEM_NBR,tmap,FROM_X,FROM_X?T(0):(T)S.cg[scene].beta,sv,threadIdx.x);
             if constexpr(sizeof(T)==8) if(warp==0) chunk_runs(rec[ITEM_COUNT],(rec[ITEM_COUNT]+31)>>5,run);
             __syncthreads();
             add_sks(scene);
@@ -1230,7 +1237,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
 #pragma unroll
                     for(int w2=0;w2<NW;++w2){T* p=&tile_of(w2)[ch][e>>11];a+=*p;*p=T(0);}
                     v[ch]=a;}
-                flush(rec,e,v[0],v[1],v[2]);}
+                add_tile_node(S,rec,e,v[0],v[1],v[2]);}
             __syncthreads();
         }
     }
@@ -1244,7 +1251,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
             __syncwarp();
             if(w+dw<nwork) mine=S.items[item(w+dw)*ITEM_WORDS+lane];
             const int scene=rec[ITEM_SCENE];
-            stage_vector<P,FROM_X,32>(S,rec+ITEM_NBR,tmap,FROM_X?T(0):(T)S.cg[scene].beta,sv,lane);
+            stage_vector<T,32>(S,rec+ITEM_NBR,tmap,FROM_X,FROM_X?T(0):(T)S.cg[scene].beta,sv,lane);
             if constexpr(sizeof(T)==8) chunk_runs(rec[ITEM_COUNT],(rec[ITEM_COUNT]+31)>>5,run);
             __syncwarp();
             add_sks(scene);
@@ -1255,16 +1262,61 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
                 T* p=&q[0][e>>11];
                 const T v0=p[0],v1=p[TILE_S],v2=p[2*TILE_S];
                 p[0]=p[TILE_S]=p[2*TILE_S]=T(0);
-                flush(rec,e,v0,v1,v2);}
+                add_tile_node(S,rec,e,v0,v1,v2);}
             __syncwarp();
         }
     }
     add_sks(-1);
 }
 
-// CG start: r = b - (x + dt^2/m K x), Project(r) (MPM_CG_System.h:220-225, intended semantics of
-// Project_Helper.h:30-45; the grid update flagged the nodes), then the first convergence check of the
-// restated CG loop (iteration 0).
+// r = b - (x + dt^2/m K x) on a node block, two nodes per lane, Project(r) (MPM_CG_System.h:
+// 220-225, intended semantics of Project_Helper.h:30-45; the grid update flagged the nodes),
+// K x cleared; <r,r>_M and max|r|^2.
+template<class T> __device__ __forceinline__ void cg_start_block(const DevState<T>& S,int blk,T dt2,NodeSum<T>& rr,T& amax)
+{
+    T m[2];V4<T> x[2],b[2],k[2];unsigned char pj[2];
+#pragma unroll
+    for(int h=0;h<2;++h){const long long n=((long long)blk<<6)+h*32+(threadIdx.x&31);m[h]=S.gm[n];x[h]=S.gx[n];b[h]=S.gr[n];k[h]=S.gf[n];pj[h]=S.gproj[n];}
+#pragma unroll
+    for(int h=0;h<2;++h){
+        const long long n=((long long)blk<<6)+h*32+(threadIdx.x&31);
+        if(m[h]>T(0)){
+            const T c=dt2/m[h];
+            T r[3]={b[h].x-(c*k[h].x+x[h].x),b[h].y-(c*k[h].y+x[h].y),b[h].z-(c*k[h].z+x[h].z)};
+            if(pj[h]) r[0]=r[1]=r[2]=T(0);
+            S.gr[n]=V4<T>{r[0],r[1],r[2],T(0)};
+            rr.add(r[0]*(r[0]*m[h])+r[1]*(r[1]*m[h])+r[2]*(r[2]*m[h]));
+            const T cn=r[0]*r[0]+r[1]*r[1]+r[2]*r[2];
+            amax=cn>amax?cn:amax;}
+        S.gf[n]=V4<T>{T(0),T(0),T(0),T(0)};}
+}
+// The vector update of a loop trip (k_cg_update) on the node block that starts at node n0.
+template<class T> __device__ __forceinline__ void cg_update_block(const DevState<T>& S,long long n0,T alpha,T beta,T dt2,NodeSum<T>& rr,NodeSum<T>& rs,
+    NodeSum<T>& ss,T& amax)
+{
+    T m[2];V4<T> s[2],k[2],x[2],r[2];unsigned char pj[2];
+#pragma unroll
+    for(int h=0;h<2;++h){const long long n=n0+h*32+(threadIdx.x&31);m[h]=S.gm[n];s[h]=S.gs[n];k[h]=S.gf[n];x[h]=S.gx[n];r[h]=S.gr[n];pj[h]=S.gproj[n];}
+#pragma unroll
+    for(int h=0;h<2;++h){
+        const long long n=n0+h*32+(threadIdx.x&31);
+        if(m[h]>T(0)){
+            const T c=dt2/m[h];
+            s[h].x=r[h].x+beta*s[h].x;s[h].y=r[h].y+beta*s[h].y;s[h].z=r[h].z+beta*s[h].z;
+            T q[3]={c*k[h].x+s[h].x,c*k[h].y+s[h].y,c*k[h].z+s[h].z};
+            if(pj[h]) q[0]=q[1]=q[2]=T(0);
+            x[h].x=alpha*s[h].x+x[h].x;x[h].y=alpha*s[h].y+x[h].y;x[h].z=alpha*s[h].z+x[h].z;
+            r[h].x=-alpha*q[0]+r[h].x;r[h].y=-alpha*q[1]+r[h].y;r[h].z=-alpha*q[2]+r[h].z;
+            S.gs[n]=s[h];S.gx[n]=x[h];S.gr[n]=r[h];
+            rr.add(r[h].x*(r[h].x*m[h])+r[h].y*(r[h].y*m[h])+r[h].z*(r[h].z*m[h]));
+            rs.add(r[h].x*(s[h].x*m[h])+r[h].y*(s[h].y*m[h])+r[h].z*(s[h].z*m[h]));
+            ss.add(s[h].x*(s[h].x*m[h])+s[h].y*(s[h].y*m[h])+s[h].z*(s[h].z*m[h]));
+            const T cn=r[h].x*r[h].x+r[h].y*r[h].y+r[h].z*r[h].z;
+            amax=cn>amax?cn:amax;}
+        S.gf[n]=V4<T>{T(0),T(0),T(0),T(0)};}
+}
+// CG start: cg_start_block on every block, then the first convergence check of the restated CG
+// loop (iteration 0).
 template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_start(DevState<typename P::T> S,unsigned long long cond,int use_cond)
 {
     pdl_enter();
@@ -1280,22 +1332,7 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_start(Dev
     for(int blk=wr.b;blk<wr.b1;++blk){
         const int sb=S.active_scene[blk];
         if(sb!=scene){if(scene>=0) flush(scene,false);scene=sb;}
-        T m[2];V4<T> x[2],b[2],k[2];unsigned char pj[2];
-#pragma unroll
-        for(int h=0;h<2;++h){const long long n=((long long)blk<<6)+h*32+(threadIdx.x&31);m[h]=S.gm[n];x[h]=S.gx[n];b[h]=S.gr[n];k[h]=S.gf[n];pj[h]=S.gproj[n];}
-#pragma unroll
-        for(int h=0;h<2;++h){
-            const long long n=((long long)blk<<6)+h*32+(threadIdx.x&31);
-            if(m[h]>T(0)){
-                const T c=dt2/m[h];
-                T r[3]={b[h].x-(c*k[h].x+x[h].x),b[h].y-(c*k[h].y+x[h].y),b[h].z-(c*k[h].z+x[h].z)};
-                if(pj[h]) r[0]=r[1]=r[2]=T(0);       // Project, flagged by the grid update
-                S.gr[n]=V4<T>{r[0],r[1],r[2],T(0)};
-                rr.add(r[0]*(r[0]*m[h])+r[1]*(r[1]*m[h])+r[2]*(r[2]*m[h]));
-                const T cn=r[0]*r[0]+r[1]*r[1]+r[2]*r[2];
-                amax=cn>amax?cn:amax;}
-            S.gf[n]=V4<T>{T(0),T(0),T(0),T(0)};}
-    }
+        cg_start_block(S,blk,dt2,rr,amax);}
     if(scene>=0) flush(scene,true);
     __shared__ int any;
     if(threadIdx.x==0) any=0;
@@ -1317,7 +1354,7 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_start(Dev
 // A warp's share of the node blocks of the scenes in the list: a contiguous range of list
 // blocks, so that the warp meets each scene once and streams whole blocks (64 nodes, two
 // per lane). next() moves to list block bw (non-decreasing) and tells whether the scene
-// changed; node(h) is the lane's h-th node (h = 0, 1) of that block.
+// changed; node0 is that block's first node.
 struct WarpBlocks {
     int b,b1,j=0,scene=-1;long long base=0;
     __device__ __forceinline__ explicit WarpBlocks(const WarpRange& r):b(r.b),b1(r.b1){}
@@ -1328,7 +1365,7 @@ struct WarpBlocks {
         scene=sm.scene[j];base=sr[scene].b0-sm.pre[j];
         return true;
     }
-    __device__ __forceinline__ long long node(int bw,int h) const {return ((base+bw)<<6)+h*32+(threadIdx.x&31);}
+    __device__ __forceinline__ long long node0(int bw) const {return (base+bw)<<6;}
 };
 // The vector update of a loop trip, one pass over the nodes: s = r + beta s_old, q = s +
 // dt^2/m K s, Project(q), x += alpha s, r -= alpha q (Interior only), K s cleared for the next
@@ -1363,27 +1400,7 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
             const CGState& st=S.cg[wb.scene];
             const double sq=(double)dt2*S.acc[wb.scene].sks+st.msq;
             alpha=(T)(sq!=0.?st.rho/sq:(double)FLT_MAX);beta=(T)st.beta;}
-        T m[2];V4<T> s[2],k[2],x[2],r[2];unsigned char pj[2];
-#pragma unroll
-        for(int h=0;h<2;++h){const long long n=wb.node(bw,h);m[h]=S.gm[n];s[h]=S.gs[n];k[h]=S.gf[n];x[h]=S.gx[n];r[h]=S.gr[n];pj[h]=S.gproj[n];}
-#pragma unroll
-        for(int h=0;h<2;++h){
-            const long long n=wb.node(bw,h);
-            if(m[h]>T(0)){
-                const T c=dt2/m[h];
-                s[h].x=r[h].x+beta*s[h].x;s[h].y=r[h].y+beta*s[h].y;s[h].z=r[h].z+beta*s[h].z;
-                T q[3]={c*k[h].x+s[h].x,c*k[h].y+s[h].y,c*k[h].z+s[h].z};
-                if(pj[h]) q[0]=q[1]=q[2]=T(0);
-                x[h].x=alpha*s[h].x+x[h].x;x[h].y=alpha*s[h].y+x[h].y;x[h].z=alpha*s[h].z+x[h].z;
-                r[h].x=-alpha*q[0]+r[h].x;r[h].y=-alpha*q[1]+r[h].y;r[h].z=-alpha*q[2]+r[h].z;
-                S.gs[n]=s[h];S.gx[n]=x[h];S.gr[n]=r[h];
-                rr.add(r[h].x*(r[h].x*m[h])+r[h].y*(r[h].y*m[h])+r[h].z*(r[h].z*m[h]));
-                rs.add(r[h].x*(s[h].x*m[h])+r[h].y*(s[h].y*m[h])+r[h].z*(s[h].z*m[h]));
-                ss.add(s[h].x*(s[h].x*m[h])+s[h].y*(s[h].y*m[h])+s[h].z*(s[h].z*m[h]));
-                const T cn=(r[h].x*r[h].x+r[h].y*r[h].y+r[h].z*r[h].z);
-                amax=cn>amax?cn:amax;}
-            S.gf[n]=V4<T>{T(0),T(0),T(0),T(0)};}
-    }
+        cg_update_block(S,wb.node0(bw),alpha,beta,dt2,rr,rs,ss,amax);}
     if(wb.scene>=0) flush(wb.scene,true);
     __shared__ int any;
     if(threadIdx.x==0) any=0;
@@ -1409,6 +1426,147 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
         if(S.ctr->loop_iters>=max_trips) any=0;
         S.ctr->any_active=any;
         if(use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond,any?1u:0u);}
+}
+
+// =====================================================================================
+// The whole CG solve of a small single scene in one cooperative kernel (FP32 storage). A loop
+// trip as separate kernels costs two launches, two chains of dependent loads until a CTA
+// has its work item, and two last-CTA reductions, about 25 us in which a small scene computes
+// for a few. Here the CTAs stay: each keeps its work item's record (and, with one pass per
+// warp, its pairs) on chip, the node blocks are spread over all warps, and the phases
+// (product, vector update) are separated by grid barriers whose arrivals carry the sums.
+// With fewer work items than CTAs an item's passes are split over 2 or 4 CTAs.
+// =====================================================================================
+// One arrival per CTA; thread 0 waits for all (bounded) and runs `post`. False after the limit.
+constexpr int SOLVE_SPIN_LIMIT=1<<20;
+template<class F> __device__ __forceinline__ bool solve_barrier(Counters* ctr,unsigned target,F post)
+{
+    __shared__ bool ok;
+    __syncthreads();
+    if(threadIdx.x==0){
+        __threadfence();
+        atomicAdd(&ctr->solve_arrived,1u);
+        int spins=0;
+        while(*(volatile unsigned*)&ctr->solve_arrived<target&&++spins<SOLVE_SPIN_LIMIT) if(spins>64) __nanosleep(32);
+        __threadfence();
+        ok=*(volatile unsigned*)&ctr->solve_arrived>=target;
+        if(!ok) atomicOr(&ctr->error,ERR_GRID_WAIT);
+        post();}
+    __syncthreads();
+    return ok;
+}
+template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(DevState<typename P::T> S,int max_trips)
+{
+    using T=typename P::T;
+    static_assert(sizeof(T)==4,"pair tables are FP32 only");
+    constexpr int NW=XFER_THREADS/32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int rec[ITEM_WORDS];
+    __shared__ unsigned tmap[TILE_N];
+    __shared__ double part[NW][4];
+    __shared__ T sh_alpha,sh_beta;
+    __shared__ int sh_stop;
+    const int warp=threadIdx.x>>5,lane=threadIdx.x&31;
+    auto tile_of=[&](int w){return reinterpret_cast<T (*)[TILE_S]>(smem_raw+w*hess_warp_bytes<T>());};
+    T (*q)[TILE_S]=tile_of(warp);
+    T (*sv)[TILE_S]=tile_of(0)+3;
+    V4<float> (*slots)[32]=reinterpret_cast<V4<float> (*)[32]>(smem_raw+warp*hess_warp_bytes<T>()+6*TILE_S*sizeof(T));
+    for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x) tmap[t]=tile_map_entry(t);
+    for(int t=lane;t<3*TILE_S;t+=32) (&q[0][0])[t]=T(0);
+    Counters* ctr=S.ctr;
+    const int G=(int)gridDim.x;
+    const int nc=(int)min(ctr->n_chunks,(unsigned)S.chunk_cap),na=(int)min(ctr->n_active,(unsigned)S.block_cap);
+    const int split=4*nc<=G?4:2*nc<=G?2:1,units=nc*split;
+    const int per=(na+G*NW-1)/(G*NW),b0=min(na,((int)blockIdx.x*NW+warp)*per),b1=min(na,b0+per);
+    const SceneDev<T>& sc=S.scenes[0];
+    const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
+    PairPass pass;                       // the warp's resident pass, when the CTA has one unit
+    int held=-1;                         // unit whose record is in rec
+    int phase=0;
+    auto arrived=[&]{return (unsigned)(phase+1)*(unsigned)G;};
+    // K v for v = x, or s = r + beta s_old with s^T K s into part[][0]
+    auto product=[&](bool from_x,T beta){
+        double sks=0.;
+        for(int u=blockIdx.x;u<units;u+=G){
+            if(u!=held){
+                __syncthreads();
+                if(warp==0) rec[lane]=S.items[(long long)(u/split)*ITEM_WORDS+lane];
+                held=u;pass.ready=false;
+                __syncthreads();}
+            stage_vector<T,XFER_THREADS>(S,rec+ITEM_NBR,tmap,from_x,beta,sv,threadIdx.x);
+            __syncthreads();
+            hessian_pairs(S,sc,rec[ITEM_START],rec[ITEM_PAIRS],(warp+NW*(u%split))*32,NW*split*32,sv,q,slots,sks,pass);
+            __syncthreads();
+            for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x){
+                const unsigned e=tmap[t];
+                T v[3];
+#pragma unroll
+                for(int ch=0;ch<3;++ch){T a=T(0);
+#pragma unroll
+                    for(int w2=0;w2<NW;++w2){T* p=&tile_of(w2)[ch][e>>11];a+=*p;*p=T(0);}
+                    v[ch]=a;}
+                add_tile_node(S,rec,e,v[0],v[1],v[2]);}}
+        const double s=warp_sum<double>(sks);
+        if(lane==0) part[warp][0]=s;};
+    // thread 0: the CTA's sums into the slot of this phase
+    auto contribute=[&](int ns,bool with_max){
+        __syncthreads();
+        if(threadIdx.x==0){
+            SolveSlot& o=ctr->solve[phase&3];
+            for(int k=0;k<ns;++k){double s=0.;for(int w=0;w<NW;++w) s+=part[w][k];if(s!=0.) atomicAdd(&o.sum[k],s);}
+            if(with_max){double m=0.;for(int w=0;w<NW;++w) m=fmax(m,part[w][3]);if(m>0.) atomicMax(&o.max0,dbits(m));}}};
+    auto clear_ahead=[&]{               // the slot two phases on: read by nobody any more
+        if(blockIdx.x==0){SolveSlot& o=ctr->solve[(phase+2)&3];o.sum[0]=o.sum[1]=o.sum[2]=0.;o.max0=0ull;}};
+    auto read_slot=[&](double (&s)[3],double& mx){
+        const volatile SolveSlot& o=ctr->solve[phase&3];
+        s[0]=o.sum[0];s[1]=o.sum[1];s[2]=o.sum[2];mx=bitsd(o.max0);};
+    const double eps=1.1920928955078125e-07;     // FP32, as k_cg_start and k_cg_update
+    // x = v*: r = b - A x and the first check
+    product(true,T(0));
+    if(!solve_barrier(ctr,arrived(),clear_ahead)) return;
+    ++phase;
+    {   NodeSum<T> rr;T amax=T(0);
+        for(int blk=b0;blk<b1;++blk) cg_start_block(S,blk,dt2,rr,amax);
+        const double a=warp_sum<double>(rr.value()),m=warp_max<double>((double)amax);
+        if(lane==0){part[warp][0]=a;part[warp][3]=m;}}
+    contribute(1,true);
+    double rho=0.,msq=0.,rmax=0.,beta=0.;        // thread 0 of every CTA: equal values
+    int iters=0,converged=0;
+    const double tol=S.cg[0].tol,tol2=tol*tol;
+    // sqrt(mx) <= tol; the root (on the barriers' critical path) only where rounding could decide
+    auto small=[&](double mx){return mx<tol2*(1.-1e-14)?true:mx>tol2*(1.+1e-14)?false:sqrt(mx)<=tol;};
+    if(!solve_barrier(ctr,arrived(),[&]{
+        double s[3],mx;read_slot(s,mx);clear_ahead();
+        rmax=mx;rho=msq=s[0];
+        converged=small(mx)&&(0>=sc.cg_min_iters||sqrt(mx)<eps);
+        sh_stop=converged||sc.cg_max_iters<=0||max_trips<=0;sh_beta=T(0);})) return;
+    while(!sh_stop){
+        ++phase;
+        const T be=sh_beta;
+        product(false,be);
+        contribute(1,false);
+        if(!solve_barrier(ctr,arrived(),[&]{
+            double s[3],mx;read_slot(s,mx);clear_ahead();
+            const double sq=(double)dt2*s[0]+msq;
+            sh_alpha=(T)(sq!=0.?rho/sq:(double)FLT_MAX);})) return;
+        ++phase;
+        {   const T alpha=sh_alpha;
+            NodeSum<T> rr,rs,ss;T amax=T(0);
+            for(int blk=b0;blk<b1;++blk) cg_update_block(S,((long long)blk<<6),alpha,be,dt2,rr,rs,ss,amax);
+            const double a=warp_sum<double>(rr.value()),b=warp_sum<double>(rs.value()),c=warp_sum<double>(ss.value()),m=warp_max<double>((double)amax);
+            if(lane==0){part[warp][0]=a;part[warp][1]=b;part[warp][2]=c;part[warp][3]=m;}}
+        contribute(3,true);
+        if(!solve_barrier(ctr,arrived(),[&]{
+            double s[3],mx;read_slot(s,mx);clear_ahead();
+            ++iters;rmax=mx;
+            converged=small(mx)&&(iters>=sc.cg_min_iters||sqrt(mx)<eps);
+            beta=s[0]/rho;rho=s[0];msq=s[0]+beta*(2.*s[1]+beta*s[2]);
+            sh_beta=(T)beta;sh_stop=converged||iters>=sc.cg_max_iters||iters>=max_trips;})) return;}
+    if(blockIdx.x==0&&threadIdx.x==0){
+        CGState& st=S.cg[0];
+        st.rho=rho;st.beta=beta;st.msq=msq;st.residual=sqrt(rmax);st.iters=iters;st.done=1;st.converged=converged;
+        if(!converged) atomicOr(&ctr->error,ERR_CG_NOT_CONVERGED);
+        ctr->any_active=0;ctr->loop_iters=iters;ctr->total_trips+=iters;}
 }
 
 // =====================================================================================
