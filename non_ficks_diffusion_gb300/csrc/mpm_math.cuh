@@ -540,10 +540,54 @@ static __host__ __device__ __noinline__ ClampResult clamp_fp64_cold(ClampArgs a)
     return r;
 }
 
+// Polar rotation of F near a rotation, without an SVD: with e = F^T F - I,
+//   R = F (I + e)^(-1/2) = F + F e (-1/2 + e (3/8 - e (5/16 - e 35/128))) + O(63/256 |e|^5).
+// e is evaluated to twice FP32 precision and the correction added last, so that R is the exact
+// rotation rounded to FP32, but for the series' end: below 2e-10 for |e| <= 0.0149 (Frobenius
+// norm, a bound of the eigenvalues of F^T F). Returns false, R untouched, when |e|^2 >= lim2.
+constexpr float POLAR_SERIES_MAX=0.0149f;
+MPM_HD bool polar_near(const float* F,float lim2,float* R)
+{
+    float c[6];                      // e from plain FP32 products, for the test: 00, 01, 02, 11, 12, 22
+    c[0]=F[0]*F[0]+F[3]*F[3]+(F[6]*F[6]-1.f);c[1]=F[0]*F[1]+F[3]*F[4]+F[6]*F[7];c[2]=F[0]*F[2]+F[3]*F[5]+F[6]*F[8];
+    c[3]=F[1]*F[1]+F[4]*F[4]+(F[7]*F[7]-1.f);c[4]=F[1]*F[2]+F[4]*F[5]+F[7]*F[8];c[5]=F[2]*F[2]+F[5]*F[5]+(F[8]*F[8]-1.f);
+    if(!(c[0]*c[0]+c[3]*c[3]+c[5]*c[5]+2.f*(c[1]*c[1]+c[2]*c[2]+c[4]*c[4])<lim2)) return false;
+    float e[6];
+    {   const int a[6]={0,0,0,1,1,2},b[6]={0,1,2,1,2,2};
+#pragma unroll
+        for(int k=0;k<6;++k){
+            const F2x d=ff_dot3(F[a[k]],F[b[k]],F[3+a[k]],F[3+b[k]],F[6+a[k]],F[6+b[k]]);
+            e[k]=(a[k]==b[k]?d.h-1.f:d.h)+d.l;}}
+    // H <- s I + e H, symmetric (polynomials of e commute)
+    float H[6];
+#pragma unroll
+    for(int k=0;k<6;++k) H[k]=e[k]*0.2734375f;
+    auto horner=[&](float s){
+        const float h0=H[0]+s,h1=H[1],h2=H[2],h3=H[3]+s,h4=H[4],h5=H[5]+s;
+        H[0]=e[0]*h0+e[1]*h1+e[2]*h2;H[1]=e[0]*h1+e[1]*h3+e[2]*h4;H[2]=e[0]*h2+e[1]*h4+e[2]*h5;
+        H[3]=e[1]*h1+e[3]*h3+e[4]*h4;H[4]=e[1]*h2+e[3]*h4+e[4]*h5;H[5]=e[2]*h2+e[4]*h4+e[5]*h5;};
+    horner(-0.3125f);horner(0.375f);horner(-0.5f);
+#pragma unroll
+    for(int i=0;i<3;++i){
+        const float f0=F[3*i],f1=F[3*i+1],f2=F[3*i+2];
+        R[3*i]=f0+(f0*H[0]+f1*H[1]+f2*H[2]);R[3*i+1]=f1+(f0*H[1]+f1*H[3]+f2*H[4]);R[3*i+2]=f2+(f0*H[2]+f1*H[4]+f2*H[5]);}
+    return true;
+}
+
+// Hardened Lame parameters (reference :53-60).
+template<class T> MPM_HD void harden(const T Jp,const T lambda0,const T mu0,const int plastic,const T hardening,const T hardening_max,T& lambda,T& mu)
+{
+    if(plastic){
+        T power=hardening*(T(1)-Jp);if(power>hardening_max) power=hardening_max;
+        const T e=mpm_exp<T>(power);
+        lambda=e*lambda0;mu=e*mu0;}
+    else{lambda=lambda0;mu=mu0;}
+}
 // Precompute: SVD of Fe, clamp of the singular values to [cy, sy], Jp update (det of the
 // reference's Fp <- V S^-1 U^T Fe Fp), Fe <- U S_hat V^T, hardened Lame parameters,
 // Re = U V^T. Writes Fe, Jp in place (rounded to T).
 //
+// FP32 storage: a Fe near a rotation and for certain inside the yield band takes polar_near.
 // TS == float: everything in FP32. TS == double (mixed and FP64 variants): the SVD is
 // first done in FP32. If those singular values lie inside [cy, sy] by a margin far above
 // the FP32 error, no clamp happens in exact arithmetic, so Fe and Jp are unchanged and
@@ -559,8 +603,16 @@ template<class T,class TS> MPM_HD void precompute(T* Fe,T& Jp,const T lambda0,co
     float F32[9],U32[9],s32[3],V32[9];
 #pragma unroll
     for(int k=0;k<9;++k) F32[k]=(float)Fe[k];
-    svd3<float>(F32,U32,s32,V32);
     const float margin=1e-5f;
+    if constexpr(sizeof(T)==4){
+        // no clamp for certain, all singular values inside the yield band: only the rotation is
+        // needed (unstrained and lightly strained bodies; the SVD below took half of P2G there)
+        const float lim=plastic?fminf(fminf((sy-margin)*(sy-margin)-1.f,1.f-(cy+margin)*(cy+margin)),POLAR_SERIES_MAX):POLAR_SERIES_MAX;
+        if(lim>0.f&&polar_near(F32,lim*lim,Re)){
+            Je=det3_dot2(F32);
+            harden(Jp,lambda0,mu0,plastic,hardening,hardening_max,lambda,mu);
+            return;}}
+    svd3<float>(F32,U32,s32,V32);
     const bool inside=s32[0]<(float)sy-margin&&s32[2]>(float)cy+margin;
     if constexpr(sizeof(TS)==4){
         if(plastic){
@@ -604,11 +656,7 @@ template<class T,class TS> MPM_HD void precompute(T* Fe,T& Jp,const T lambda0,co
 #pragma unroll
             for(int k=0;k<9;++k) Re[k]=(T)R32[k];
             Je=(T)det3_dot2(F32);}}
-    if(plastic){
-        T power=hardening*(T(1)-Jp);if(power>hardening_max) power=hardening_max;
-        const T e=mpm_exp<T>(power);
-        lambda=e*lambda0;mu=e*mu0;}
-    else{lambda=lambda0;mu=mu0;}
+    harden(Jp,lambda0,mu0,plastic,hardening,hardening_max,lambda,mu);
 }
 
 // First Piola-Kirchhoff stress P = 2 mu (Fe - Re) + lambda (Je-1) cof(Fe), reference :63-67.

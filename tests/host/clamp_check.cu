@@ -56,6 +56,23 @@ int main()
             for(int k=0;k<9;++k) d=std::fmax(d,std::fmax(std::fabs(Fm[k]-Fx[k]),std::fabs(Rm[k]-Rx[k])));
             worst=std::fmax(worst,d*std::ldexp(1.,24));}
         std::printf("%s %.4f ",names[mode],worst);}
+    // the rotation near a rotation (polar_near, FP32 storage in both variants): Re and Je
+    for(int mode=0;mode<3;++mode){
+        std::mt19937_64 g(31+mode);
+        std::uniform_real_distribution<double> u(-1.,1.);
+        const double strain=mode==0?1e-7:mode==1?1e-3:0.007;     // the last reaches the series' limit
+        double worst=0;
+        for(int it=0;it<20000;++it){
+            double A[9],B[9],s[3],F[9];
+            rotation(g,A);rotation(g,B);
+            for(double& x:s) x=1+strain*u(g);
+            for(int i=0;i<3;++i) for(int j=0;j<3;++j) F[3*i+j]=A[3*i]*s[0]*B[3*j]+A[3*i+1]*s[1]*B[3*j+1]+A[3*i+2]*s[2]*B[3*j+2];
+            float Ff[9],R[9];double Fx[9],Rx[9],lx,mx,Jx,Jq=1.;
+            for(int k=0;k<9;++k){Ff[k]=(float)F[k];Fx[k]=Ff[k];}
+            if(!polar_near(Ff,POLAR_SERIES_MAX*POLAR_SERIES_MAX,R)) continue;
+            precompute<double,double>(Fx,Jq,1e4,2e4,0,10.,(double)cy,(double)sy,10.,Rx,lx,mx,Jx);
+            for(int k=0;k<9;++k) worst=std::fmax(worst,std::fabs(R[k]-Rx[k])*std::ldexp(1.,24));}
+        std::printf("%s %.4f ",mode==0?"rigid":mode==1?"light":"limit",worst);}
     std::printf("\n");
     return 0;
 }

@@ -27,3 +27,9 @@ def clamp_check(tmp_path_factory):
 @pytest.mark.parametrize("family", ["wide", "band", "equal", "lower", "upper", "near", "pair", "far"])
 def test_corrected_clamp_rounds_like_fp64(clamp_check, family):
     assert clamp_check[family] <= 1.1
+
+
+@pytest.mark.parametrize("family", ["rigid", "light", "limit"])
+def test_rotation_near_a_rotation_rounds_like_fp64(clamp_check, family):
+    # entries up to 1: half a unit of rounding, and a tenth for the series' end
+    assert clamp_check[family] <= 0.6
