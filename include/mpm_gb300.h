@@ -332,7 +332,7 @@ MPM_API mpm_status mpm_autotune(struct mpm_context* ctx, double dt, int substeps
  * begin_bit upward in ceil((end_bit-begin_bit)/8) 8-bit digits, ties keeping input order.
  * Work runs on `stream` (NULL: the default stream) and is not waited for.
  * Limit: n <= MPM_NOALLOC_SORT_MAX (1,048,576); larger n returns MPM_BAD_ARG.
- * The working memory is one fixed static device area of about 8.3 MB per GPU, held from
+ * The working memory is one fixed static device area of about 9.5 MB per GPU, held from
  * library load to process exit and shared by every call on that GPU: calls that overlap
  * on the GPU (different streams, other threads) race and must be serialised by the
  * caller. Every byte of it is rewritten before it is read, so a call does not depend on

@@ -10,9 +10,7 @@ namespace mpm {
 
 constexpr int RS_THREADS=256, RS_WARPS=RS_THREADS/32;
 // Keys per thread of a radix tile: small inputs use short tiles so that every SM has one.
-constexpr int RS_ITEMS_SMALL=4, RS_ITEMS=16, RS_TILE=RS_THREADS*RS_ITEMS;
-constexpr long long RS_SMALL_N=1<<21;
-__host__ __device__ constexpr int rs_items(long long n){return n<RS_SMALL_N?RS_ITEMS_SMALL:RS_ITEMS;}
+constexpr int RS_ITEMS_SMALL=4, RS_ITEMS=16;
 // Tile size of the one-sweep passes: short tiles give small inputs one per SM; long ones
 // keep the look-back chain short on large inputs.
 __host__ __device__ constexpr int os_items(long long n){return n<(1LL<<18)?RS_ITEMS_SMALL:RS_ITEMS;}
@@ -112,7 +110,8 @@ template<class T> __global__ void __launch_bounds__(256) k_keys(DevState<T> S,un
 // ---- one-sweep radix pass (decoupled look-back) ----
 // One kernel per 8-bit pass. Tiles are taken in the order of an atomic counter, so every
 // tile before the one a CTA holds is held by a CTA that has already started. A tile ranks
-// its keys stably (as k_radix_scatter), publishes its per-digit counts, then walks back
+// its keys stably (peers with the same digit by lane order, on top of the warp's running
+// per-digit count), publishes its per-digit counts, then walks back
 // over the earlier tiles' published words until it meets an inclusive prefix; the sum is
 // the tile's offset inside each digit. Status word per (tile, digit): 2 flag bits
 // (0 none, 1 count of the tile, 2 inclusive prefix) over a 30-bit count; the array and
@@ -214,85 +213,6 @@ template<int ITEMS> __global__ void __launch_bounds__(RS_THREADS) k_onesweep(con
 
 // Non-template kernels here are static: every translation unit that includes this header
 // gets its own copy.
-// ---- radix sort: 8-bit digits, per-tile histograms laid out [digit][tile] ----
-template<int ITEMS> static __global__ void __launch_bounds__(RS_THREADS) k_radix_hist(const unsigned* __restrict__ keys,long long n,int shift,
-                                                           unsigned* __restrict__ counts,int num_tiles)
-{
-    __shared__ unsigned h[256];
-    for(int tile=blockIdx.x;tile<num_tiles;tile+=gridDim.x){
-        h[threadIdx.x]=0;
-        __syncthreads();
-        const long long base=(long long)tile*RS_THREADS*ITEMS;
-#pragma unroll 4
-        for(int j=0;j<ITEMS;++j){
-            const long long idx=base+j*RS_THREADS+threadIdx.x;
-            if(idx<n) atomicAdd(&h[(keys[idx]>>shift)&255u],1u);}
-        __syncthreads();
-        counts[(long long)threadIdx.x*num_tiles+tile]=h[threadIdx.x];
-        __syncthreads();
-    }
-}
-
-// Stable scatter: warp w of a tile owns the contiguous keys [w*32*ITEMS, (w+1)*32*ITEMS) and walks
-// them 32 at a time in index order; peers with the same digit are ranked by lane order
-// (match.any) on top of the warp's running per-digit count; warps are then offset by an
-// exclusive scan over warps per digit.
-template<int ITEMS> static __global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const unsigned* __restrict__ kin,const int* __restrict__ vin,
-                                                              unsigned* __restrict__ kout,int* __restrict__ vout,long long n,int shift,
-                                                              const unsigned* __restrict__ offsets,int num_tiles)
-{
-    __shared__ unsigned wcnt[RS_WARPS][256];
-    const int w=threadIdx.x>>5,lane=threadIdx.x&31;
-    for(int tile=blockIdx.x;tile<num_tiles;tile+=gridDim.x){
-        for(int t=threadIdx.x;t<RS_WARPS*256;t+=RS_THREADS) (&wcnt[0][0])[t]=0;
-        __syncthreads();
-        const long long base=(long long)tile*RS_THREADS*ITEMS+(long long)w*(ITEMS*32);
-        unsigned k[ITEMS];unsigned short r[ITEMS];
-#pragma unroll
-        for(int j=0;j<ITEMS;++j){
-            const long long idx=base+j*32+lane;
-            const bool valid=idx<n;
-            k[j]=valid?kin[idx]:0u;
-            const unsigned d=(k[j]>>shift)&255u;
-            const unsigned peers=__match_any_sync(0xffffffffu,valid?d:(256u+lane));
-            const unsigned rank=__popc(peers&lanemask_lt());
-            const unsigned before=valid?wcnt[w][d]:0u;
-            __syncwarp();
-            if(valid&&rank==0) wcnt[w][d]=before+__popc(peers);
-            __syncwarp();
-            r[j]=(unsigned short)(before+rank);}
-        __syncthreads();
-        {   // exclusive scan over warps, one digit per thread
-            const int d=threadIdx.x;unsigned run=0;
-#pragma unroll
-            for(int ww=0;ww<RS_WARPS;++ww){const unsigned c=wcnt[ww][d];wcnt[ww][d]=run;run+=c;}}
-        __syncthreads();
-#pragma unroll
-        for(int j=0;j<ITEMS;++j){
-            const long long idx=base+j*32+lane;
-            if(idx<n){
-                const unsigned d=(k[j]>>shift)&255u;
-                const long long pos=(long long)offsets[(long long)d*num_tiles+tile]+wcnt[w][d]+r[j];
-                kout[pos]=k[j];vout[pos]=vin?vin[idx]:(int)idx;}}
-        __syncthreads();
-    }
-}
-
-// ---- device-wide exclusive scan of uint32 (segments of SC_SEG, three kernels) ----
-template<class F> __device__ __forceinline__ unsigned seg_sum(F get,long long n,long long seg)
-{
-    unsigned s=0;const long long base=seg*SC_SEG;
-#pragma unroll
-    for(int j=0;j<SC_ITEMS;++j){const long long i=base+j*SC_THREADS+threadIdx.x;if(i<n) s+=get(i);}
-    __shared__ unsigned red[SC_THREADS/32];
-    for(int o=16;o>0;o>>=1) s+=__shfl_xor_sync(0xffffffffu,s,o);
-    if((threadIdx.x&31)==0) red[threadIdx.x>>5]=s;
-    __syncthreads();
-    unsigned t=0;
-    if(threadIdx.x<32){t=threadIdx.x<SC_THREADS/32?red[threadIdx.x]:0u;for(int o=16;o>0;o>>=1) t+=__shfl_xor_sync(0xffffffffu,t,o);}
-    __syncthreads();
-    return t;   // valid in thread 0
-}
 // CTA-wide exclusive scan of one value per thread; returns the prefix, *total the sum.
 __device__ __forceinline__ unsigned cta_exclusive_scan(unsigned v,unsigned* total)
 {
@@ -312,44 +232,6 @@ __device__ __forceinline__ unsigned cta_exclusive_scan(unsigned v,unsigned* tota
     if(total) *total=wsum[nw-1];
     __syncthreads();
     return excl;
-}
-
-static __global__ void __launch_bounds__(SC_THREADS) k_scan_sums(const unsigned* __restrict__ in,long long n,unsigned* __restrict__ sums)
-{
-    const long long nseg=(n+SC_SEG-1)/SC_SEG;
-    for(long long seg=blockIdx.x;seg<nseg;seg+=gridDim.x){
-        const unsigned t=seg_sum([&](long long i){return in[i];},n,seg);
-        if(threadIdx.x==0) sums[seg]=t;}
-}
-// One CTA: exclusive scan of sums[0..nseg) in place; writes the grand total to *total and,
-// if cap_check>=0, flags ERR_CAPACITY when the total exceeds it.
-static __global__ void __launch_bounds__(1024) k_scan_top(unsigned* sums,long long nseg,unsigned* total,long long cap_check,unsigned* err)
-{
-    unsigned carry=0;
-    for(long long base=0;base<nseg;base+=blockDim.x){
-        const long long i=base+threadIdx.x;
-        const unsigned v=i<nseg?sums[i]:0u;
-        unsigned tot;const unsigned e=cta_exclusive_scan(v,&tot);
-        if(i<nseg) sums[i]=carry+e;
-        carry+=tot;}
-    if(threadIdx.x==0){
-        if(total) *total=carry;
-        if(cap_check>=0&&(long long)carry>cap_check&&err) atomicOr(err,ERR_CAPACITY);}
-}
-static __global__ void __launch_bounds__(SC_THREADS) k_scan_apply(const unsigned* __restrict__ in,unsigned* __restrict__ out,long long n,
-                                                           const unsigned* __restrict__ sums)
-{
-    const long long nseg=(n+SC_SEG-1)/SC_SEG;
-    for(long long seg=blockIdx.x;seg<nseg;seg+=gridDim.x){
-        const long long base=seg*SC_SEG+(long long)threadIdx.x*SC_ITEMS;
-        unsigned v[SC_ITEMS],s=0;
-#pragma unroll
-        for(int j=0;j<SC_ITEMS;++j){v[j]=base+j<n?in[base+j]:0u;s+=v[j];}
-        const unsigned off=sums[seg]+cta_exclusive_scan(s,nullptr);
-        unsigned run=off;
-#pragma unroll
-        for(int j=0;j<SC_ITEMS;++j){if(base+j<n) out[base+j]=run;run+=v[j];}
-    }
 }
 
 // Exclusive prefix of the CTA's segment total `total` over segments taken in the order of
