@@ -70,6 +70,9 @@ struct mpm_context {
     double* d_dt=nullptr; double last_dt=-1;
     double time=0;                            // simulation clock (seconds)
     FrameState* frame=nullptr; FrameState* h_frame=nullptr;
+    // of mpm_max_particle_velocity, which the host-driven time stepping calls before every
+    // substep: allocating and freeing it there cost 15 us of each substep
+    unsigned long long* vmax=nullptr; unsigned long long* h_vmax=nullptr;
     void* staging=nullptr; size_t staging_bytes=0;
     int* inv=nullptr;                         // slot of each particle by global insertion index (direct transfers)
     long long order_epoch=0,inv_epoch=-1;     // the particle order changes with every substep; inv follows it
@@ -898,6 +901,8 @@ mpm_status mpm_create(const mpm_config* cfg,mpm_context** out)
     ok&=cudaMalloc((void**)&c->d_dt,sizeof(double))==cudaSuccess;
     ok&=cudaMalloc((void**)&c->frame,sizeof(FrameState))==cudaSuccess;
     ok&=cudaMallocHost((void**)&c->h_frame,sizeof(FrameState))==cudaSuccess;
+    ok&=cudaMalloc((void**)&c->vmax,sizeof(*c->vmax))==cudaSuccess;
+    ok&=cudaMallocHost((void**)&c->h_vmax,sizeof(*c->h_vmax))==cudaSuccess;
     ok&=cudaMallocHost((void**)&c->h_ctr,sizeof(Counters))==cudaSuccess;
     ok&=cudaMallocHost((void**)&c->h_cg,sizeof(CGState)*c0.max_scenes)==cudaSuccess;
     if(!ok) return bail(MPM_CUDA_ERROR);
@@ -915,12 +920,13 @@ mpm_status mpm_destroy(mpm_context* c)
     for(int p=0;p<2;++p){if(c->gexec[p]) cudaGraphExecDestroy(c->gexec[p]);if(c->fgexec[p]) cudaGraphExecDestroy(c->fgexec[p]);}
     void* bufs[]={c->pstate[0],c->pstate[1],c->pid[0],c->pid[1],c->scn[0],c->scn[1],c->cache,c->keys[0],c->keys[1],c->vals[0],c->vals[1],
                   c->sortws,c->chunk_start,c->items,c->bitmap,c->blockmap,c->active_gb,c->active_scene,c->gv,c->gf,c->gx,c->gr,c->gs,c->gm,c->gproj,
-                  c->scenes_dev,c->scene_block_base,c->cg,c->acc,c->acc2,c->ctr,c->staging,c->d_dt,c->frame,c->inv,
+                  c->scenes_dev,c->scene_block_base,c->cg,c->acc,c->acc2,c->ctr,c->staging,c->d_dt,c->frame,c->vmax,c->inv,
                   c->srange,c->alist,c->mkeys[0],c->mkeys[1],c->mvals[0],c->mvals[1],c->mwords,c->manchor};
     for(void* p:bufs) if(p) cudaFree(p);
     if(c->h_ctr) cudaFreeHost(c->h_ctr);
     if(c->h_cg) cudaFreeHost(c->h_cg);
     if(c->h_frame) cudaFreeHost(c->h_frame);
+    if(c->h_vmax) cudaFreeHost(c->h_vmax);
     for(auto& e:c->ev_pair) if(e) cudaEventDestroy(e);
     if(c->stream) cudaStreamDestroy(c->stream);
     if(c->stream2) cudaStreamDestroy(c->stream2);
@@ -1139,15 +1145,11 @@ mpm_status mpm_max_particle_velocity(mpm_context* c,int scene,double* vmax)
     return dispatch(c,[&](auto p)->mpm_status{
         using P=decltype(p);
         DevState<TT<P>> S=make_state<P>(c,c->cur,0.0);
-        unsigned long long* tmp=nullptr;
-        CUDA_TRY(c,cudaMalloc(&tmp,8));
-        CUDA_TRY(c,cudaMemsetAsync(tmp,0,8,c->stream));
-        k_vmax<TT<P>><<<grid_for(c,4),256,0,c->stream>>>(S,scene,tmp);c->launches++;
-        unsigned long long h=0;
-        CUDA_TRY(c,cudaMemcpyAsync(&h,tmp,8,cudaMemcpyDeviceToHost,c->stream));
+        CUDA_TRY(c,cudaMemsetAsync(c->vmax,0,sizeof(*c->vmax),c->stream));
+        k_vmax<TT<P>><<<grid_for(c,4),256,0,c->stream>>>(S,scene,c->vmax);c->launches++;
+        CUDA_TRY(c,cudaMemcpyAsync(c->h_vmax,c->vmax,sizeof(*c->vmax),cudaMemcpyDeviceToHost,c->stream));
         CUDA_TRY(c,cudaStreamSynchronize(c->stream));
-        cudaFree(tmp);
-        double v2;std::memcpy(&v2,&h,8);*vmax=std::sqrt(v2);
+        double v2;std::memcpy(&v2,c->h_vmax,8);*vmax=std::sqrt(v2);
         return MPM_OK;});
 }
 
