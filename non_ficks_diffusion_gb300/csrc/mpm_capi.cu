@@ -162,7 +162,7 @@ template<class P> DevState<TT<P>> make_state(mpm_context* c,int parity,double dt
     const int fin=c->sort_passes&1;   // the sort's final ping-pong buffer
     S.keys=c->keys[fin];S.perm=c->vals[fin];
     S.chunk_start=c->chunk_start;S.chunk_cap=c->chunk_cap;S.items=c->items;
-    S.pairs=c->mkeys[0];                      // free between the binning and the next substep's
+    S.pairs=c->mkeys[0];S.src=c->mvals[0];    // free between the binning and the next substep's
     S.bitmap=c->bitmap;S.bitmap_words=c->bitmap_words;
     S.blockmap=c->blockmap;S.active_gb=c->active_gb;S.active_scene=c->active_scene;S.block_cap=c->block_cap;
     S.gv=(V4<T>*)c->gv;S.gf=(V4<T>*)c->gf;S.gx=(V4<T>*)c->gx;S.gr=(V4<T>*)c->gr;S.gs=(V4<T>*)c->gs;S.gm=(T*)c->gm;S.gproj=c->gproj;
@@ -174,7 +174,8 @@ template<class P> DevState<TT<P>> make_state(mpm_context* c,int parity,double dt
 }
 
 // Keys, stable radix sort, work items and active blocks for the current particle buffer.
-template<class P> void enqueue_binning(mpm_context* c,cudaStream_t st,const DevState<TT<P>>& S)
+// `order`: also the storage order of the work items' particles, which FP32 substeps need.
+template<class P> void enqueue_binning(mpm_context* c,cudaStream_t st,const DevState<TT<P>>& S,bool order)
 {
     const long long n=c->n_total;
     {PhaseScope ps(c,PH_KEYS,st);
@@ -244,7 +245,7 @@ template<class P> void enqueue_binning(mpm_context* c,cudaStream_t st,const DevS
         const long long bseg=(c->bitmap_words+BM_SEG-1)/BM_SEG;
         const int gb=(int)std::max<long long>(1,std::min<long long>(bseg,grid_for(c,8)));
         launch_dep(c,k_bitmap_index<TT<P>>,gb,SC_THREADS,0,st,S,c->sortws+c->bin_blocks_off,c->sortws+1029);counted(c,PH_BIN);
-        launch_dep(c,k_clear_nodes<TT<P>>,grid_for(c,8),256,0,st,S);counted(c,PH_BIN);}
+        launch_dep(c,k_items<TT<P>>,grid_for(c,16),XFER_THREADS,order?order_bytes(c->cfg.chunk):0,st,S,order?1:0);counted(c,PH_BIN);}
 }
 
 int max_cg_iters(mpm_context* c){int m=0;for(auto& s:c->scenes) m=std::max(m,s.desc.cg_max_iters);return m;}
@@ -299,10 +300,20 @@ template<class P> cudaError_t launch_solve(mpm_context* c,cudaStream_t st,const 
 template<class P> DevState<TT<P>> enqueue_pre(mpm_context* c,cudaStream_t st,int parity,double dt,unsigned long long cond,int use_cond,int stop_after)
 {
     DevState<TT<P>> S=make_state<P>(c,parity,dt);
-    enqueue_binning<P>(c,st,S);
-    {PhaseScope ps(c,PH_P2G,st);
-        with_minb(c->minb_p2g,[&](auto m){launch_dep(c,k_p2g<P,decltype(m)::value>,grid_for(c,c->xfer_grid),XFER_THREADS,p2g_smem_bytes<TT<P>>(c->cfg.chunk),st,S);});counted(c,PH_P2G);}
     DevState<TT<P>> S2=make_state<P>(c,parity^1,dt);
+    if constexpr(sizeof(TT<P>)==8){
+        enqueue_binning<P>(c,st,S,false);
+        PhaseScope ps(c,PH_P2G,st);
+        with_minb(c->minb_p2g,[&](auto m){launch_dep(c,k_p2g<decltype(m)::value>,grid_for(c,c->xfer_grid),XFER_THREADS,p2g_smem_bytes<TT<P>>(c->cfg.chunk),st,S);});counted(c,PH_P2G);}
+    else{
+        enqueue_binning<P>(c,st,S,true);
+        PhaseScope ps(c,PH_P2G,st);
+        const int g=(int)std::max<long long>(1,std::min<long long>((c->n_total+XFER_THREADS-1)/XFER_THREADS,grid_for(c,16)));
+        launch_dep(c,k_particles<P>,g,XFER_THREADS,0,st,S);counted(c,PH_P2G);
+        with_minb(c->minb_p2g,[&](auto m){
+            const long long warp_min=(long long)c->num_sms*decltype(m)::value*(XFER_THREADS/32);   // the warps resident
+            launch_dep(c,k_p2g_scatter<decltype(m)::value>,grid_for(c,c->xfer_grid),XFER_THREADS,(XFER_THREADS/32)*scatter_warp_bytes(),st,S2,warp_min);});
+        counted(c,PH_P2G);}
     {PhaseScope ps(c,PH_GRID,st);launch_dep(c,k_grid_update<TT<P>>,grid_for(c,c->node_grid),NODE_THREADS,0,st,S2);counted(c,PH_GRID);}
     if(stop_after==1||stop_after==2) return S2;
     {PhaseScope ps(c,PH_HESS,st);
@@ -713,7 +724,8 @@ template<class T> __global__ void k_vmax(DevState<T> S,int scene,unsigned long l
 template<class P> void set_smem_limits()
 {
     for(int v:kXferVariants) with_minb(v,[&](auto m){
-        cudaFuncSetAttribute(k_p2g<P,decltype(m)::value>,cudaFuncAttributeMaxDynamicSharedMemorySize,p2g_smem_bytes<TT<P>>(4096));
+        if constexpr(sizeof(TT<P>)==8)
+            cudaFuncSetAttribute(k_p2g<decltype(m)::value>,cudaFuncAttributeMaxDynamicSharedMemorySize,p2g_smem_bytes<TT<P>>(4096));
         cudaFuncSetAttribute(k_hessian<P,false,decltype(m)::value>,cudaFuncAttributeMaxDynamicSharedMemorySize,hess_kernel_smem_bytes<TT<P>>());
         cudaFuncSetAttribute(k_hessian<P,true,decltype(m)::value>,cudaFuncAttributeMaxDynamicSharedMemorySize,hess_kernel_smem_bytes<TT<P>>());});
 }
@@ -779,7 +791,7 @@ template<class P> void enqueue_volume_pass(mpm_context* c)
     // always the full sort: before the first grid build the previous keys are all ones, so
     // every particle would count as moved
     const int inc=c->sort_incremental;c->sort_incremental=0;
-    enqueue_binning<P>(c,st,S);
+    enqueue_binning<P>(c,st,S,false);
     c->sort_incremental=inc;
     k_permute<TT<P>><<<grid_for(c,4),256,0,st>>>(S);counted(c,PH_P2G);
     DevState<TT<P>> S2=make_state<P>(c,c->cur^1,0.0);

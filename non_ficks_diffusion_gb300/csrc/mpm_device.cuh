@@ -4,8 +4,8 @@
 // ([field][capacity]): X0..2, V0..2, Fe00..Fe22 (row-major), Jp, m, V0, lambda0, mu0.
 // Two such buffers alternate every substep: the transfer kernel reads particle i of the
 // old buffer through the sort permutation and writes it to slot i of the new one, so the
-// state is always stored in cell order. A per-particle cache of the CG's Hessian action
-// (stencil coordinates, left stretch and three coefficients) is written by the same kernel.
+// state is always stored in cell order. The same kernel writes a per-particle cache of what
+// the scatter and the CG's Hessian action need (stencil coordinates, strain, coefficients).
 //
 // Grid: 4x4x4 node blocks. Cell (i,j,k) of a scene with counts n is stored at block
 // (b = (i+4)>>2, ...), local (l = (i+4)&3, ...); each scene owns a dense range of
@@ -20,11 +20,11 @@ namespace mpm {
 
 constexpr int NB_FIELDS=20;
 enum { FX=0, FV=3, FF=6, FJP=15, FM=16, FV0=17, FLAM0=18, FMU0=19 };
-// CG cache: V4 vectors per particle ([vector][capacity]), written by P2G in the order of the
-// new buffer and read by every Hessian product: (x0, x1, x2, c1), (Sxx, Sxy, Sxz, Syy),
-// (Syz, Szz, c2, c3) with the stencil coordinates x and the coefficients of HessianData
-// (mpm_math.cuh); FP64 adds the six entries of its K inverse in two more vectors.
-template<class T> __host__ __device__ constexpr int cg_vectors(){return sizeof(T)==8?5:3;}
+// Transfer cache: V4 vectors per particle ([vector][capacity]) in the order of the new buffer,
+// written before the scatter and read by it and by every Hessian product: (x0, x1, x2, c1),
+// (Exx, Exy, Exz, Eyy), (Eyz, Ezz, c2, c3) with the stencil coordinates x and HessianData
+// (mpm_math.cuh); then FP32 has (m, V0, V1, V2), FP64 the six entries of its K inverse.
+template<class T> __host__ __device__ constexpr int cg_vectors(){return sizeof(T)==8?5:4;}
 constexpr unsigned KEY_SENTINEL=0xFFFFFFFFu;
 constexpr int MAX_BARRIERS=16;
 constexpr int MAX_SCENES=256;
@@ -79,7 +79,7 @@ struct SceneRange { int c0,c1,b0,b1; };
 // scenes' work items and nodes.
 struct ActiveList { int n; int scene[MAX_SCENES]; int cpre[MAX_SCENES+1]; int bpre[MAX_SCENES+1]; };
 
-// Record of a work item, ITEM_WORDS ints, written by P2G for the later transfer kernels: first
+// Record of a work item, ITEM_WORDS ints, written for the later transfer kernels: first
 // slot, particles, scene, length of the pair table (FP32), and the active indices of the 27
 // blocks around it (-1: inactive). One 128-byte load replaces a chain of five dependent ones
 // (start, key, scene, bitmap, block map).
@@ -129,8 +129,9 @@ template<class T> struct DevState {
     unsigned* keys; int* perm;      // sorted keys and source slots (output of the sort)
     // work items
     int* chunk_start; long long chunk_cap;
+    int* src;                       // FP32: old slot of every new position (k_items)
     unsigned* pairs;                // FP32 pair tables, a work item's from its first slot on (see pair_table)
-    int* items;                     // work-item records, written by P2G
+    int* items;                     // work-item records
     // blocks
     unsigned* bitmap; long long bitmap_words;
     int* blockmap;                  // global block id -> active index (valid where the bitmap bit is set)

@@ -706,23 +706,31 @@ template<class T> MPM_HD void dP_dF(const T* Fe,const T* Re,const T lambda,const
     for(int k=0;k<9;++k) dP[k]=m2*(dF[k]-dR[k])+lh*H[k]+lj*dH[k];
 }
 
-// The elastic Hessian of one particle in the rotation-free form the CG products use. With the
-// left polar form F = S R (S = R F^T symmetric), J = det F and dF = G F:
+// The stress and the elastic Hessian of one particle in the rotation-free form of the
+// transfers. With the left polar form F = S R (S symmetric), E = S - I, J = det F and dF = G F:
 //   dF F^T = G S^2,  cof(F) F^T = J I,  cof(F):dF = J tr G,  d(cof F) F^T = J (tr G I - G^T),
-// and R W R^T = W' solves W' S + S W' = M - M^T for M = G S, so that dP of dP_dF becomes
+// and R W R^T = W' solves W' S + S W' = M - M^T for M = G S, so that P of stress_P and dP of
+// dP_dF become
+//   V0 P F^T  = c1 E S + c3 I,
 //   V0 dP F^T = c1 (M - W') S + c2 tr G I - c3 G^T,
 //   c1 = 2 mu V0,  c3 = lambda V0 J (J - 1),  c2 = lambda V0 J^2 + c3.
 // Nine numbers and about 110 operations per product instead of Fe, Re, lambda, mu and V0
-// (21) and about 260. An EOS fluid is S = I, c1 = c3 = 0 with its coefficient in c2.
-template<class T> struct HessianData { T S[6],c1,c2,c3; };     // S: xx, xy, xz, yy, yz, zz
+// (21) and about 260. E is kept, not S, and formed from F - R, so that a small strain keeps
+// its relative accuracy (the stress is as accurate as stress_P's from the same F and R). An
+// EOS fluid has c1 = c3 = 0, its coefficient of the product in c2 and that of the explicit
+// force in Exx.
+template<class T> struct HessianData { T E[6],c1,c2,c3; };     // E: xx, xy, xz, yy, yz, zz
 template<class T> MPM_HD void hessian_data(const T* F,const T* R,const T lambda,const T mu,const T Je,const T V0,HessianData<T>& h)
 {
-    T Q[9];mat_mul_bt(R,F,Q);
-    h.S[0]=Q[0];h.S[1]=T(0.5)*(Q[1]+Q[3]);h.S[2]=T(0.5)*(Q[2]+Q[6]);
-    h.S[3]=Q[4];h.S[4]=T(0.5)*(Q[5]+Q[7]);h.S[5]=Q[8];
+    T D[9],Q[9];
+#pragma unroll
+    for(int k=0;k<9;++k) D[k]=F[k]-R[k];
+    mat_mul_bt(R,D,Q);
+    h.E[0]=Q[0];h.E[1]=T(0.5)*(Q[1]+Q[3]);h.E[2]=T(0.5)*(Q[2]+Q[6]);
+    h.E[3]=Q[4];h.E[4]=T(0.5)*(Q[5]+Q[7]);h.E[5]=Q[8];
     h.c1=T(2)*mu*V0;h.c3=lambda*V0*(Je*(Je-T(1)));h.c2=lambda*V0*(Je*Je)+h.c3;
 }
-// Inverse of the 3x3 matrix K of W' (entries 00, 01, 02, 11, 12, 22).
+// Inverse of the 3x3 matrix K of W' (entries 00, 01, 02, 11, 12, 22), S = I + E.
 template<class T> MPM_HD void skew_system_inverse(const T* S,T* Ki)
 {
     const T k00=S[3]+S[0],k01=S[4],k02=-S[2],k11=S[5]+S[0],k12=S[1],k22=S[5]+S[3];

@@ -63,6 +63,12 @@ template<class T> struct ChunkInfo {
     int b[3];        // block coordinates inside the scene
     long long gb;
 };
+// Block coordinates of global block gb of a scene (block ids have 26 bits: 32-bit divisions).
+template<class T> __device__ __forceinline__ void block_coords(const SceneDev<T>& sc,long long gb,int* b)
+{
+    const unsigned lb=(unsigned)(gb-sc.block_base),n0=(unsigned)sc.nb[0],n1=(unsigned)sc.nb[1],q=lb/n0,q2=q/n1;
+    b[0]=(int)(lb-q*n0);b[1]=(int)(q-q2*n1);b[2]=(int)q2;
+}
 // The geometry of work item c; lanes (threads) 0..26 of the caller fill nbr[27].
 template<class T> __device__ __forceinline__ bool load_chunk(const DevState<T>& S,long long c,unsigned nc,unsigned nv,ChunkInfo<T>& ci,int* nbr,
                                                              int lane=-1)
@@ -73,8 +79,7 @@ template<class T> __device__ __forceinline__ bool load_chunk(const DevState<T>& 
     ci.gb=(long long)(S.keys[ci.s]>>6);
     ci.scene=scene_of_block(S.scene_block_base,S.n_scenes,ci.gb);
     const SceneDev<T>& sc=S.scenes[ci.scene];
-    long long lb=ci.gb-sc.block_base;
-    ci.b[0]=(int)(lb%sc.nb[0]);lb/=sc.nb[0];ci.b[1]=(int)(lb%sc.nb[1]);ci.b[2]=(int)(lb/sc.nb[1]);
+    block_coords(sc,ci.gb,ci.b);
     if(lane<27){
         const int ox=lane%3-1,oy=(lane/3)%3-1,oz=lane/9-1;
         const long long g2=ci.gb+ox+(long long)sc.nb[0]*(oy+(long long)sc.nb[1]*oz);
@@ -122,10 +127,9 @@ template<class T> __device__ __forceinline__ void make_stencil(const SceneDev<T>
 // Node centre of a grid node.
 template<class T> __device__ __forceinline__ void node_center(const DevState<T>& S,const SceneDev<T>& sc,long long node,int blk,T* x)
 {
-    long long lb=(long long)S.active_gb[blk]-sc.block_base;
-    const int bx=(int)(lb%sc.nb[0]);lb/=sc.nb[0];const int by=(int)(lb%sc.nb[1]),bz=(int)(lb/sc.nb[1]);
+    int b[3];block_coords(sc,S.active_gb[blk],b);
     const int l=(int)(node&63);
-    const int c[3]={4*bx+(l&3)-4,4*by+((l>>2)&3)-4,4*bz+(l>>4)-4};
+    const int c[3]={4*b[0]+(l&3)-4,4*b[1]+((l>>2)&3)-4,4*b[2]+(l>>4)-4};
 #pragma unroll
     for(int a=0;a<3;++a) x[a]=((T)c[a]+(T)0.5)*sc.dx[a];
 }
@@ -340,7 +344,7 @@ __device__ __forceinline__ int list_find(const ListSmem& sm,int w)
 // cell order of a work item of up to `chunk` particles (per-warp cell counts, slot -> item
 // map, item cells).
 template<class T> __host__ __device__ constexpr int p2g_tile_bytes(){return (XFER_THREADS/32)*7*TILE_S*(int)sizeof(T);}
-__host__ __device__ constexpr int order_bytes(int chunk){return (XFER_THREADS/32)*64*4+((chunk*3+15)&~15);}
+__host__ __device__ constexpr int order_bytes(int chunk){return (XFER_THREADS/32)*64*4+64*4+((chunk*5+15)&~15);}
 template<class T> __host__ __device__ constexpr int p2g_smem_bytes(int chunk){return p2g_tile_bytes<T>()+order_bytes(chunk);}
 template<class T> constexpr int hess_smem_bytes(){return (XFER_THREADS/32)*3*TILE_S*(int)sizeof(T)+3*TILE_S*(int)sizeof(T);}
 template<class T> constexpr int hess_warp_smem_bytes(){return (XFER_THREADS/32)*6*TILE_S*(int)sizeof(T);}
@@ -388,26 +392,37 @@ __device__ __forceinline__ void chunk_runs(int np,int stride,int* run)
 
 // Stable counting sort of a work item's particles by the scatter rank of their cell (the
 // low 6 key bits through crank): on return inv[k] is the item position of the k-th
-// particle in (rank, item position) order, and cellv[j] the cell of item position j. Warp
-// w owns the item positions [w*seg, (w+1)*seg); a first pass counts ranks per warp, a warp
-// scan turns the counts into (rank, warp)-major offsets, and a second pass places every
-// particle. The particles of a block keep their order from one substep to the next (the
-// block sort is stable), so writing the new buffer in this order makes the chunk
-// rank-sorted for the Hessian and G2P of this substep and nearly so for the next P2G.
-__device__ __forceinline__ void chunk_cell_order(const unsigned* keys,int s,int np,const unsigned char* crank,int (*cnt)[64],unsigned short* inv,unsigned char* cellv)
+// particle in (rank, item position) order, cellv[j] the cell of item position j, and
+// cnt[w][r] where warp w's particles of rank r begin. Warp w owns the item positions [w*seg,
+// (w+1)*seg): it numbers its particles inside their cell (loc) and counts the ranks, a warp
+// scan turns the counts into (rank, warp)-major offsets, and every particle is placed. The
+// particles of a block keep their order from one substep to the next (the block sort is
+// stable), so writing the new buffer in this order makes the chunk rank-sorted for the
+// Hessian and G2P of this substep and nearly so for the next P2G. Returns the end of rank r
+// in rank_end[r].
+__device__ __forceinline__ void chunk_cell_order(const unsigned* keys,int s,int np,const unsigned char* crank,int (*cnt)[64],unsigned short* inv,
+    unsigned short* loc,unsigned char* cellv,int* rank_end)
 {
     const int lane=threadIdx.x&31,warp=threadIdx.x>>5,nw=blockDim.x>>5;
     for(int t=threadIdx.x;t<nw*64;t+=blockDim.x) (&cnt[0][0])[t]=0;
     __syncthreads();
     const int seg=(np+nw-1)/nw,b0=warp*seg,b1=min(np,b0+seg);
     const unsigned below=lane_bits_below();
+    unsigned key=b0+lane<b1?keys[s+b0+lane]:0u;
     for(int g=b0;g<b1;g+=32){
         const int j=g+lane;const bool ok=j<b1;
-        const unsigned cell=ok?(keys[s+j]&63u):0u;
-        if(ok) cellv[j]=(unsigned char)cell;
-        const unsigned rk=ok?(unsigned)crank[cell]:64u+lane;
-        const unsigned peers=__match_any_sync(0xffffffffu,rk);
-        if(ok&&(peers&below)==0) cnt[warp][rk]+=__popc(peers);
+        const unsigned cell=key&63u;
+        key=j+32<b1?keys[s+j+32]:0u;
+        const unsigned rk=crank[cell];
+        // lanes of the same cell by six ballots (match.any costs more the more cells a warp has)
+        unsigned peers=__ballot_sync(0xffffffffu,ok);
+#pragma unroll
+        for(int b=0;b<6;++b){const bool bit=(cell>>b)&1u;const unsigned m=__ballot_sync(0xffffffffu,bit);peers&=bit?m:~m;}
+        const int before=ok?cnt[warp][rk]:0,rank=__popc(peers&below);
+        __syncwarp();
+        if(ok){
+            cellv[j]=(unsigned char)cell;loc[j]=(unsigned short)(before+rank);
+            if(rank==0) cnt[warp][rk]=before+__popc(peers);}
         __syncwarp();}
     __syncthreads();
     if(warp==0){
@@ -418,18 +433,12 @@ __device__ __forceinline__ void chunk_cell_order(const unsigned* keys,int s,int 
 #pragma unroll
         for(int o=1;o<32;o<<=1){const int u=__shfl_up_sync(0xffffffffu,incl,o);if(lane>=o) incl+=u;}
         int o0=incl-(t0+t1),o1=o0+t0;
+        rank_end[c0]=o1;rank_end[c1]=incl;
         for(int w=0;w<nw;++w){
             const int a=cnt[w][c0],b=cnt[w][c1];
             cnt[w][c0]=o0;o0+=a;cnt[w][c1]=o1;o1+=b;}}
     __syncthreads();
-    for(int g=b0;g<b1;g+=32){
-        const int j=g+lane;const bool ok=j<b1;
-        const unsigned rk=ok?(unsigned)crank[cellv[j]]:64u+lane;
-        const unsigned peers=__match_any_sync(0xffffffffu,rk);
-        if(ok) inv[cnt[warp][rk]+__popc(peers&below)]=(unsigned short)j;
-        __syncwarp();
-        if(ok&&(peers&below)==0) cnt[warp][rk]+=__popc(peers);
-        __syncwarp();}
+    for(int j=b0+lane;j<b1;j+=32) inv[cnt[warp][crank[cellv[j]]]+loc[j]]=(unsigned short)j;
     __syncthreads();
 }
 
@@ -456,11 +465,17 @@ __device__ __forceinline__ double cy(const C3<double>& a){return a.y;}
 // distinct banks wherever a level has enough cells. Entry: positions of the two
 // particles in the item (12 bits each), cell (6 bits), PAIR_TWO when there is a second one.
 constexpr unsigned PAIR_TWO=1u<<30;
-__device__ __forceinline__ unsigned pair_entry(int k,bool two,unsigned cell,int stride,const int* run)
+// Stored position of cell-ordered slot k of a work item (chunk_runs); rs = 1/stride. The
+// quotient is exact: k + 1/2 lies at least 1/256 from a multiple of stride <= 128, in units of
+// the quotient, and FP32 rounding of values below 4,096 stays under that.
+__device__ __forceinline__ int slot_position(int k,int stride,float rs,const int* run)
 {
-    const int L0=k/stride,p0=run[k-L0*stride]+L0;
-    int p1=p0;
-    if(two){const int L1=(k+1)/stride;p1=run[k+1-L1*stride]+L1;}
+    const int L=(int)(((float)k+0.5f)*rs);
+    return run[k-L*stride]+L;
+}
+__device__ __forceinline__ unsigned pair_entry(int k,bool two,unsigned cell,int stride,float rs,const int* run)
+{
+    const int p0=slot_position(k,stride,rs,run),p1=two?slot_position(k+1,stride,rs,run):p0;
     return (unsigned)p0|((unsigned)p1<<12)|(cell<<24)|(two?PAIR_TWO:0u);
 }
 // Called by every warp of the CTA, which writes the levels warp, warp + nw, ...; rank_end[r] is
@@ -474,6 +489,7 @@ __device__ __forceinline__ int pair_table(const int* rank_end,const unsigned cha
     if(lane==0) s0=0;
     const unsigned below=lane_bits_below();
     const unsigned c0=cell_of[2*lane],c1=cell_of[2*lane+1];
+    const float rs=1.f/(float)stride;
     int base=0;
     for(int j=0,mine=warp;;++j){
         const int k0=s0+2*j,k1=e0+2*j;
@@ -482,8 +498,8 @@ __device__ __forceinline__ int pair_table(const int* rank_end,const unsigned cha
         const int b1=base+__popc(m0);
         if(j==mine){                                   // uniform over the warp
             mine+=nw;
-            if(k0<e0) out[base+__popc(m0&below)]=pair_entry(k0,k0+1<e0,c0,stride,run);
-            if(k1<e1) out[b1+__popc(m1&below)]=pair_entry(k1,k1+1<e1,c1,stride,run);}
+            if(k0<e0) out[base+__popc(m0&below)]=pair_entry(k0,k0+1<e0,c0,stride,rs,run);
+            if(k1<e1) out[b1+__popc(m1&below)]=pair_entry(k1,k1+1<e1,c1,stride,rs,run);}
         base=b1+__popc(m1);}
     return base;
 }
@@ -528,77 +544,87 @@ struct ScatterRounds {
     }
 };
 
-// One pass of a work item's particles through P2G: pass qi gives lane L the cell-ordered
-// particle L*stride + qi (item position inv[k] in the sorted order, read through the sort
-// permutation from the old buffer), which is stored at position run[qi] + L of the new
-// buffer. Precompute (plasticity), the new buffer's state, cache and key, then the scatter
-// of m, m v and f into the warp's tile in rounds of lanes in distinct cells. Called by
-// every lane of the warp.
-template<class P> __device__ __forceinline__ void p2g_pass(const DevState<typename P::T>& S,const SceneDev<typename P::T>& sc,
-    const ChunkInfo<typename P::T>& ci,const int* run,const unsigned short* inv,const unsigned char* cellv,int qi,int stride,int np,
-    typename P::T (*tile)[TILE_S])
+// Plasticity and transfer data of the particle in old slot src, for position i of the new buffer
+// (cell `cell` of block b): the state, the cache and its identity are written there.
+// Returned: stencil coordinates, HessianData, mass and velocity.
+template<class T> struct Transferred { T x[3],m,V[3];HessianData<T> h; };
+template<class P> __device__ __forceinline__ void update_particle(const DevState<typename P::T>& S,const SceneDev<typename P::T>& sc,const int* b,unsigned cell,
+    int src,long long i,Transferred<typename P::T>& o)
 {
     using T=typename P::T; using TS=typename P::TS;
-    // cell-ordered slot k: item position inv[k] in, position run[qi] + lane out
+    const long long pc=S.pcap;
+    const T* Pin=S.pcur;T* Pout=S.pnxt;
+    T F[9],X[3];
+#pragma unroll
+    for(int a=0;a<3;++a){X[a]=Pin[(FX+a)*pc+src];o.V[a]=Pin[(FV+a)*pc+src];}
+#pragma unroll
+    for(int k=0;k<9;++k) F[k]=Pin[(FF+k)*pc+src];
+    T Jp=Pin[FJP*pc+src];
+    o.m=Pin[FM*pc+src];
+    const T V0=Pin[FV0*pc+src],lam0=Pin[FLAM0*pc+src],mu0=Pin[FMU0*pc+src];
+    S.pid_nxt[i]=S.pid_cur[src];S.scn_nxt[i]=S.scn_cur[src];
+#pragma unroll
+    for(int a=0;a<3;++a){Pout[(FX+a)*pc+i]=X[a];Pout[(FV+a)*pc+i]=o.V[a];}
+    Pout[FM*pc+i]=o.m;Pout[FV0*pc+i]=V0;Pout[FLAM0*pc+i]=lam0;Pout[FMU0*pc+i]=mu0;
+    stencil_coord(sc,b,cell,X,o.x);
+    if(sc.eos){
+        // EOS fluid (MPM_Example.cpp:737-738): no constitutive update; the density is the Jp
+        // slot. The CG's coefficient V0 k gamma rho^(gamma-1), the explicit V0/rho k rho^(gamma-1).
+        const T pw=tpow(Jp,sc.eos_gamma-T(1));
+        o.h=HessianData<T>{{V0/Jp*sc.bulk*pw,T(0),T(0),T(0),T(0),T(0)},T(0),V0*sc.bulk*sc.eos_gamma*pw,T(0)};}
+    else{
+        T R[9],lam,mu,Je;
+        precompute<T,TS>(F,Jp,lam0,mu0,sc.plastic,sc.hardening,sc.cy,sc.sy,sc.hmax,R,lam,mu,Je);
+        hessian_data(F,R,lam,mu,Je,V0,o.h);}
+#pragma unroll
+    for(int k=0;k<9;++k) Pout[(FF+k)*pc+i]=F[k];
+    Pout[FJP*pc+i]=Jp;
+    S.cache[i]=V4<T>{o.x[0],o.x[1],o.x[2],o.h.c1};
+    S.cache[pc+i]=V4<T>{o.h.E[0],o.h.E[1],o.h.E[2],o.h.E[3]};
+    S.cache[2*pc+i]=V4<T>{o.h.E[4],o.h.E[5],o.h.c2,o.h.c3};
+    if constexpr(sizeof(T)==8){
+        const T Sm[6]={T(1)+o.h.E[0],o.h.E[1],o.h.E[2],T(1)+o.h.E[3],o.h.E[4],T(1)+o.h.E[5]};
+        T Ki[6];skew_system_inverse(Sm,Ki);
+        S.cache[3*pc+i]=V4<T>{Ki[0],Ki[1],Ki[2],Ki[3]};
+        S.cache[4*pc+i]=V4<T>{Ki[4],Ki[5],T(0),T(0)};}
+    else S.cache[3*pc+i]=V4<T>{o.m,o.V[0],o.V[1],o.V[2]};
+}
+// V0 P F^T (00, 01, 02, 11, 12, 22) of HessianData; an EOS fluid's pressure enters as -c I.
+template<class T> __device__ __forceinline__ void transfer_stress(const HessianData<T>& h,bool eos,T* A)
+{
+    const T* E=h.E;
+    A[0]=h.c1*(E[0]+(E[0]*E[0]+E[1]*E[1]+E[2]*E[2]))+h.c3;
+    A[1]=h.c1*(E[1]+(E[0]*E[1]+E[1]*E[3]+E[2]*E[4]));
+    A[2]=h.c1*(E[2]+(E[0]*E[2]+E[1]*E[4]+E[2]*E[5]));
+    A[3]=h.c1*(E[3]+(E[1]*E[1]+E[3]*E[3]+E[4]*E[4]))+h.c3;
+    A[4]=h.c1*(E[4]+(E[1]*E[2]+E[3]*E[4]+E[4]*E[5]));
+    A[5]=h.c1*(E[5]+(E[2]*E[2]+E[4]*E[4]+E[5]*E[5]))+h.c3;
+    if(eos) A[0]=A[3]=A[5]=-E[0];
+}
+
+// FP64: one pass of a work item's particles through P2G. Pass qi gives lane L the cell-ordered
+// particle L*stride + qi (item position inv[k] in the sorted order, read through the sort
+// permutation from the old buffer), which is stored at position run[qi] + L of the new
+// buffer, then scattered (m, m v and f; gravity enters in the grid update) into the warp's
+// tile in rounds of lanes in distinct cells. Called by every lane of the warp.
+__device__ __forceinline__ void p2g_pass(const DevState<double>& S,const SceneDev<double>& sc,const ChunkInfo<double>& ci,const int* run,
+    const unsigned short* inv,const unsigned char* cellv,int qi,int stride,int np,double (*tile)[TILE_S])
+{
+    using T=double;
     const int k=(int)(threadIdx.x&31)*stride+qi;
     const bool valid=k<np;
-    const int i=ci.s+run[qi]+(int)(threadIdx.x&31);
-    T A[9],X[3],V[3],m=T(0);
+    T A[6];
+    Transferred<T> o;
     Stencil<T> st;
     unsigned cell=0;
     if(valid){
-        const long long pc=S.pcap;
         const int jj=inv[k];
-        const int src=S.perm[ci.s+jj];
-        const T* Pin=S.pcur;T* Pout=S.pnxt;
-        T F[9];
-#pragma unroll
-        for(int a=0;a<3;++a){X[a]=Pin[(FX+a)*pc+src];V[a]=Pin[(FV+a)*pc+src];}
-#pragma unroll
-        for(int k=0;k<9;++k) F[k]=Pin[(FF+k)*pc+src];
-        T Jp=Pin[FJP*pc+src];
-        m=Pin[FM*pc+src];
-        const T V0=Pin[FV0*pc+src],lam0=Pin[FLAM0*pc+src],mu0=Pin[FMU0*pc+src];
-        T R[9],lam,mu,Je;
-        if(sc.eos){
-            // EOS fluid (MPM_Example.cpp:737-738): no constitutive update; the
-            // density is the Jp slot. lam: the CG's coefficient V0 k gamma rho^(gamma-1);
-            // mu: the explicit one V0/rho k rho^(gamma-1).
-            const T pw=tpow(Jp,sc.eos_gamma-T(1));
-            lam=V0*sc.bulk*sc.eos_gamma*pw;mu=V0/Jp*sc.bulk*pw;Je=T(1);
-#pragma unroll
-            for(int k=0;k<9;++k) R[k]=(k%4==0)?T(1):T(0);}
-        else precompute<T,TS>(F,Jp,lam0,mu0,sc.plastic,sc.hardening,sc.cy,sc.sy,sc.hmax,R,lam,mu,Je);
-#pragma unroll
-        for(int a=0;a<3;++a){Pout[(FX+a)*pc+i]=X[a];Pout[(FV+a)*pc+i]=V[a];}
-#pragma unroll
-        for(int k=0;k<9;++k) Pout[(FF+k)*pc+i]=F[k];
-        Pout[FJP*pc+i]=Jp;Pout[FM*pc+i]=m;Pout[FV0*pc+i]=V0;Pout[FLAM0*pc+i]=lam0;Pout[FMU0*pc+i]=mu0;
-        S.pid_nxt[i]=S.pid_cur[src];S.scn_nxt[i]=S.scn_cur[src];
-        HessianData<T> h;
-        if(sc.eos){
-            // f += coefficient grad w, i.e. A = -coefficient I
-#pragma unroll
-            for(int k=0;k<9;++k) A[k]=(k%4==0)?-mu:T(0);
-            h=HessianData<T>{{T(1),T(0),T(0),T(1),T(0),T(1)},T(0),lam,T(0)};}
-        else{
-            hessian_data(F,R,lam,mu,Je,V0,h);
-            // V0 P Fe^T
-            T Pk[9];stress_P(F,R,lam,mu,Je,Pk);mat_mul_bt(Pk,F,A);
-#pragma unroll
-            for(int k=0;k<9;++k) A[k]*=V0;}
+        const long long i=ci.s+run[qi]+(int)(threadIdx.x&31);
         cell=cellv[jj];
-        const unsigned key=((unsigned)ci.gb<<6)|cell;
-        S.keys[i]=key;
-        T x[3];stencil_coord(sc,ci.b,cell,X,x);
-        stencil_from_coord(sc,cell,x,st);
-        S.cache[i]=V4<T>{x[0],x[1],x[2],h.c1};
-        S.cache[pc+i]=V4<T>{h.S[0],h.S[1],h.S[2],h.S[3]};
-        S.cache[2*pc+i]=V4<T>{h.S[4],h.S[5],h.c2,h.c3};
-        if constexpr(sizeof(T)==8){
-            T Ki[6];skew_system_inverse(h.S,Ki);
-            S.cache[3*pc+i]=V4<T>{Ki[0],Ki[1],Ki[2],Ki[3]};
-            S.cache[4*pc+i]=V4<T>{Ki[4],Ki[5],T(0),T(0)};}}
+        update_particle<PrecFP64>(S,sc,ci.b,cell,S.perm[ci.s+jj],i,o);
+        S.keys[i]=((unsigned)ci.gb<<6)|cell;
+        transfer_stress(o.h,sc.eos!=0,A);
+        stencil_from_coord(sc,cell,o.x,st);}
     const ScatterRounds R(valid,cell);
     for(int r=0;r<R.rounds;++r){
         const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
@@ -606,46 +632,26 @@ template<class P> __device__ __forceinline__ void p2g_pass(const DevState<typena
             const int tb=tile_addr(st.r[0]-1,st.r[1]-1,st.r[2]-1);
 #pragma unroll
             for(int k=0;k<3;++k){opaque(st.w[0][k]);opaque(st.dw[0][k]);}
-            const T mv0=m*V[0],mv1=m*V[1],mv2=m*V[2];
-            const T mg0=sc.gravity[0]*m,mg1=sc.gravity[1]*m,mg2=sc.gravity[2]*m;
+            const T mv0=o.m*o.V[0],mv1=o.m*o.V[1],mv2=o.m*o.V[2];
 #pragma unroll
             for(int ox=0;ox<3;++ox)
 #pragma unroll
             for(int oy=0;oy<3;++oy){
-                // at this (x, y): w = wxy wz and f_a = m g_a w - sum_k A_ak grad_k w
-                // = al_a wz - be_a dwz
+                // at this (x, y): w = wxy wz and f_a = -sum_k A_ak grad_k w = -(al_a wz + be_a dwz)
                 const T dxy=st.dw[0][ox]*st.w[1][oy],xdy=st.w[0][ox]*st.dw[1][oy],wxy=st.w[0][ox]*st.w[1][oy];
-                const T cm=m*wxy,cv0=mv0*wxy,cv1=mv1*wxy,cv2=mv2*wxy;
-                const T al0=mg0*wxy-(A[0]*dxy+A[1]*xdy),al1=mg1*wxy-(A[3]*dxy+A[4]*xdy),al2=mg2*wxy-(A[6]*dxy+A[7]*xdy);
-                const T be0=A[2]*wxy,be1=A[5]*wxy,be2=A[8]*wxy;
-                if constexpr(sizeof(T)==4){
-                    // channels (0, 1), (2, 3) and (4, 5) as packed pairs, channel 6 scalar:
-                    // each lane of a pair is the same fused multiply-add as the scalar form
-                    const float2 c01=make_float2(cm,cv0),c23=make_float2(cv1,cv2);
-                    const float2 al45=make_float2(al0,al1),nbe45=make_float2(-be0,-be1);
+                const T cm=o.m*wxy,cv0=mv0*wxy,cv1=mv1*wxy,cv2=mv2*wxy;
+                const T al0=-(A[0]*dxy+A[1]*xdy),al1=-(A[1]*dxy+A[3]*xdy),al2=-(A[2]*dxy+A[4]*xdy);
+                const T be0=A[2]*wxy,be1=A[4]*wxy,be2=A[5]*wxy;
 #pragma unroll
-                    for(int oz=0;oz<3;++oz){
-                        const T wz=st.w[2][oz],dz=st.dw[2][oz];
-                        const int t=tb+tile_addr(ox,oy,oz);
-                        const float2 q01=pfma(c01,pdup(wz),make_float2(tile[0][t],tile[1][t]));
-                        const float2 q23=pfma(c23,pdup(wz),make_float2(tile[2][t],tile[3][t]));
-                        const float2 q45=pfma(nbe45,pdup(dz),pfma(al45,pdup(wz),make_float2(tile[4][t],tile[5][t])));
-                        tile[0][t]=q01.x;tile[1][t]=q01.y;tile[2][t]=q23.x;tile[3][t]=q23.y;
-                        tile[4][t]=q45.x;tile[5][t]=q45.y;
-                        tile[6][t]=tfma(-be2,dz,tfma(al2,wz,tile[6][t]));
-                        __syncwarp(rmask);}}
-                else{
-#pragma unroll
-                    for(int oz=0;oz<3;++oz){
-                        const T wz=st.w[2][oz],dz=st.dw[2][oz];
-                        const int t=tb+tile_addr(ox,oy,oz);
-                        tile[0][t]=tfma(cm,wz,tile[0][t]);
-                        tile[1][t]=tfma(cv0,wz,tile[1][t]);tile[2][t]=tfma(cv1,wz,tile[2][t]);tile[3][t]=tfma(cv2,wz,tile[3][t]);
-                        // two fused multiply-adds per channel: tile + al wz - be dz
-                        tile[4][t]=tfma(-be0,dz,tfma(al0,wz,tile[4][t]));
-                        tile[5][t]=tfma(-be1,dz,tfma(al1,wz,tile[5][t]));
-                        tile[6][t]=tfma(-be2,dz,tfma(al2,wz,tile[6][t]));
-                        __syncwarp(rmask);}}}}
+                for(int oz=0;oz<3;++oz){
+                    const T wz=st.w[2][oz],dz=st.dw[2][oz];
+                    const int t=tb+tile_addr(ox,oy,oz);
+                    tile[0][t]=tfma(cm,wz,tile[0][t]);
+                    tile[1][t]=tfma(cv0,wz,tile[1][t]);tile[2][t]=tfma(cv1,wz,tile[2][t]);tile[3][t]=tfma(cv2,wz,tile[3][t]);
+                    tile[4][t]=tfma(-be0,dz,tfma(al0,wz,tile[4][t]));
+                    tile[5][t]=tfma(-be1,dz,tfma(al1,wz,tile[5][t]));
+                    tile[6][t]=tfma(-be2,dz,tfma(al2,wz,tile[6][t]));
+                    __syncwarp(rmask);}}}
         __syncwarp();}
 }
 
@@ -669,25 +675,34 @@ template<class T> __device__ __forceinline__ void p2g_copy_removed(const DevStat
         S.pid_nxt[i]=S.pid_cur[src];S.scn_nxt[i]=S.scn_cur[src];}
 }
 
-// Work items handled by the whole CTA: the four warps sort the item's particles by cell
-// together, take its passes in turn into their own tiles, and the tiles are summed at the
-// flush.
-template<class P,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) k_p2g(DevState<typename P::T> S)
+// The record of a work item, by one warp (lanes 0..31); `pairs` the length of its pair table.
+template<class T> __device__ __forceinline__ void write_item(const DevState<T>& S,long long c,const ChunkInfo<T>& ci,const int* nbr,int np,int pairs)
+{
+    const int lane=threadIdx.x&31;
+    S.items[c*ITEM_WORDS+lane]=lane==ITEM_START?ci.s:lane==ITEM_COUNT?np:lane==ITEM_SCENE?ci.scene:lane==ITEM_PAIRS?pairs:
+                               lane-ITEM_NBR<27?nbr[lane-ITEM_NBR]:-1;
+}
+// FP64: plasticity and scatter in one kernel, a CTA per work item. The four warps sort the
+// item's particles by cell together, take its passes in turn into their own tiles, and the
+// tiles are summed at the flush.
+template<int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) k_p2g(DevState<double> S)
 {
     pdl_enter();
-    using T=typename P::T;
+    using T=double;
     constexpr int NW=XFER_THREADS/32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T (*acc)[7][TILE_S]=reinterpret_cast<T (*)[7][TILE_S]>(smem_raw);   // [warp][channel][node]
     int (*ocnt)[64]=reinterpret_cast<int (*)[64]>(smem_raw+p2g_tile_bytes<T>());
-    unsigned short* inv=reinterpret_cast<unsigned short*>(smem_raw+p2g_tile_bytes<T>()+NW*64*4);
-    unsigned char* cellv=reinterpret_cast<unsigned char*>(inv+S.chunk);
-    __shared__ unsigned char crank[64],cell_of[64];
+    int* rank_end=reinterpret_cast<int*>(ocnt+NW);
+    unsigned short* inv=reinterpret_cast<unsigned short*>(rank_end+64);
+    unsigned short* loc=inv+S.chunk;
+    unsigned char* cellv=reinterpret_cast<unsigned char*>(loc+S.chunk);
+    __shared__ unsigned char crank[64];
     __shared__ int nbr[27];
     __shared__ int run[129];
     const int warp=threadIdx.x>>5;
     const unsigned nc=min(S.ctr->n_chunks,(unsigned)S.chunk_cap),nv=S.ctr->n_valid;
-    if(threadIdx.x<64){crank[threadIdx.x]=cell_ranks.rank[threadIdx.x];cell_of[threadIdx.x]=cell_ranks.cell[threadIdx.x];}   // read after the next barrier
+    if(threadIdx.x<64) crank[threadIdx.x]=cell_ranks.rank[threadIdx.x];   // read after the next barrier
     for(long long c=blockIdx.x;c<nc;c+=gridDim.x){
         ChunkInfo<T> ci;
         load_chunk(S,c,nc,nv,ci,nbr);
@@ -695,21 +710,13 @@ template<class P,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) 
         // a work item longer than `chunk` only arises when the work-item capacity was exceeded;
         // an empty record keeps the later kernels off it
         const bool over=np>S.chunk;
-        if(warp==0){
-            __syncwarp();                              // nbr was written by this warp
-            const int lane=threadIdx.x&31;
-            if(lane<ITEM_PAIRS||(lane==ITEM_PAIRS&&over)||lane>=ITEM_NBR)
-                S.items[c*ITEM_WORDS+lane]=lane==ITEM_START?ci.s:lane==ITEM_COUNT?(over?0:np):lane==ITEM_SCENE?ci.scene:
-                                           lane==ITEM_PAIRS?0:lane-ITEM_NBR<27?nbr[lane-ITEM_NBR]:-1;}
+        if(warp==0){__syncwarp();write_item(S,c,ci,nbr,over?0:np,0);}
         if(over){if(threadIdx.x==0) atomicOr(&S.ctr->error,ERR_CAPACITY);continue;}   // uniform
         if(warp==0) chunk_runs(np,stride,run);        // read after the barriers in chunk_cell_order
         for(int t=threadIdx.x;t<NW*7*TILE_S;t+=blockDim.x) (&acc[0][0][0])[t]=T(0);
-        chunk_cell_order(S.keys,ci.s,np,crank,ocnt,inv,cellv);
-        if constexpr(sizeof(T)==4){                   // the last warp's counts now hold the ends of the ranks
-            const int m=pair_table(ocnt[NW-1],cell_of,stride,run,S.pairs+ci.s);
-            if(threadIdx.x==0) S.items[c*ITEM_WORDS+ITEM_PAIRS]=m;}
+        chunk_cell_order(S.keys,ci.s,np,crank,ocnt,inv,loc,cellv,rank_end);
         const SceneDev<T>& sc=S.scenes[ci.scene];
-        for(int qi=warp;qi<stride;qi+=NW) p2g_pass<P>(S,sc,ci,run,inv,cellv,qi,stride,np,acc[warp]);
+        for(int qi=warp;qi<stride;qi+=NW) p2g_pass(S,sc,ci,run,inv,cellv,qi,stride,np,acc[warp]);
         __syncthreads();
         for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x){
             const int ta=tile_addr(t);
@@ -725,6 +732,28 @@ template<class P,int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) 
     p2g_copy_removed(S,nv);
 }
 
+// FP32, the particle part of P2G: one thread per position of the new buffer (k_items ordered
+// them). Apart from the scatter it needs no shared memory, spreads a small scene's particles
+// over all SMs and keeps the plasticity's code out of the scatter's loop, where the two
+// together overran the instruction cache (38 % of the stall cycles on yielding particles).
+// Ordering, particles and scatter against the one kernel before: 0.71 -> 0.50 ms (1.94M particles,
+// nearly all yielding), 2.15 -> 1.75 ms (64-scene batch), 82 -> 62 us (60K), 2.78 -> 2.74 ms
+// (21.5M unstrained particles). Bound by instruction issue where particles yield, else by HBM.
+template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_particles(DevState<typename P::T> S)
+{
+    pdl_enter();
+    using T=typename P::T;
+    const long long nv=S.ctr->n_valid;
+    for(long long i=blockIdx.x*(long long)blockDim.x+threadIdx.x;i<nv;i+=(long long)gridDim.x*blockDim.x){
+        const int src=S.src[i];
+        const unsigned key=S.keys[i];
+        const SceneDev<T>& sc=S.scenes[S.scn_cur[src]];
+        int b[3];block_coords(sc,(long long)(key>>6),b);
+        Transferred<T> o;
+        update_particle<P>(S,sc,b,key&63u,src,i,o);}
+    p2g_copy_removed(S,(unsigned)nv);
+}
+
 // Full permutation of the particle state (first grid build, before any P2G).
 template<class T> __global__ void __launch_bounds__(256) k_permute(DevState<T> S)
 {
@@ -735,18 +764,54 @@ template<class T> __global__ void __launch_bounds__(256) k_permute(DevState<T> S
         S.pid_nxt[i]=S.pid_cur[src];S.scn_nxt[i]=S.scn_cur[src];}
 }
 
-// Clears the accumulated node channels and records each scene's range in the work-item
-// list and in the active-block list (SceneRange; the ranges were zeroed before the key pass).
-template<class T> __global__ void __launch_bounds__(256) k_clear_nodes(DevState<T> S)
+// Clears the accumulated node channels, records each scene's range in the work-item list and
+// in the active-block list (SceneRange; the ranges were zeroed before the key pass) and, with
+// `order` (FP32 substeps), puts each work item's particles in storage order: their old slots
+// and keys by new position, the pair table and the record.
+template<class T> __global__ void __launch_bounds__(XFER_THREADS) k_items(DevState<T> S,int order)
 {
     pdl_enter();
+    constexpr int NW=XFER_THREADS/32;
     const long long na=(long long)min(S.ctr->n_active,(unsigned)S.block_cap);
     const long long nn=na*64;
     const long long t0=blockIdx.x*(long long)blockDim.x+threadIdx.x,stride=(long long)gridDim.x*blockDim.x;
+    const unsigned nc=min(S.ctr->n_chunks,(unsigned)S.chunk_cap),nv=S.ctr->n_valid;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    int (*ocnt)[64]=reinterpret_cast<int (*)[64]>(smem_raw);
+    int* rank_end=reinterpret_cast<int*>(ocnt+NW);
+    unsigned short* inv=reinterpret_cast<unsigned short*>(rank_end+64);
+    unsigned short* loc=inv+S.chunk;
+    unsigned char* cellv=reinterpret_cast<unsigned char*>(loc+S.chunk);
+    __shared__ unsigned char crank[64],cell_of[64];
+    __shared__ int nbr[27];
+    __shared__ int run[129];
+    const int warp=threadIdx.x>>5;
+    if(threadIdx.x<64){crank[threadIdx.x]=cell_ranks.rank[threadIdx.x];cell_of[threadIdx.x]=cell_ranks.cell[threadIdx.x];}   // read after the next barrier
+    for(long long c=order?(long long)blockIdx.x:nc;c<nc;c+=gridDim.x){
+        ChunkInfo<T> ci;
+        load_chunk(S,c,nc,nv,ci,nbr);
+        const int np=ci.e-ci.s,st=(np+31)>>5;
+        // a work item longer than `chunk` only arises when the work-item capacity was exceeded:
+        // it keeps its order, and an empty record keeps the later kernels off it
+        if(np>S.chunk){                               // uniform
+            if(threadIdx.x==0) atomicOr(&S.ctr->error,ERR_CAPACITY);
+            for(int i=ci.s+threadIdx.x;i<ci.e;i+=blockDim.x) S.src[i]=S.perm[i];
+            if(warp==0){__syncwarp();write_item(S,c,ci,nbr,0,0);}
+            __syncthreads();
+            continue;}
+        if(warp==0) chunk_runs(np,st,run);            // read after the barriers in chunk_cell_order
+        chunk_cell_order(S.keys,ci.s,np,crank,ocnt,inv,loc,cellv,rank_end);
+        const int pairs=pair_table(rank_end,cell_of,st,run,S.pairs+ci.s);
+        if(warp==0) write_item(S,c,ci,nbr,np,pairs);
+        const float rst=1.f/(float)st;
+        for(int k=threadIdx.x;k<np;k+=blockDim.x){
+            const int i=ci.s+slot_position(k,st,rst,run),j=inv[k];
+            S.src[i]=S.perm[ci.s+j];
+            S.keys[i]=((unsigned)ci.gb<<6)|cellv[j];}
+        __syncthreads();}
     const V4<T> z={T(0),T(0),T(0),T(0)};
     for(long long n=t0;n<nn;n+=stride){S.gv[n]=z;S.gf[n]=z;}
-    const long long nc=min(S.ctr->n_chunks,(unsigned)S.chunk_cap);
-    auto chunk_scene=[&](long long c){return scene_of_block(S.scene_block_base,S.n_scenes,(long long)(S.keys[S.chunk_start[c]]>>6));};
+    auto chunk_scene=[&](long long c){return S.scn_cur[S.perm[S.chunk_start[c]]];};
     for(long long c=t0;c<nc;c+=stride){
         const int sc=chunk_scene(c);
         if(c==0||chunk_scene(c-1)!=sc) S.srange[sc].c0=(int)c;
@@ -844,8 +909,9 @@ template<class T> __global__ void __launch_bounds__(NODE_THREADS) k_grid_update(
             const T inv=T(1)/m;
             const T v[3]={a.x*inv,a.y*inv,a.z*inv};
             const V4<T> f=S.gf[n];
-            const T c=(T)(*S.dtp)/m;
-            T vs[3]={v[0]+c*f.x,v[1]+c*f.y,v[2]+c*f.z};
+            // v* = v + dt (f/m + g): gravity needs no scatter, its force at a node is m g
+            const T dt=(T)(*S.dtp),c=dt/m;
+            T vs[3]={v[0]+(c*f.x+dt*sc.gravity[0]),v[1]+(c*f.y+dt*sc.gravity[1]),v[2]+(c*f.z+dt*sc.gravity[2])};
             unsigned char proj=0;
             if(sc.n_barriers){
                 T x[3];node_center(S,sc,n,blk,x);
@@ -878,6 +944,27 @@ template<class T> __global__ void __launch_bounds__(NODE_THREADS) k_grid_update(
     });
 }
 
+__device__ __forceinline__ float2 padd(float2 a,float2 b){return __fadd2_rn(a,b);}
+__device__ __forceinline__ float2 psub(float2 a,float2 b){return __ffma2_rn(b,make_float2(-1.f,-1.f),a);}   // exact product: rounds like a - b
+__device__ __forceinline__ float2 pabs(float2 a){return make_float2(fabsf(a.x),fabsf(a.y));}
+// Sums with a product in them as two scalar operations: the assembler fuses a packed product
+// and a packed sum of it, and the weights have to be those of bspline_weights bit for bit (a
+// node that only the edge of a stencil reaches has its mass from their last bits).
+__device__ __forceinline__ float2 sadd(float2 a,float2 b){return make_float2(__fadd_rn(a.x,b.x),__fadd_rn(a.y,b.y));}
+__device__ __forceinline__ float2 ssub(float2 a,float2 b){return make_float2(__fsub_rn(a.x,b.x),__fsub_rn(a.y,b.y));}
+// bspline_weights of two coordinates, operation for operation: the same bits.
+__device__ __forceinline__ void bspline_weights2(float2 x,float2 inv_dx,float2 (&w)[3],float2 (&dw)[3])
+{
+    const float2 half=pdup(.5f),th=pdup(1.5f);
+    w[0]=pabs(padd(ssub(pmul(pmul(half,x),x),pmul(th,x)),pdup(1.125f)));
+    dw[0]=pmul(psub(x,th),inv_dx);
+    float2 y=psub(x,pdup(1.f));
+    w[1]=pabs(ssub(pdup(.75f),pmul(y,y)));
+    dw[1]=pmul(pmul(pdup(-2.f),y),inv_dx);
+    y=psub(y,pdup(1.f));
+    w[2]=pabs(padd(sadd(pmul(pmul(half,y),y),pmul(th,y)),pdup(1.125f)));
+    dw[2]=pmul(padd(y,th),inv_dx);
+}
 // =====================================================================================
 // K5: Hessian action q_raw = K s for every scene still iterating (MPM_CG_System::Force,
 // MPM_CG_System.h:150-215): gather dF = (sum_i s_i grad w_i^T) Fe, dP = dP/dF:dF, scatter
@@ -927,7 +1014,7 @@ __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const Sce
         const long long pc=S.pcap;
         const V4<T> q0=S.cache[i],q1=S.cache[pc+i],q2=S.cache[2*pc+i],q3=S.cache[3*pc+i],q4=S.cache[4*pc+i];
         cell=S.keys[i]&63u;
-        const T Sm[6]={q1.x,q1.y,q1.z,q1.w,q2.x,q2.y},Ki[6]={q3.x,q3.y,q3.z,q3.w,q4.x,q4.y},x[3]={q0.x,q0.y,q0.z};
+        const T Sm[6]={T(1)+q1.x,q1.y,q1.z,T(1)+q1.w,q2.x,T(1)+q2.y},Ki[6]={q3.x,q3.y,q3.z,q3.w,q4.x,q4.y},x[3]={q0.x,q0.y,q0.z};
         stencil_from_coord(sc,cell,x,st);
         C3<T> G[3];
         gather_grad(st,sv,G);
@@ -954,7 +1041,7 @@ __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const Sce
         __syncwarp();}
 }
 
-// FP32: two particles of one cell per lane (the pair table), every operation on both as a
+// The FP32 products: two particles of one cell per lane (the pair table), every operation on both as a
 // packed pair: (p, q) of the two particles in one register pair, each half rounded like the
 // scalar operation. The 81 node values of the cell's stencil are read once for both, and
 // both particles' forces are added to the tile in one read and one write per node. The
@@ -965,22 +1052,6 @@ __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const Sce
 // 0.107 ms on 1.94M particles, 1.32 -> 0.83 ms on 21.5M, against one particle per lane with
 // its Fe, Re, lambda, mu and V0 read as 25 separate words. Of that the stress form of
 // HessianData gives 1.32 -> 1.08, pairs, item records and copies ahead the rest.
-__device__ __forceinline__ float2 padd(float2 a,float2 b){return __fadd2_rn(a,b);}
-__device__ __forceinline__ float2 psub(float2 a,float2 b){return __ffma2_rn(b,make_float2(-1.f,-1.f),a);}   // exact product: rounds like a - b
-__device__ __forceinline__ float2 pabs(float2 a){return make_float2(fabsf(a.x),fabsf(a.y));}
-// bspline_weights of two coordinates, operation for operation.
-__device__ __forceinline__ void bspline_weights2(float2 x,float2 inv_dx,float2 (&w)[3],float2 (&dw)[3])
-{
-    const float2 half=pdup(.5f),th=pdup(1.5f);
-    w[0]=pabs(padd(psub(pmul(pmul(half,x),x),pmul(th,x)),pdup(1.125f)));
-    dw[0]=pmul(psub(x,th),inv_dx);
-    float2 y=psub(x,pdup(1.f));
-    w[1]=pabs(psub(pdup(.75f),pmul(y,y)));
-    dw[1]=pmul(pmul(pdup(-2.f),y),inv_dx);
-    y=psub(y,pdup(1.f));
-    w[2]=pabs(padd(padd(pmul(pmul(half,y),y),pmul(th,y)),pdup(1.125f)));
-    dw[2]=pmul(padd(y,th),inv_dx);
-}
 // B = V0 dP Fe^T from G for two particles (hessian_stress).
 __device__ __forceinline__ void hessian_stress2(const float2 (&G)[3][3],const float2 (&Sm)[6],float2 c1,float2 c2,float2 cc3,float2 (&B)[3][3],float2& bg)
 {
@@ -1013,15 +1084,16 @@ __device__ __forceinline__ void hessian_stress2(const float2 (&G)[3][3],const fl
             B[i][j]=pfma(M[i][2],cS[ix[2][j]],pfma(M[i][1],cS[ix[1][j]],pfma(M[i][0],cS[ix[0][j]],g)));
             bg=i==0&&j==0?pmul(B[i][j],G[i][j]):pfma(B[i][j],G[i][j],bg);}
 }
-__device__ __forceinline__ void copy_pair(const DevState<float>& S,int s,unsigned entry,V4<float> (*slots)[32])
+// The first N cache vectors of a pair's particles into slots[N*h + k][lane].
+template<int N> __device__ __forceinline__ void copy_pair(const DevState<float>& S,int s,unsigned entry,V4<float> (*slots)[32])
 {
     const int lane=threadIdx.x&31;
 #pragma unroll
     for(int h=0;h<2;++h){
         const V4<float>* p=S.cache+s+((entry>>(12*h))&4095u);
 #pragma unroll
-        for(int k=0;k<3;++k){
-            const unsigned d=(unsigned)__cvta_generic_to_shared(&slots[3*h+k][lane]);
+        for(int k=0;k<N;++k){
+            const unsigned d=(unsigned)__cvta_generic_to_shared(&slots[N*h+k][lane]);
             asm volatile("cp.async.cg.shared.global [%0],[%1],16;"::"r"(d),"l"(p+k*S.pcap):"memory");}}
 }
 // A single pass that a warp runs again and again (k_cg_solve): once copied, its pairs stay in
@@ -1035,7 +1107,7 @@ __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const Sce
     const unsigned* tab=S.pairs+s;
     const int lane=threadIdx.x&31;
     unsigned entry=pass.entry,next=0;
-    if(!pass.ready&&m0+lane<M){entry=tab[m0+lane];copy_pair(S,s,entry,slots);}
+    if(!pass.ready&&m0+lane<M){entry=tab[m0+lane];copy_pair<3>(S,s,entry,slots);}
     pass.entry=entry;pass.ready=m0+dm>=M;
     if(m0+dm+lane<M) next=tab[m0+dm+lane];
     for(int m=m0;m<M;m+=dm){
@@ -1072,8 +1144,9 @@ __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const Sce
                     G[a][1]=first?pmul(t,xdy):pfma(t,xdy,G[a][1]);
                     G[a][2]=first?pmul(u,wxy):pfma(u,wxy,G[a][2]);}}
             const V4<float> p1=slots[1][lane],q1=slots[4][lane],p2=slots[2][lane],q2=slots[5][lane];
-            const float2 Sm[6]={make_float2(p1.x,q1.x),make_float2(p1.y,q1.y),make_float2(p1.z,q1.z),
-                                make_float2(p1.w,q1.w),make_float2(p2.x,q2.x),make_float2(p2.y,q2.y)};
+            const float2 one=pdup(1.f);
+            const float2 Sm[6]={padd(one,make_float2(p1.x,q1.x)),make_float2(p1.y,q1.y),make_float2(p1.z,q1.z),
+                                padd(one,make_float2(p1.w,q1.w)),make_float2(p2.x,q2.x),padd(one,make_float2(p2.y,q2.y))};
             const bool two=(entry&PAIR_TWO)!=0u;                    // no second particle: no force
             float2 bg;
             hessian_stress2(G,Sm,make_float2(slots[0][lane].w,two?slots[3][lane].w:0.f),make_float2(p2.z,two?q2.z:0.f),
@@ -1081,7 +1154,7 @@ __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const Sce
             sks+=(double)(bg.x+bg.y);
             weights(w,dw);}
         entry=next;
-        if(m+dm+lane<M) copy_pair(S,s,entry,slots);
+        if(m+dm+lane<M) copy_pair<3>(S,s,entry,slots);
         if(m+2*dm+lane<M) next=tab[m+2*dm+lane];
         const ScatterRounds R(valid,cell);
         for(int r=0;r<R.rounds;++r){
@@ -1267,6 +1340,143 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
         }
     }
     add_sks(-1);
+}
+
+// =====================================================================================
+// K3b: the scatter of P2G in FP32 (Rasterize, MPM_Example.cpp:520-537; Apply_Explicit_Force,
+// :757-784): m, m v and f = -sum_p V0 P Fe^T grad w of two particles of one cell per lane, as
+// the Hessian product scatters, into the warp's 7-channel tile. The stress is formed from the
+// cache that the products read. A work item is taken by a CTA, its passes split over 2 or 4
+// CTAs where items are few, or by a warp where there are at least as many as resident warps.
+// =====================================================================================
+constexpr int P2G_CH=7;
+__host__ __device__ constexpr int scatter_warp_bytes(){return P2G_CH*TILE_S*4+8*32*16;}
+__device__ __forceinline__ void scatter_pairs(const DevState<float>& S,const SceneDev<float>& sc,int s,int M,int m0,int dm,float (*tile)[TILE_S],V4<float> (*slots)[32])
+{
+    const unsigned* tab=S.pairs+s;
+    const int lane=threadIdx.x&31;
+    unsigned entry=0,next=0;
+    if(m0+lane<M){entry=tab[m0+lane];copy_pair<4>(S,s,entry,slots);}
+    if(m0+dm+lane<M) next=tab[m0+dm+lane];
+    for(int m=m0;m<M;m+=dm){
+        const bool valid=m+lane<M;
+        const unsigned cell=(entry>>24)&63u;
+        const int tb=tile_addr((int)(cell&3u),(int)((cell>>2)&3u),(int)(cell>>4));
+        float2 w[3][3],dw[3][3],mv[4],A[6];          // mv: (m, m v), A: -V0 P Fe^T
+        asm volatile("cp.async.wait_all;":::"memory");
+        if(valid){
+            const V4<float> p0=slots[0][lane],q0=slots[4][lane],p1=slots[1][lane],q1=slots[5][lane];
+            const V4<float> p2=slots[2][lane],q2=slots[6][lane],p3=slots[3][lane],q3=slots[7][lane];
+            bspline_weights2(make_float2(p0.x,q0.x),pdup(sc.inv_dx[0]),w[0],dw[0]);
+            bspline_weights2(make_float2(p0.y,q0.y),pdup(sc.inv_dx[1]),w[1],dw[1]);
+            bspline_weights2(make_float2(p0.z,q0.z),pdup(sc.inv_dx[2]),w[2],dw[2]);
+            const float on=(entry&PAIR_TWO)?1.f:0.f;   // no second particle: nothing to add
+            mv[0]=make_float2(p3.x,on*q3.x);
+            mv[1]=pmul(mv[0],make_float2(p3.y,q3.y));mv[2]=pmul(mv[0],make_float2(p3.z,q3.z));mv[3]=pmul(mv[0],make_float2(p3.w,q3.w));
+            const float2 c1=make_float2(-p0.w,-on*q0.w),c3=make_float2(-p2.w,-on*q2.w);
+            const float2 E[6]={make_float2(p1.x,q1.x),make_float2(p1.y,q1.y),make_float2(p1.z,q1.z),
+                               make_float2(p1.w,q1.w),make_float2(p2.x,q2.x),make_float2(p2.y,q2.y)};
+            auto dot=[&](int a,int b,int c,int d,int e,int f){return pfma(E[e],E[f],pfma(E[c],E[d],pmul(E[a],E[b])));};
+            A[0]=pfma(c1,padd(E[0],dot(0,0,1,1,2,2)),c3);A[1]=pmul(c1,padd(E[1],dot(0,1,1,3,2,4)));
+            A[2]=pmul(c1,padd(E[2],dot(0,2,1,4,2,5)));A[3]=pfma(c1,padd(E[3],dot(1,1,3,3,4,4)),c3);
+            A[4]=pmul(c1,padd(E[4],dot(1,2,3,4,4,5)));A[5]=pfma(c1,padd(E[5],dot(2,2,4,4,5,5)),c3);
+            if(sc.eos) A[0]=A[3]=A[5]=make_float2(p1.x,on*q1.x);}
+        entry=next;
+        if(m+dm+lane<M) copy_pair<4>(S,s,entry,slots);
+        if(m+2*dm+lane<M) next=tab[m+2*dm+lane];
+        const ScatterRounds R(valid,cell);
+        for(int r=0;r<R.rounds;++r){
+            const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
+            if(valid&&R.rank==r){
+#pragma unroll
+                for(int k=0;k<3;++k){opaque(w[0][k]);opaque(dw[0][k]);}
+#pragma unroll
+                for(int ox=0;ox<3;++ox)
+#pragma unroll
+                for(int oy=0;oy<3;++oy){
+                    const float2 dxy=pmul(dw[0][ox],w[1][oy]),xdy=pmul(w[0][ox],dw[1][oy]),wxy=pmul(w[0][ox],w[1][oy]);
+                    float2 c[4];
+#pragma unroll
+                    for(int a=0;a<4;++a) c[a]=pmul(mv[a],wxy);
+                    const float2 al[3]={pfma(A[1],xdy,pmul(A[0],dxy)),pfma(A[3],xdy,pmul(A[1],dxy)),pfma(A[4],xdy,pmul(A[2],dxy))};
+                    const float2 be[3]={pmul(A[2],wxy),pmul(A[4],wxy),pmul(A[5],wxy)};
+#pragma unroll
+                    for(int oz=0;oz<3;++oz){
+                        const int t=tb+tile_addr(ox,oy,oz);
+                        float v[P2G_CH];
+#pragma unroll
+                        for(int a=0;a<4;++a){const float2 f=pfma(c[a],w[2][oz],make_float2(tile[a][t],0.f));v[a]=f.x+f.y;}
+#pragma unroll
+                        for(int a=0;a<3;++a){
+                            const float2 f=pfma(be[a],dw[2][oz],pfma(al[a],w[2][oz],make_float2(tile[4+a][t],0.f)));
+                            v[4+a]=f.x+f.y;}
+#pragma unroll
+                        for(int a=0;a<P2G_CH;++a) tile[a][t]=v[a];
+                        __syncwarp(rmask);}}}
+            __syncwarp();}
+    }
+}
+template<int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) k_p2g_scatter(DevState<float> S,long long warp_min)
+{
+    pdl_enter();
+    constexpr int NW=XFER_THREADS/32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int rec_s[NW][ITEM_WORDS];
+    __shared__ unsigned tmap[TILE_N];
+    const int warp=threadIdx.x>>5,lane=threadIdx.x&31;
+    const long long nc=min(S.ctr->n_chunks,(unsigned)S.chunk_cap),G=gridDim.x,resident=warp_min/NW;
+    const bool by_warp=nc>=warp_min;
+    const int split=4*nc<=resident?4:2*nc<=resident?2:1;
+    const long long units=by_warp?(nc+NW-1)/NW:nc*split;
+    if(blockIdx.x>=units) return;
+    auto tile_of=[&](int w){return reinterpret_cast<float (*)[TILE_S]>(smem_raw+w*scatter_warp_bytes());};   // [channel][node]
+    float (*tile)[TILE_S]=tile_of(warp);
+    V4<float> (*slots)[32]=reinterpret_cast<V4<float> (*)[32]>(smem_raw+warp*scatter_warp_bytes()+P2G_CH*TILE_S*4);
+    for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x) tmap[t]=tile_map_entry(t);
+    for(int t=lane;t<P2G_CH*TILE_S;t+=32) (&tile[0][0])[t]=0.f;
+    __syncthreads();
+    // one vector atomic per touched node and channel group
+    auto flush=[&](const int* rec,unsigned e,const float (&v)[P2G_CH]){
+        if(v[0]==0.f&&v[4]==0.f&&v[5]==0.f&&v[6]==0.f) return;
+        const int blk=rec[ITEM_NBR+(e&31u)];
+        if(blk<0){atomicOr(&S.ctr->error,ERR_CAPACITY);return;}
+        const long long node=(long long)blk*64+((e>>5)&63u);
+        atomic_add_v3(S.gv+node,v[1],v[2],v[3],v[0]);
+        atomic_add_v3(S.gf+node,v[4],v[5],v[6],0.f);};
+    if(by_warp){
+        int* rec=rec_s[warp];
+        const long long w0=(long long)blockIdx.x*NW+warp,dwork=G*NW;
+        int mine=w0<nc?S.items[w0*ITEM_WORDS+lane]:0;
+        for(long long c=w0;c<nc;c+=dwork){
+            rec[lane]=mine;
+            __syncwarp();
+            if(c+dwork<nc) mine=S.items[(c+dwork)*ITEM_WORDS+lane];
+            scatter_pairs(S,S.scenes[rec[ITEM_SCENE]],rec[ITEM_START],rec[ITEM_PAIRS],0,32,tile,slots);
+            __syncwarp();
+            for(int t=lane;t<TILE_N;t+=32){
+                const unsigned e=tmap[t];
+                float v[P2G_CH];
+#pragma unroll
+                for(int ch=0;ch<P2G_CH;++ch){float* p=&tile[ch][e>>11];v[ch]=*p;*p=0.f;}
+                flush(rec,e,v);}
+            __syncwarp();}
+        return;}
+    int* rec=rec_s[0];
+    for(long long u=blockIdx.x;u<units;u+=G){
+        if(warp==0) rec[lane]=S.items[(u/split)*ITEM_WORDS+lane];
+        __syncthreads();
+        scatter_pairs(S,S.scenes[rec[ITEM_SCENE]],rec[ITEM_START],rec[ITEM_PAIRS],(warp+NW*(int)(u%split))*32,NW*split*32,tile,slots);
+        __syncthreads();
+        for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x){
+            const unsigned e=tmap[t];
+            float v[P2G_CH];
+#pragma unroll
+            for(int ch=0;ch<P2G_CH;++ch){float a=0.f;
+#pragma unroll
+                for(int w2=0;w2<NW;++w2){float* p=&tile_of(w2)[ch][e>>11];a+=*p;*p=0.f;}
+                v[ch]=a;}
+            flush(rec,e,v);}
+        __syncthreads();}
 }
 
 // r = b - (x + dt^2/m K x) on a node block, two nodes per lane, Project(r) (MPM_CG_System.h:
