@@ -179,13 +179,12 @@ template<class P> void enqueue_binning(mpm_context* c,cudaStream_t st,const DevS
 {
     const long long n=c->n_total;
     {PhaseScope ps(c,PH_KEYS,st);
-        cudaMemsetAsync(c->ctr,0,offsetof(Counters,error),st);
-        cudaMemsetAsync(c->bitmap,0,c->bitmap_words*sizeof(unsigned),st);
-        cudaMemsetAsync(c->srange,0,sizeof(SceneRange)*c->scenes.size(),st);
         const int g=(int)std::min<long long>((n+256*KEY_ITEMS-1)/(256*KEY_ITEMS),grid_for(c,8));
         const int items=os_items(n);
         const long long num_tiles=(n+(long long)RS_THREADS*items-1)/((long long)RS_THREADS*items);
-        cudaMemsetAsync(c->sortws,0,sizeof(unsigned)*(c->sort_status_off+(long long)c->sort_passes*num_tiles*256),st);
+        const long long cleared=c->sort_status_off+(long long)c->sort_passes*num_tiles*256;
+        launch_dep(c,k_clear<TT<P>>,(int)std::min<long long>((cleared+c->bitmap_words)/1024+1,grid_for(c,8)),256,0,st,S,c->sortws,cleared);
+        counted(c,PH_KEYS);
         if(c->sort_incremental){
             const int fin=c->sort_passes&1;
             const int gk=(int)std::max<long long>(1,std::min<long long>((n+256*MV_ITEMS-1)/(256*MV_ITEMS),grid_for(c,8)));
