@@ -200,6 +200,18 @@ template<> struct NodeSum<float> { float h=0.f,l=0.f;
     __device__ __forceinline__ void add(float x)
     {const float s=__fadd_rn(h,x),z=__fadd_rn(s,-h);l+=__fadd_rn(__fadd_rn(h,-__fadd_rn(s,-z)),__fadd_rn(x,-z));h=s;}
     __device__ __forceinline__ double value() const {return (double)h+(double)l;} };
+// The sum of a warp's lanes. FP32 adds the lanes' pairs by the same TwoSum and converts once: an
+// FP64 addition keeps the SM's FP64 units busy for 16 cycles a warp, and the five steps of
+// four quantities took 1 us of a CG trip of a small scene.
+__device__ __forceinline__ double warp_value(NodeSum<float> v)
+{
+#pragma unroll
+    for(int o=16;o>0;o>>=1){
+        const float h=__shfl_xor_sync(0xffffffffu,v.h,o),l=__shfl_xor_sync(0xffffffffu,v.l,o);
+        v.add(h);v.l=__fadd_rn(v.l,l);}
+    return v.value();
+}
+__device__ __forceinline__ double warp_value(NodeSum<double> v){return warp_sum<double>(v.h);}
 // The reduction of kernels whose warps walk contiguous block ranges: a warp's last scene goes
 // into its slot here, an earlier one (rare) straight to the accumulators; one warp joins the
 // slots (mostly one scene) and adds them. Against per-scene shared arrays this spares a
@@ -211,9 +223,10 @@ template<int NS> __device__ __forceinline__ void add_scene(SceneAcc* acc,int sc,
     for(int k=0;k<NS;++k) if(s[k]!=0.) atomicAdd(&acc[sc].sum[k],s[k]);
     if(mx>0.) atomicMax(&acc[sc].max0,dbits(mx));
 }
-template<int NS> __device__ __forceinline__ void flush_scene(WarpParts& W,SceneAcc* acc,int sc,bool last,double a,double b,double c,double mx)
+template<int NS,class T> __device__ __forceinline__ void flush_scene(WarpParts& W,SceneAcc* acc,int sc,bool last,const NodeSum<T>& a,const NodeSum<T>& b,
+    const NodeSum<T>& c,T mx)
 {
-    const double s[3]={warp_sum<double>(a),NS>1?warp_sum<double>(b):0.,NS>2?warp_sum<double>(c):0.},m=warp_max<double>(mx);
+    const double s[3]={warp_value(a),NS>1?warp_value(b):0.,NS>2?warp_value(c):0.},m=(double)warp_max<T>(mx);
     if((threadIdx.x&31)!=0) return;
     if(!last){add_scene<NS>(acc,sc,s,m);return;}
     const int w=threadIdx.x>>5;
@@ -1001,7 +1014,7 @@ template<class T> __device__ __forceinline__ void hessian_stress(const C3<T> (&G
 // vector tile sv, forms B and scatters B grad w into the warp's private tile in rounds of
 // lanes in distinct cells. Called by every lane of the warp.
 __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const SceneDev<double>& sc,int s,const int* run,int qi,int stride,int np,
-    const double (*sv)[TILE_S],double (*tile)[TILE_S],double& sks)
+    const double (*sv)[TILE_S],double (*tile)[TILE_S],NodeSum<double>& sks)
 {
     using T=double;
     const int j=(int)(threadIdx.x&31)*stride+qi;
@@ -1019,7 +1032,7 @@ __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const Sce
         C3<T> G[3];
         gather_grad(st,sv,G);
         T bg;hessian_stress<T>(G,Sm,q0.w,q2.z,q2.w,Ki,B,bg);
-        sks+=bg;}
+        sks.add(bg);}
     const ScatterRounds R(valid,cell);
     for(int r=0;r<R.rounds;++r){
         const unsigned rmask=__ballot_sync(0xffffffffu,valid&&R.rank==r);
@@ -1101,7 +1114,7 @@ template<int N> __device__ __forceinline__ void copy_pair(const DevState<float>&
 struct PairPass { unsigned entry=0u; bool ready=false; };
 // The passes m0, m0 + dm, ... (pair index of the pass's first lane) of a work item of M pairs.
 __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const SceneDev<float>& sc,int s,int M,int m0,int dm,
-    const float (*sv)[TILE_S],float (*tile)[TILE_S],V4<float> (*slots)[32],double& sks,
+    const float (*sv)[TILE_S],float (*tile)[TILE_S],V4<float> (*slots)[32],NodeSum<float>& sks,
     PairPass& pass)
 {
     const unsigned* tab=S.pairs+s;
@@ -1151,7 +1164,7 @@ __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const Sce
             float2 bg;
             hessian_stress2(G,Sm,make_float2(slots[0][lane].w,two?slots[3][lane].w:0.f),make_float2(p2.z,two?q2.z:0.f),
                             make_float2(p2.w,two?q2.w:0.f),B,bg);
-            sks+=(double)(bg.x+bg.y);
+            sks.add(bg.x+bg.y);
             weights(w,dw);}
         entry=next;
         if(m+dm+lane<M) copy_pair<3>(S,s,entry,slots);
@@ -1274,12 +1287,12 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
         if(FROM_X) return w;
         const int j=list_find(lsm,(int)w);return S.srange[lsm.scene[j]].c0+(w-lsm.pre[j]);};
     // s^T K s of a loop trip (k_cg_update), per lane until the warp's scene changes
-    double sks=0.;int sks_scene=-1;
+    NodeSum<T> sks;int sks_scene=-1;
     auto add_sks=[&](int next){
         if(!FROM_X&&sks_scene>=0&&sks_scene!=next){
-            const double v=warp_sum<double>(sks);
+            const double v=warp_value(sks);
             if(lane==0&&v!=0.) atomicAdd(&S.acc[sks_scene].sks,v);
-            sks=0.;}
+            sks=NodeSum<T>();}
         sks_scene=next;};
     // the passes of an item: pairs (FP32) or cell-ordered particles (FP64), `first` of every `of`
     auto passes=[&](const SceneDev<T>& sc,const int* rec,const T (*sv)[TILE_S],int* run,int first,int of){
@@ -1538,7 +1551,7 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_start(Dev
     if(blockIdx.x>=wr.parts) return;
     if((threadIdx.x&31)==0) W.scene[threadIdx.x>>5]=-1;
     int scene=-1;NodeSum<T> rr;T amax=T(0);
-    auto flush=[&](int sc,bool last){flush_scene<1>(W,S.acc,sc,last,rr.value(),0.,0.,(double)amax);rr=NodeSum<T>();amax=T(0);};
+    auto flush=[&](int sc,bool last){flush_scene<1,T>(W,S.acc,sc,last,rr,rr,rr,amax);rr=NodeSum<T>();amax=T(0);};
     for(int blk=wr.b;blk<wr.b1;++blk){
         const int sb=S.active_scene[blk];
         if(sb!=scene){if(scene>=0) flush(scene,false);scene=sb;}
@@ -1601,7 +1614,7 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
     const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
     NodeSum<T> rr,rs,ss;T amax=T(0),alpha=T(0),beta=T(0);
     auto flush=[&](int sc,bool last){
-        flush_scene<3>(W,S.acc,sc,last,rr.value(),rs.value(),ss.value(),(double)amax);
+        flush_scene<3,T>(W,S.acc,sc,last,rr,rs,ss,amax);
         rr=rs=ss=NodeSum<T>();amax=T(0);};
     for(int bw=wb.b;bw<wb.b1;++bw){
         const int prev=wb.scene;
@@ -1647,21 +1660,29 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
 // (product, vector update) are separated by grid barriers whose arrivals carry the sums.
 // With fewer work items than CTAs an item's passes are split over 2 or 4 CTAs.
 // =====================================================================================
-// One arrival per CTA; thread 0 waits for all (bounded) and runs `post`. False after the limit.
+// One arrival per CTA, after warp 0 has run `pre`; thread 0 runs `idle` while the others arrive,
+// waits for all (bounded) and runs `post`. False after the limit. A round trip to L2 or a few
+// dependent FP64 operations here are time of every CTA: the poll is the acquire (a fence
+// and a second read after it took 0.7 us), and what the threads do not wait for is in `idle`.
 constexpr int SOLVE_SPIN_LIMIT=1<<20;
-template<class F> __device__ __forceinline__ bool solve_barrier(Counters* ctr,unsigned target,F post)
+__device__ __forceinline__ unsigned load_acquire(const unsigned* p){unsigned v;asm volatile("ld.acquire.gpu.global.u32 %0,[%1];":"=r"(v):"l"(p):"memory");return v;}
+template<class F0,class F1,class F2> __device__ __forceinline__ bool solve_barrier(Counters* ctr,unsigned target,F0 pre,F1 idle,F2 post)
 {
     __shared__ bool ok;
     __syncthreads();
-    if(threadIdx.x==0){
-        __threadfence();
-        atomicAdd(&ctr->solve_arrived,1u);
-        int spins=0;
-        while(*(volatile unsigned*)&ctr->solve_arrived<target&&++spins<SOLVE_SPIN_LIMIT) if(spins>64) __nanosleep(32);
-        __threadfence();
-        ok=*(volatile unsigned*)&ctr->solve_arrived>=target;
-        if(!ok) atomicOr(&ctr->error,ERR_GRID_WAIT);
-        post();}
+    if(threadIdx.x<32){
+        pre();
+        __syncwarp();
+        if(threadIdx.x==0){
+            __threadfence();
+            atomicAdd(&ctr->solve_arrived,1u);
+            idle();
+            int spins=0;
+            unsigned seen;
+            while((seen=load_acquire(&ctr->solve_arrived))<target&&++spins<SOLVE_SPIN_LIMIT) if(spins>64) __nanosleep(32);
+            ok=seen>=target;
+            if(!ok) atomicOr(&ctr->error,ERR_GRID_WAIT);
+            post();}}
     __syncthreads();
     return ok;
 }
@@ -1696,7 +1717,7 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
     auto arrived=[&]{return (unsigned)(phase+1)*(unsigned)G;};
     // K v for v = x, or s = r + beta s_old with s^T K s into part[][0]
     auto product=[&](bool from_x,T beta){
-        double sks=0.;
+        NodeSum<T> sks;
         for(int u=blockIdx.x;u<units;u+=G){
             if(u!=held){
                 __syncthreads();
@@ -1716,16 +1737,19 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
                     for(int w2=0;w2<NW;++w2){T* p=&tile_of(w2)[ch][e>>11];a+=*p;*p=T(0);}
                     v[ch]=a;}
                 add_tile_node(S,rec,e,v[0],v[1],v[2]);}}
-        const double s=warp_sum<double>(sks);
+        const double s=warp_value(sks);
         if(lane==0) part[warp][0]=s;};
-    // thread 0: the CTA's sums into the slot of this phase
+    // warp 0: the CTA's sums into the slot of this phase, a sum per lane
     auto contribute=[&](int ns,bool with_max){
-        __syncthreads();
-        if(threadIdx.x==0){
-            SolveSlot& o=ctr->solve[phase&3];
-            for(int k=0;k<ns;++k){double s=0.;for(int w=0;w<NW;++w) s+=part[w][k];if(s!=0.) atomicAdd(&o.sum[k],s);}
-            if(with_max){double m=0.;for(int w=0;w<NW;++w) m=fmax(m,part[w][3]);if(m>0.) atomicMax(&o.max0,dbits(m));}}};
-    auto clear_ahead=[&]{               // the slot two phases on: read by nobody any more
+        SolveSlot& o=ctr->solve[phase&3];
+        if(lane<ns){
+            double v=0.;
+#pragma unroll
+            for(int w=0;w<NW;++w) v+=part[w][lane];
+            if(v!=0.) atomicAdd(&o.sum[lane],v);}
+        if(lane==3&&with_max){double m=0.;for(int w=0;w<NW;++w) m=fmax(m,part[w][3]);if(m>0.) atomicMax(&o.max0,dbits(m));}};
+    // the slot two phases on: its readers have all arrived at the barrier before this one
+    auto clear_ahead=[&]{
         if(blockIdx.x==0){SolveSlot& o=ctr->solve[(phase+2)&3];o.sum[0]=o.sum[1]=o.sum[2]=0.;o.max0=0ull;}};
     auto read_slot=[&](double (&s)[3],double& mx){
         const volatile SolveSlot& o=ctr->solve[phase&3];
@@ -1733,20 +1757,19 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
     const double eps=1.1920928955078125e-07;     // FP32, as k_cg_start and k_cg_update
     // x = v*: r = b - A x and the first check
     product(true,T(0));
-    if(!solve_barrier(ctr,arrived(),clear_ahead)) return;
+    if(!solve_barrier(ctr,arrived(),[]{},clear_ahead,[]{})) return;
     ++phase;
     {   NodeSum<T> rr;T amax=T(0);
         for(int blk=b0;blk<b1;++blk) cg_start_block(S,blk,dt2,rr,amax);
-        const double a=warp_sum<double>(rr.value()),m=warp_max<double>((double)amax);
+        const double a=warp_value(rr),m=(double)warp_max<T>(amax);
         if(lane==0){part[warp][0]=a;part[warp][3]=m;}}
-    contribute(1,true);
-    double rho=0.,msq=0.,rmax=0.,beta=0.;        // thread 0 of every CTA: equal values
+    double rho=0.,msq=0.,rmax=0.,beta=0.,rs_sum=0.,ss_sum=0.;        // thread 0 of every CTA: equal values
     int iters=0,converged=0;
     const double tol=S.cg[0].tol,tol2=tol*tol;
     // sqrt(mx) <= tol; the root (on the barriers' critical path) only where rounding could decide
     auto small=[&](double mx){return mx<tol2*(1.-1e-14)?true:mx>tol2*(1.+1e-14)?false:sqrt(mx)<=tol;};
-    if(!solve_barrier(ctr,arrived(),[&]{
-        double s[3],mx;read_slot(s,mx);clear_ahead();
+    if(!solve_barrier(ctr,arrived(),[&]{contribute(1,true);},clear_ahead,[&]{
+        double s[3],mx;read_slot(s,mx);
         rmax=mx;rho=msq=s[0];
         converged=small(mx)&&(0>=sc.cg_min_iters||sqrt(mx)<eps);
         sh_stop=converged||sc.cg_max_iters<=0||max_trips<=0;sh_beta=T(0);})) return;
@@ -1754,23 +1777,23 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
         ++phase;
         const T be=sh_beta;
         product(false,be);
-        contribute(1,false);
-        if(!solve_barrier(ctr,arrived(),[&]{
-            double s[3],mx;read_slot(s,mx);clear_ahead();
+        if(!solve_barrier(ctr,arrived(),[&]{contribute(1,false);},[&]{
+            clear_ahead();
+            if(phase>2) msq=rho+beta*(2.*rs_sum+beta*ss_sum);},[&]{
+            double s[3],mx;read_slot(s,mx);
             const double sq=(double)dt2*s[0]+msq;
             sh_alpha=(T)(sq!=0.?rho/sq:(double)FLT_MAX);})) return;
         ++phase;
         {   const T alpha=sh_alpha;
             NodeSum<T> rr,rs,ss;T amax=T(0);
             for(int blk=b0;blk<b1;++blk) cg_update_block(S,((long long)blk<<6),alpha,be,dt2,rr,rs,ss,amax);
-            const double a=warp_sum<double>(rr.value()),b=warp_sum<double>(rs.value()),c=warp_sum<double>(ss.value()),m=warp_max<double>((double)amax);
+            const double a=warp_value(rr),b=warp_value(rs),c=warp_value(ss),m=(double)warp_max<T>(amax);
             if(lane==0){part[warp][0]=a;part[warp][1]=b;part[warp][2]=c;part[warp][3]=m;}}
-        contribute(3,true);
-        if(!solve_barrier(ctr,arrived(),[&]{
-            double s[3],mx;read_slot(s,mx);clear_ahead();
+        if(!solve_barrier(ctr,arrived(),[&]{contribute(3,true);},clear_ahead,[&]{
+            double s[3],mx;read_slot(s,mx);
             ++iters;rmax=mx;
             converged=small(mx)&&(iters>=sc.cg_min_iters||sqrt(mx)<eps);
-            beta=s[0]/rho;rho=s[0];msq=s[0]+beta*(2.*s[1]+beta*s[2]);
+            beta=s[0]/rho;rho=s[0];rs_sum=s[1];ss_sum=s[2];
             sh_beta=(T)beta;sh_stop=converged||iters>=sc.cg_max_iters||iters>=max_trips;})) return;}
     if(blockIdx.x==0&&threadIdx.x==0){
         CGState& st=S.cg[0];
