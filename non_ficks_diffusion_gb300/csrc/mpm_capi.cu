@@ -162,7 +162,7 @@ template<class P> DevState<TT<P>> make_state(mpm_context* c,int parity,double dt
     const int fin=c->sort_passes&1;   // the sort's final ping-pong buffer
     S.keys=c->keys[fin];S.perm=c->vals[fin];
     S.chunk_start=c->chunk_start;S.chunk_cap=c->chunk_cap;S.items=c->items;
-    S.pairs=c->mkeys[0];S.src=c->mvals[0];    // free between the binning and the next substep's
+    S.pairs=c->mkeys[0];S.src=c->mvals[0];S.units=c->mvals[1];   // free between the binning and the next substep's
     S.bitmap=c->bitmap;S.bitmap_words=c->bitmap_words;
     S.blockmap=c->blockmap;S.active_gb=c->active_gb;S.active_scene=c->active_scene;S.block_cap=c->block_cap;
     S.gv=(V4<T>*)c->gv;S.gf=(V4<T>*)c->gf;S.gx=(V4<T>*)c->gx;S.gr=(V4<T>*)c->gr;S.gs=(V4<T>*)c->gs;S.gm=(T*)c->gm;S.gproj=c->gproj;
@@ -173,8 +173,27 @@ template<class P> DevState<TT<P>> make_state(mpm_context* c,int parity,double dt
     return S;
 }
 
+// Whether a graph's substep solves in one cooperative kernel (k_cg_solve): one scene in FP32
+// storage, the Hessian's form left to the library, at most SOLVE_MAX particles. Substeps
+// measured as a loop of kernels -> one kernel: 3K particles 158 -> 128 us, 20K 295 -> 222,
+// 61K 345 -> 281, 237K 342 -> 328, 400K 499 -> 454, 1.2M 1,218 -> 1,174; from 2M on the
+// loop with a warp per work item is faster (1,820 against 1,905, at 4M 3,454 against 3,910).
+constexpr long long SOLVE_MAX=1LL<<20;
+template<class P> bool solve_in_one(const mpm_context* c)
+{
+    return sizeof(TT<P>)==4&&c->coop&&c->scenes.size()==1&&c->hess_warp==HESS_AUTO&&c->n_total<=SOLVE_MAX;
+}
+// Whether it deals out units: the list costs k_items an atomic per work item (1 us), which 3K
+// particles do not earn back (106.4 -> 107.4 us) and 8K do (140.7 -> 139.8); resting snow has a
+// unit for about 160 particles, and with more units than CTAs (100K) the list is not used.
+template<class P> bool solve_units(const mpm_context* c)
+{
+    return solve_in_one<P>(c)&&c->n_total>=4096&&c->n_total<=160LL*4*c->num_sms;
+}
+
 // Keys, stable radix sort, work items and active blocks for the current particle buffer.
-// `order`: also the storage order of the work items' particles, which FP32 substeps need.
+// `order`: also the storage order of the work items' particles, which FP32 substeps need, and
+// the units of k_cg_solve where it runs.
 template<class P> void enqueue_binning(mpm_context* c,cudaStream_t st,const DevState<TT<P>>& S,bool order)
 {
     const long long n=c->n_total;
@@ -244,7 +263,7 @@ template<class P> void enqueue_binning(mpm_context* c,cudaStream_t st,const DevS
         const long long bseg=(c->bitmap_words+BM_SEG-1)/BM_SEG;
         const int gb=(int)std::max<long long>(1,std::min<long long>(bseg,grid_for(c,8)));
         launch_dep(c,k_bitmap_index<TT<P>>,gb,SC_THREADS,0,st,S,c->sortws+c->bin_blocks_off,c->sortws+1029);counted(c,PH_BIN);
-        launch_dep(c,k_items<TT<P>>,grid_for(c,16),XFER_THREADS,order?order_bytes(c->cfg.chunk):0,st,S,order?1:0);counted(c,PH_BIN);}
+        launch_dep(c,k_items<TT<P>>,grid_for(c,16),XFER_THREADS,order?order_bytes(c->cfg.chunk):0,st,S,order?1:0,order&&solve_units<P>(c)?1:0);counted(c,PH_BIN);}
 }
 
 int max_cg_iters(mpm_context* c){int m=0;for(auto& s:c->scenes) m=std::max(m,s.desc.cg_max_iters);return m;}
@@ -266,18 +285,9 @@ template<class P> void enqueue_cg_body(mpm_context* c,cudaStream_t st,const DevS
         launch_dep(c,k_cg_update<P>,grid_for(c,c->node_grid),NODE_THREADS,0,st,S2,cond,use_cond,max_cg_iters(c)+1);counted(c,PH_CGNODE);}
 }
 
-// Whether a graph's substep solves in one cooperative kernel (k_cg_solve): one scene in FP32
-// storage, the Hessian's form left to the library, at most SOLVE_MAX particles. Substeps
-// measured as a loop of kernels -> one kernel: 3K particles 158 -> 128 us, 20K 295 -> 222,
-// 61K 345 -> 281, 237K 342 -> 328, 400K 499 -> 454, 1.2M 1,218 -> 1,174; from 2M on the
-// loop with a warp per work item is faster (1,820 against 1,905, at 4M 3,454 against 3,910).
-constexpr long long SOLVE_MAX=1LL<<20;
-template<class P> bool solve_in_one(const mpm_context* c)
-{
-    return sizeof(TT<P>)==4&&c->coop&&c->scenes.size()==1&&c->hess_warp==HESS_AUTO&&c->n_total<=SOLVE_MAX;
-}
 // CTAs of k_cg_solve: at most those that fit the GPU at once (the launch is cooperative); fewer
-// for few particles, where more would only take part in the barriers.
+// for few particles, where more would only take part in the barriers (with units the kernel
+// sends those home).
 template<class P> cudaError_t launch_solve(mpm_context* c,cudaStream_t st,const DevState<TT<P>>& S2)
 {
     if constexpr(sizeof(TT<P>)==4){
@@ -288,7 +298,7 @@ template<class P> cudaError_t launch_solve(mpm_context* c,cudaStream_t st,const 
         cudaLaunchAttribute at[1];
         at[0].id=cudaLaunchAttributeCooperative;at[0].val.cooperative=1;
         cudaLaunchConfig_t cfg={};
-        cfg.gridDim=dim3((unsigned)std::min<long long>((long long)c->num_sms*std::max(per_sm,1),std::max<long long>(c->num_sms,c->n_total/128)));
+        cfg.gridDim=dim3((unsigned)std::min<long long>((long long)c->num_sms*std::max(per_sm,1),std::max<long long>(c->num_sms,c->n_total/(solve_units<P>(c)?64:128))));
         cfg.blockDim=dim3(XFER_THREADS);cfg.dynamicSmemBytes=smem;cfg.stream=st;cfg.attrs=at;cfg.numAttrs=1;
         return cudaLaunchKernelEx(&cfg,k_cg_solve<P>,S2,max_cg_iters(c)+1);}
     else return cudaErrorNotSupported;

@@ -86,12 +86,16 @@ struct ActiveList { int n; int scene[MAX_SCENES]; int cpre[MAX_SCENES+1]; int bp
 constexpr int ITEM_WORDS=32;
 enum { ITEM_START=0, ITEM_COUNT=1, ITEM_SCENE=2, ITEM_PAIRS=3, ITEM_NBR=4 };
 
+// A unit of k_cg_solve: SOLVE_UNIT pairs of a work item, one pass for each warp of a CTA.
+// Entry: work item << 6 | unit in the item (at most 4096 / 128 = 32).
+constexpr int SOLVE_UNIT=128;
 // Sums of one phase of k_cg_solve.
 struct SolveSlot { double sum[3]; unsigned long long max0; };
 struct Counters {
     // zeroed before every substep (up to `error`)
     SolveSlot solve[4];        // k_cg_solve, by phase mod 4
     unsigned solve_arrived;    // its grid barrier: arrivals so far
+    unsigned n_units;          // its units of work
     unsigned n_valid;          // valid particles after the key pass
     unsigned n_chunks;
     unsigned n_active;         // active node blocks
@@ -130,6 +134,7 @@ template<class T> struct DevState {
     // work items
     int* chunk_start; long long chunk_cap;
     int* src;                       // FP32: old slot of every new position (k_items)
+    int* units;                     // units of k_cg_solve, an item's in a row, items in any order
     unsigned* pairs;                // FP32 pair tables, a work item's from its first slot on (see pair_table)
     int* items;                     // work-item records
     // blocks

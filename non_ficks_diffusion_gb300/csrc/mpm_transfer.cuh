@@ -780,8 +780,8 @@ template<class T> __global__ void __launch_bounds__(256) k_permute(DevState<T> S
 // Clears the accumulated node channels, records each scene's range in the work-item list and
 // in the active-block list (SceneRange; the ranges were zeroed before the key pass) and, with
 // `order` (FP32 substeps), puts each work item's particles in storage order: their old slots
-// and keys by new position, the pair table and the record.
-template<class T> __global__ void __launch_bounds__(XFER_THREADS) k_items(DevState<T> S,int order)
+// and keys by new position, the pair table and the record, and with `units` those of k_cg_solve.
+template<class T> __global__ void __launch_bounds__(XFER_THREADS,10) k_items(DevState<T> S,int order,int units)
 {
     pdl_enter();
     constexpr int NW=XFER_THREADS/32;
@@ -816,6 +816,12 @@ template<class T> __global__ void __launch_bounds__(XFER_THREADS) k_items(DevSta
         chunk_cell_order(S.keys,ci.s,np,crank,ocnt,inv,loc,cellv,rank_end);
         const int pairs=pair_table(rank_end,cell_of,st,run,S.pairs+ci.s);
         if(warp==0) write_item(S,c,ci,nbr,np,pairs);
+        if(units&&warp==1){
+            const int nu=(pairs+SOLVE_UNIT-1)/SOLVE_UNIT,lane=threadIdx.x&31;
+            unsigned u0=0;
+            if(lane==0) u0=atomicAdd(&S.ctr->n_units,(unsigned)nu);
+            u0=__shfl_sync(0xffffffffu,u0,0);
+            if(lane<nu) S.units[u0+lane]=(int)((unsigned)c<<6)|lane;}
         const float rst=1.f/(float)st;
         for(int k=threadIdx.x;k<np;k+=blockDim.x){
             const int i=ci.s+slot_position(k,st,rst,run),j=inv[k];
@@ -1658,7 +1664,10 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
 // for a few. Here the CTAs stay: each keeps its work item's record (and, with one pass per
 // warp, its pairs) on chip, the node blocks are spread over all warps, and the phases
 // (product, vector update) are separated by grid barriers whose arrivals carry the sums.
-// With fewer work items than CTAs an item's passes are split over 2 or 4 CTAs.
+// The particles are dealt out in units of one pass per warp where there are CTAs for all of them: a
+// compressed block's item has four where most have one, and the CTA that took it kept all
+// others waiting (60K particles of compressed snow 230 -> 216 us a substep, 40K 201 -> 192,
+// 20K of fluid 200 -> 193).
 // =====================================================================================
 // One arrival per CTA, after warp 0 has run `pre`; thread 0 runs `idle` while the others arrive,
 // waits for all (bounded) and runs `post`. False after the limit. A round trip to L2 or a few
@@ -1690,6 +1699,7 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
 {
     using T=typename P::T;
     static_assert(sizeof(T)==4,"pair tables are FP32 only");
+    static_assert(SOLVE_UNIT==32*(XFER_THREADS/32),"a unit is one pass per warp");
     constexpr int NW=XFER_THREADS/32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int rec[ITEM_WORDS];
@@ -1705,14 +1715,23 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
     for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x) tmap[t]=tile_map_entry(t);
     for(int t=lane;t<3*TILE_S;t+=32) (&q[0][0])[t]=T(0);
     Counters* ctr=S.ctr;
-    const int G=(int)gridDim.x;
     const int nc=(int)min(ctr->n_chunks,(unsigned)S.chunk_cap),na=(int)min(ctr->n_active,(unsigned)S.block_cap);
-    const int split=4*nc<=G?4:2*nc<=G?2:1,units=nc*split;
+    // A CTA for each unit where the launch has that many: nobody waits for a compressed block.
+    // The CTAs without a unit or a warp's node block would only make the barriers longer. With
+    // more units than CTAs whole items, or halves or quarters of their passes, are cheaper: a
+    // second unit of another item is staged and flushed again (100K particles at rest 277
+    // against 255 us a substep, 900K 1,476 against 1,293).
+    const unsigned U=ctr->n_units;
+    const bool listed=U!=0u&&U<=gridDim.x;
+    const int G=listed?(int)min(gridDim.x,max(U,((unsigned)na+NW-1u)/NW)):(int)gridDim.x;
+    if((int)blockIdx.x>=G) return;
+    const int split=4*nc<=G?4:2*nc<=G?2:1,units=listed?(int)U:nc*split;
     const int per=(na+G*NW-1)/(G*NW),b0=min(na,((int)blockIdx.x*NW+warp)*per),b1=min(na,b0+per);
     const SceneDev<T>& sc=S.scenes[0];
     const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
     PairPass pass;                       // the warp's resident pass, when the CTA has one unit
-    int held=-1;                         // unit whose record is in rec
+    int held=-1;                         // unit whose item's record is in rec
+    unsigned entry=0;                    // its entry
     int phase=0;
     auto arrived=[&]{return (unsigned)(phase+1)*(unsigned)G;};
     // K v for v = x, or s = r + beta s_old with s^T K s into part[][0]
@@ -1720,13 +1739,15 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
         NodeSum<T> sks;
         for(int u=blockIdx.x;u<units;u+=G){
             if(u!=held){
+                entry=listed?(unsigned)S.units[u]:((unsigned)(u/split)<<6)|(unsigned)(u%split);
                 __syncthreads();
-                if(warp==0) rec[lane]=S.items[(long long)(u/split)*ITEM_WORDS+lane];
+                if(warp==0) rec[lane]=S.items[(long long)(entry>>6)*ITEM_WORDS+lane];
                 held=u;pass.ready=false;
                 __syncthreads();}
             stage_vector<T,XFER_THREADS>(S,rec+ITEM_NBR,tmap,from_x,beta,sv,threadIdx.x);
             __syncthreads();
-            hessian_pairs(S,sc,rec[ITEM_START],rec[ITEM_PAIRS],(warp+NW*(u%split))*32,NW*split*32,sv,q,slots,sks,pass);
+            const int M=rec[ITEM_PAIRS],parts=listed?(M+SOLVE_UNIT-1)/SOLVE_UNIT:split;
+            hessian_pairs(S,sc,rec[ITEM_START],M,(warp+NW*(int)(entry&63u))*32,NW*parts*32,sv,q,slots,sks,pass);
             __syncthreads();
             for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x){
                 const unsigned e=tmap[t];
