@@ -149,15 +149,19 @@ WORKLOADS_PRESET = {"c0": 100, "c1": 101, "c2": 102, "c3": 103, "c4": 104}
 
 def algorithmic_bytes(phase, n_particles, n_nodes, s):
     """Algorithmic DRAM bytes of one launch of a phase kernel (FP32/mixed: s=4, FP64: s=8).
-    p2g:     read 20 state words (through the sort order) + key + order index + id/scene,
-             write 20 state words + 11 cache words + id/scene; nodes: 2 vector accumulators.
-    hessian: read X(3) Fe(9) Re(9) lambda mu V0 + key; nodes: read r and s (4 words each),
-             accumulate q (4 words).
+    p2g:     read 20 state words (through the sort order) + order index + id/scene, write 20
+             state words + cache + id/scene; nodes: 2 vector accumulators. FP64 one kernel,
+             cache 20 words + key; FP32 two (the mean of both is given), cache 16 words
+             written and read again by the scatter with the pair table.
+    hessian: read 12 cache words + half a pair entry (FP64: 20 + key); nodes: read r and s
+             (4 words each), accumulate q (4 words).
     g2p:     read X V Fe + key, write X V Fe; nodes: read v and v* (4 words each)."""
     if phase == "p2g":
-        return n_particles * (51 * s + 24) + n_nodes * 8 * s
+        if s == 8:
+            return n_particles * (60 * s + 24) + n_nodes * 8 * s
+        return (n_particles * (72 * s + 22) + n_nodes * 8 * s) / 2
     if phase == "hessian":
-        return n_particles * (24 * s + 4) + n_nodes * 12 * s
+        return n_particles * ((20 * s + 4) if s == 8 else (12 * s + 2)) + n_nodes * 12 * s
     if phase == "g2p":
         return n_particles * (30 * s + 4) + n_nodes * 8 * s
     return None
@@ -392,7 +396,7 @@ def run_gb300(args, ws, rank, local):
     nodes_avg = node_sum / phase_steps
     if dominant == "hessian":
         # algorithmic bytes of all Hessian launches of the timed substeps over their count
-        scene_bytes = scene_n * (24 * s_bytes + 4) + nodes_avg * 12 * s_bytes
+        scene_bytes = algorithmic_bytes("hessian", scene_n, nodes_avg, s_bytes)
         alg = float((hess_scene_launches * scene_bytes).sum() / nl) if nl else None
     else:
         alg = algorithmic_bytes(dominant, n_particles, float(nodes_avg.sum()), s_bytes)
@@ -504,9 +508,11 @@ def run_gb300(args, ws, rank, local):
 
 
 def substep_bytes(n_particles, n_nodes, n_cg, s):
-    """Algorithmic DRAM bytes of one substep: N_p s (71 + 24 n_cg) + N_n s (20 + 29 n_cg)
-    (state, cache and grid channels each read or written once per phase)."""
-    return n_particles * s * (71 + 24 * n_cg) + n_nodes * s * (20 + 29 * n_cg)
+    """Algorithmic DRAM bytes of one substep (state, cache and grid channels each read or
+    written once per phase): N_p s (103 + 12 n_cg) + N_n s (20 + 33 n_cg), FP64 with 20
+    cache words."""
+    p, c = (95, 20) if s == 8 else (103, 12)
+    return n_particles * s * (p + c * n_cg) + n_nodes * s * (20 + 33 * n_cg)
 
 
 def run_accuracy(args):

@@ -45,7 +45,7 @@ typedef enum mpm_status {
 
 typedef enum mpm_precision {
     MPM_PRECISION_FP32 = 0,  /* everything FP32 (the reference's shipped T=float) */
-    MPM_PRECISION_MIXED = 1, /* FP32 state, transfers and CG vectors; FP64 SVD/polar, CG dots and norms */
+    MPM_PRECISION_MIXED = 1, /* FP32 state, transfers and CG vectors; SVD/polar to FP64-class accuracy, FP64 CG norms */
     MPM_PRECISION_FP64 = 2   /* everything FP64 (the reference built with T=double) */
 } mpm_precision;
 
@@ -276,7 +276,7 @@ MPM_API mpm_status mpm_advance_to_time(struct mpm_context* ctx, double target_ti
 typedef struct mpm_launch_config {
     int chunk;            /* particles per work item (the "particles per block" of a CTA) */
     int ctas_hessian;     /* occupancy variant: resident CTAs per SM the registers are capped */
-    int ctas_p2g;         /*   for (3, 4, 5, 6 or 8) */
+    int ctas_p2g;         /*   for (3, 4, 5, 6 or 8); P2G's scatter in FP32 storage */
     int ctas_g2p;
     int grid_per_sm;      /* CTAs per SM launched for the grid-stride loop over work items */
     int node_grid_per_sm; /* CTAs per SM of the node kernels (grid update, CG vector updates) */
@@ -286,7 +286,9 @@ typedef struct mpm_launch_config {
                                when the launch has at least as many work items as warps can be
                                resident (the first product and the early CG trips of a large
                                scene or batch), else a CTA per item (small scenes, and the last
-                               trips when few scenes still iterate).
+                               trips when few scenes still iterate). With 2, the graphs of a
+                               single FP32 or mixed scene of at most 2^20 particles run the
+                               whole CG as one cooperative kernel.
                                Default 2 */
     int incremental_sort; /* binning of a substep: 0 a full stable radix sort of the cell keys;
                              1 the same order obtained by sorting only the particles whose

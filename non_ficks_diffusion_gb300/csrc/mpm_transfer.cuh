@@ -353,14 +353,12 @@ __device__ __forceinline__ int list_find(const ListSmem& sm,int w)
 // MPM_Example.cpp:757-784). Reads the old particle buffer through the sort permutation and
 // writes the new one, cell-ordered inside every work item, with its keys and the CG cache.
 // =====================================================================================
-// Shared-memory bytes of one P2G / Hessian CTA: the warps' private tiles and, for P2G, the
+// Shared-memory bytes of one FP64 P2G CTA: the warps' private tiles and (also k_items) the
 // cell order of a work item of up to `chunk` particles (per-warp cell counts, slot -> item
 // map, item cells).
 template<class T> __host__ __device__ constexpr int p2g_tile_bytes(){return (XFER_THREADS/32)*7*TILE_S*(int)sizeof(T);}
 __host__ __device__ constexpr int order_bytes(int chunk){return (XFER_THREADS/32)*64*4+64*4+((chunk*5+15)&~15);}
 template<class T> __host__ __device__ constexpr int p2g_smem_bytes(int chunk){return p2g_tile_bytes<T>()+order_bytes(chunk);}
-template<class T> constexpr int hess_smem_bytes(){return (XFER_THREADS/32)*3*TILE_S*(int)sizeof(T)+3*TILE_S*(int)sizeof(T);}
-template<class T> constexpr int hess_warp_smem_bytes(){return (XFER_THREADS/32)*6*TILE_S*(int)sizeof(T);}
 
 // Scatter order of a block's 64 cells: by the shared-memory bank of the cell's tile address
 // (tile_addr mod 32), then by cell index. With TSZ = 40 every bank holds exactly two cells,
@@ -455,18 +453,11 @@ __device__ __forceinline__ void chunk_cell_order(const unsigned* keys,int s,int 
     __syncthreads();
 }
 
-// A vector over the three components of a node value. FP32 holds components 0 and 1 as a
-// packed pair (one instruction for two fused multiply-adds, each rounded like fmaf).
+// A vector over the three components of a node value (FP64).
 template<class T> struct C3 { T x,y,z; };
-template<> struct C3<float> { float2 xy; float z; };
 template<class T> __device__ __forceinline__ C3<T> c3(T x,T y,T z){return C3<T>{x,y,z};}
-template<> __device__ __forceinline__ C3<float> c3<float>(float x,float y,float z){return C3<float>{make_float2(x,y),z};}
-__device__ __forceinline__ C3<float> madd(const C3<float>& a,float s,const C3<float>& c){return C3<float>{pfma(a.xy,pdup(s),c.xy),fmaf(a.z,s,c.z)};}
 __device__ __forceinline__ C3<double> madd(const C3<double>& a,double s,const C3<double>& c){return C3<double>{fma(a.x,s,c.x),fma(a.y,s,c.y),fma(a.z,s,c.z)};}
-__device__ __forceinline__ C3<float> mul(const C3<float>& a,float s){return C3<float>{pmul(a.xy,pdup(s)),a.z*s};}
 __device__ __forceinline__ C3<double> mul(const C3<double>& a,double s){return C3<double>{a.x*s,a.y*s,a.z*s};}
-__device__ __forceinline__ float cx(const C3<float>& a){return a.xy.x;}
-__device__ __forceinline__ float cy(const C3<float>& a){return a.xy.y;}
 __device__ __forceinline__ double cx(const C3<double>& a){return a.x;}
 __device__ __forceinline__ double cy(const C3<double>& a){return a.y;}
 
