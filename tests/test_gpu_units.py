@@ -29,7 +29,8 @@ def test_units_match_the_oracle(built_lib, cells):
     rng = np.random.default_rng(7)
     cell = np.stack(np.meshgrid(*[np.arange(20, 28)] * 3, indexing="ij"), -1).reshape(-1, 3).repeat(8, 0)
     X = ((cell + 0.05 + 0.9 * rng.random((4096, 3))) / 32.0).astype(np.float32).astype(np.float64)
-    p = {k: np.concatenate([a, {"X": X, "V": np.zeros((4096, 3))}.get(k, np.full(4096, a[0]))]) for k, a in p.items()}
+    rest = {"X": X, "V": np.zeros((4096, 3)), **{k: np.full(4096, p[k][0]) for k in ("mass", "lambda0", "mu0")}}
+    p = {k: np.concatenate([p[k], rest[k]]) for k in p}
     n = len(p["mass"])
     ctx = capi.Context(precision="fp32", max_particles=n, max_scenes=1)
     ctx.add_scene(desc)
