@@ -508,11 +508,9 @@ def run_gb300(args, ws, rank, local):
 
 
 def substep_bytes(n_particles, n_nodes, n_cg, s):
-    """Algorithmic DRAM bytes of one substep (state, cache and grid channels each read or
-    written once per phase): N_p s (103 + 12 n_cg) + N_n s (20 + 33 n_cg), FP64 with 20
-    cache words."""
-    p, c = (95, 20) if s == 8 else (103, 12)
-    return n_particles * s * (p + c * n_cg) + n_nodes * s * (20 + 33 * n_cg)
+    """Algorithmic DRAM bytes of one substep: N_p s (71 + 24 n_cg) + N_n s (20 + 29 n_cg)
+    (state, cache and grid channels each read or written once per phase)."""
+    return n_particles * s * (71 + 24 * n_cg) + n_nodes * s * (20 + 29 * n_cg)
 
 
 def run_accuracy(args):

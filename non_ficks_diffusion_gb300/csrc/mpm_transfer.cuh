@@ -1657,8 +1657,8 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
 // (product, vector update) are separated by grid barriers whose arrivals carry the sums.
 // The particles are dealt out in units of one pass per warp where there are CTAs for all of them: a
 // compressed block's item has four where most have one, and the CTA that took it kept all
-// others waiting (60K particles of compressed snow 230 -> 216 us a substep, 40K 201 -> 192,
-// 20K of fluid 200 -> 193).
+// others waiting (61K particles of compressed snow 227 -> 210 us a substep, 40K 194 -> 186,
+// 20K of fluid 202 -> 191).
 // =====================================================================================
 // One arrival per CTA, after warp 0 has run `pre`; thread 0 runs `idle` while the others arrive,
 // waits for all (bounded) and runs `post`. False after the limit. A round trip to L2 or a few
