@@ -175,9 +175,9 @@ template<class P> DevState<TT<P>> make_state(mpm_context* c,int parity,double dt
 
 // Whether a graph's substep solves in one cooperative kernel (k_cg_solve): one scene in FP32
 // storage, the Hessian's form left to the library, at most SOLVE_MAX particles. Substeps
-// measured as a loop of kernels -> one kernel: 3K particles 158 -> 128 us, 20K 295 -> 222,
-// 61K 345 -> 281, 237K 342 -> 328, 400K 499 -> 454, 1.2M 1,218 -> 1,174; from 2M on the
-// loop with a warp per work item is faster (1,820 against 1,905, at 4M 3,454 against 3,910).
+// measured as a loop of kernels -> one kernel: 3K particles 143 -> 112 us, 20K 284 -> 193,
+// 61K 298 -> 207, 237K 308 -> 294, 400K 671 -> 578, 1M 1,377 -> 1,359; from 2M on the loop
+// with a warp per work item is faster (1,820 against 1,905, at 4M 3,454 against 3,910).
 constexpr long long SOLVE_MAX=1LL<<20;
 template<class P> bool solve_in_one(const mpm_context* c)
 {
