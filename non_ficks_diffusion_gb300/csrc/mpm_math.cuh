@@ -544,7 +544,9 @@ static __host__ __device__ __noinline__ ClampResult clamp_fp64_cold(ClampArgs a)
 //   R = F (I + e)^(-1/2) = F + F e (-1/2 + e (3/8 - e (5/16 - e 35/128))) + O(63/256 |e|^5).
 // e is evaluated to twice FP32 precision and the correction added last, so that R is the exact
 // rotation rounded to FP32, but for the series' end: below 2e-10 for |e| <= 0.0149 (Frobenius
-// norm, a bound of the eigenvalues of F^T F). Returns false, R untouched, when |e|^2 >= lim2.
+// norm, a bound of the eigenvalues of F^T F). Returns false, R untouched, when |e|^2 >= lim2
+// or det F < 0: e is as small near a reflection, whose least singular value is negative and
+// whose polar rotation is not F (1 + e)^(-1/2).
 constexpr float POLAR_SERIES_MAX=0.0149f;
 MPM_HD bool polar_near(const float* F,float lim2,float* R)
 {
@@ -552,6 +554,7 @@ MPM_HD bool polar_near(const float* F,float lim2,float* R)
     c[0]=F[0]*F[0]+F[3]*F[3]+(F[6]*F[6]-1.f);c[1]=F[0]*F[1]+F[3]*F[4]+F[6]*F[7];c[2]=F[0]*F[2]+F[3]*F[5]+F[6]*F[8];
     c[3]=F[1]*F[1]+F[4]*F[4]+(F[7]*F[7]-1.f);c[4]=F[1]*F[2]+F[4]*F[5]+F[7]*F[8];c[5]=F[2]*F[2]+F[5]*F[5]+(F[8]*F[8]-1.f);
     if(!(c[0]*c[0]+c[3]*c[3]+c[5]*c[5]+2.f*(c[1]*c[1]+c[2]*c[2]+c[4]*c[4])<lim2)) return false;
+    if(!(det3(F)>0.f)) return false;          // here |det F| is within 3 % of 1
     float e[6];
     {   const int a[6]={0,0,0,1,1,2},b[6]={0,1,2,1,2,2};
 #pragma unroll
