@@ -743,5 +743,103 @@ template<class T> MPM_HD void skew_system_inverse(const T* S,T* Ki)
 #pragma unroll
     for(int k=0;k<6;++k) Ki[k]*=inv;
 }
+// V0 P F^T (00, 01, 02, 11, 12, 22) of HessianData; an EOS fluid's pressure enters as -c I.
+template<class T> MPM_HD void transfer_stress(const HessianData<T>& h,bool eos,T* A)
+{
+    const T* E=h.E;
+    A[0]=h.c1*(E[0]+(E[0]*E[0]+E[1]*E[1]+E[2]*E[2]))+h.c3;
+    A[1]=h.c1*(E[1]+(E[0]*E[1]+E[1]*E[3]+E[2]*E[4]));
+    A[2]=h.c1*(E[2]+(E[0]*E[2]+E[1]*E[4]+E[2]*E[5]));
+    A[3]=h.c1*(E[3]+(E[1]*E[1]+E[3]*E[3]+E[4]*E[4]))+h.c3;
+    A[4]=h.c1*(E[4]+(E[1]*E[2]+E[3]*E[4]+E[4]*E[5]));
+    A[5]=h.c1*(E[5]+(E[2]*E[2]+E[4]*E[4]+E[5]*E[5]))+h.c3;
+    if(eos) A[0]=A[3]=A[5]=-E[0];
+}
+
+// A vector over the three components of a node value (FP64).
+template<class T> struct C3 { T x,y,z; };
+template<class T> MPM_HD C3<T> c3(T x,T y,T z){return C3<T>{x,y,z};}
+MPM_HD C3<double> madd(const C3<double>& a,double s,const C3<double>& c){return C3<double>{fma(a.x,s,c.x),fma(a.y,s,c.y),fma(a.z,s,c.z)};}
+MPM_HD C3<double> mul(const C3<double>& a,double s){return C3<double>{a.x*s,a.y*s,a.z*s};}
+MPM_HD double cx(const C3<double>& a){return a.x;}
+MPM_HD double cy(const C3<double>& a){return a.y;}
+
+// B = V0 dP Fe^T from G, by columns (HessianData), and bg = B:G, the particle's part of
+// s^T K s. FP32 solves the 3x3 system of the rotation part itself (hessian_stress2); FP64, whose
+// arithmetic is 64 times slower against the same memory, reads the inverse that P2G stored.
+template<class T> MPM_HD void hessian_stress(const C3<T> (&G)[3],const T* Sm,T c1,T c2,T cc3,const T* Ki,C3<T> (&B)[3],T& bg)
+{
+    const T S[3][3]={{Sm[0],Sm[1],Sm[2]},{Sm[1],Sm[3],Sm[4]},{Sm[2],Sm[4],Sm[5]}};
+    C3<T> M[3];
+#pragma unroll
+    for(int j=0;j<3;++j) M[j]=madd(G[2],S[2][j],madd(G[1],S[1][j],mul(G[0],S[0][j])));
+    const T L0=cy(M[0])-cx(M[1]),L1=M[0].z-cx(M[2]),L2=M[1].z-cy(M[2]);
+    const T a=Ki[0]*L0+Ki[1]*L1+Ki[2]*L2,b=Ki[1]*L0+Ki[3]*L1+Ki[4]*L2,c=Ki[2]*L0+Ki[4]*L1+Ki[5]*L2;
+    const C3<T> N[3]={c3<T>(cx(M[0]),cy(M[0])-a,M[0].z-b),c3<T>(cx(M[1])+a,cy(M[1]),M[1].z-c),c3<T>(cx(M[2])+b,cy(M[2])+c,M[2].z)};
+    const T tr=c2*(cx(G[0])+cy(G[1])+G[2].z);
+    // columns j of -c3 G^T (rows j of G), then c1 N S and the trace on the diagonal
+    const C3<T> gt[3]={c3<T>(cx(G[0]),cx(G[1]),cx(G[2])),c3<T>(cy(G[0]),cy(G[1]),cy(G[2])),c3<T>(G[0].z,G[1].z,G[2].z)};
+#pragma unroll
+    for(int j=0;j<3;++j)
+        B[j]=madd(N[2],c1*S[2][j],madd(N[1],c1*S[1][j],madd(N[0],c1*S[0][j],mul(gt[j],-cc3))));
+    B[0]=c3<T>(cx(B[0])+tr,cy(B[0]),B[0].z);B[1]=c3<T>(cx(B[1]),cy(B[1])+tr,B[1].z);B[2]=c3<T>(cx(B[2]),cy(B[2]),B[2].z+tr);
+    bg=T(0);
+#pragma unroll
+    for(int j=0;j<3;++j) bg+=cx(B[j])*cx(G[j])+cy(B[j])*cy(G[j])+B[j].z*G[j].z;
+}
+
+// Packed pairs of single-precision operations: one instruction does the work of two, and
+// each half rounds exactly like the scalar fmaf / multiply / sum (their form in host code).
+MPM_HD float2 pdup(float a){return make_float2(a,a);}
+#if defined(__CUDA_ARCH__)&&__CUDA_ARCH__>=1000
+MPM_HD float2 pfma(float2 a,float2 b,float2 c){return __ffma2_rn(a,b,c);}
+MPM_HD float2 pmul(float2 a,float2 b){return __fmul2_rn(a,b);}
+MPM_HD float2 padd(float2 a,float2 b){return __fadd2_rn(a,b);}
+#else
+MPM_HD float2 pfma(float2 a,float2 b,float2 c){return make_float2(fmaf(a.x,b.x,c.x),fmaf(a.y,b.y,c.y));}
+MPM_HD float2 pmul(float2 a,float2 b){return make_float2(a.x*b.x,a.y*b.y);}
+MPM_HD float2 padd(float2 a,float2 b){return make_float2(a.x+b.x,a.y+b.y);}
+#endif
+MPM_HD float2 psub(float2 a,float2 b){return pfma(b,make_float2(-1.f,-1.f),a);}   // exact product: rounds like a - b
+// transfer_stress for two particles of snow.
+MPM_HD void transfer_stress2(const float2 (&E)[6],float2 c1,float2 c3,float2 (&A)[6])
+{
+    auto dot=[&](int a,int b,int c,int d,int e,int f){return pfma(E[e],E[f],pfma(E[c],E[d],pmul(E[a],E[b])));};
+    A[0]=pfma(c1,padd(E[0],dot(0,0,1,1,2,2)),c3);A[1]=pmul(c1,padd(E[1],dot(0,1,1,3,2,4)));
+    A[2]=pmul(c1,padd(E[2],dot(0,2,1,4,2,5)));A[3]=pfma(c1,padd(E[3],dot(1,1,3,3,4,4)),c3);
+    A[4]=pmul(c1,padd(E[4],dot(1,2,3,4,4,5)));A[5]=pfma(c1,padd(E[5],dot(2,2,4,4,5,5)),c3);
+}
+// B = V0 dP Fe^T from G for two particles (hessian_stress).
+MPM_HD void hessian_stress2(const float2 (&G)[3][3],const float2 (&Sm)[6],float2 c1,float2 c2,float2 cc3,float2 (&B)[3][3],float2& bg)
+{
+    const int ix[3][3]={{0,1,2},{1,3,4},{2,4,5}};
+    float2 M[3][3];
+#pragma unroll
+    for(int i=0;i<3;++i)
+#pragma unroll
+        for(int j=0;j<3;++j) M[i][j]=pfma(G[i][2],Sm[ix[2][j]],pfma(G[i][1],Sm[ix[1][j]],pmul(G[i][0],Sm[ix[0][j]])));
+    // K a = L for the axial vector (a, b, c) of W' (skew_system_inverse)
+    const float2 k00=padd(Sm[3],Sm[0]),k01=Sm[4],k02=pmul(Sm[2],pdup(-1.f)),k11=padd(Sm[5],Sm[0]),k12=Sm[1],k22=padd(Sm[5],Sm[3]);
+    auto det2=[](float2 p,float2 q,float2 r,float2 s){return psub(pmul(p,q),pmul(r,s));};
+    const float2 i00=det2(k11,k22,k12,k12),i01=det2(k02,k12,k01,k22),i02=det2(k01,k12,k02,k11);
+    const float2 i11=det2(k00,k22,k02,k02),i12=det2(k01,k02,k00,k12),i22=det2(k00,k11,k01,k01);
+    const float2 det=pfma(k02,i02,pfma(k01,i01,pmul(k00,i00)));
+    const float2 inv=make_float2(1.f/det.x,1.f/det.y);
+    const float2 L0=pmul(psub(M[1][0],M[0][1]),inv),L1=pmul(psub(M[2][0],M[0][2]),inv),L2=pmul(psub(M[2][1],M[1][2]),inv);
+    const float2 a=pfma(i02,L2,pfma(i01,L1,pmul(i00,L0))),b=pfma(i12,L2,pfma(i11,L1,pmul(i01,L0))),c=pfma(i22,L2,pfma(i12,L1,pmul(i02,L0)));
+    M[0][1]=padd(M[0][1],a);M[0][2]=padd(M[0][2],b);M[1][2]=padd(M[1][2],c);
+    M[1][0]=psub(M[1][0],a);M[2][0]=psub(M[2][0],b);M[2][1]=psub(M[2][1],c);
+    const float2 tr=pmul(c2,padd(padd(G[0][0],G[1][1]),G[2][2])),n3=pmul(cc3,pdup(-1.f));
+    float2 cS[6];
+#pragma unroll
+    for(int k=0;k<6;++k) cS[k]=pmul(c1,Sm[k]);
+#pragma unroll
+    for(int i=0;i<3;++i)
+#pragma unroll
+        for(int j=0;j<3;++j){
+            const float2 g=i==j?pfma(n3,G[j][i],tr):pmul(n3,G[j][i]);
+            B[i][j]=pfma(M[i][2],cS[ix[2][j]],pfma(M[i][1],cS[ix[1][j]],pfma(M[i][0],cS[ix[0][j]],g)));
+            bg=i==0&&j==0?pmul(B[i][j],G[i][j]):pfma(B[i][j],G[i][j],bg);}
+}
 
 } // namespace mpm
