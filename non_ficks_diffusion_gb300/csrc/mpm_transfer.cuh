@@ -1139,10 +1139,31 @@ __device__ __forceinline__ unsigned tile_map_entry(int t)
     const int idx=(tx+3)/4+3*((ty+3)/4)+9*((tz+3)/4),l=((tx+3)&3)|(((ty+3)&3)<<2)|(((tz+3)&3)<<4);
     return (unsigned)idx|((unsigned)l<<5)|((unsigned)tile_addr(t)<<11);
 }
-// The gathered vector at the item's tile nodes, by NT threads: the loads of a batch of nodes
+// The products scale the gathered vector by the power of two below dt: G, and with it B, K s and
+// s^T K s, then have the magnitudes that dt^2 K has beside the masses, in range where a stiff
+// material's own are not (at 6e25 Pa and 1e10 m/s FP32 overflows in s^T K s). The scaling is
+// exact: no bit changes where nothing leaves the range.
+template<class T> struct ProductScale {
+    T scale;       // of the gathered vector, so of K s in the grid; s^T K s has its square
+    T kdt;         // dt^2/scale, for K s
+    T sks;         // dt^2/scale^2, for s^T K s
+    __device__ __forceinline__ explicit ProductScale(T dt)
+    {
+        T inv;
+        if constexpr(sizeof(T)==4){
+            const int e=min(max(__float_as_int(dt)&0x7f800000,0x00800000),0x7e800000);
+            scale=__int_as_float(e);inv=__int_as_float(0x7f000000-e);}
+        else{
+            const int e=min(max(__double2hiint(dt)&0x7ff00000,0x00100000),0x7fd00000);
+            scale=__hiloint2double(e,0);inv=__hiloint2double(0x7fe00000-e,0);}
+        const T f=dt*inv;
+        kdt=dt*f;sks=f*f;
+    }
+};
+// The gathered vector at the item's tile nodes, times `scale`, by NT threads: the loads of a batch of nodes
 // are all issued before one is used (a node's address needs only the item record).
 template<class T,int NT> __device__ __forceinline__ void stage_vector(const DevState<T>& S,const int* nbr,const unsigned* tmap,bool from_x,
-    T beta,T (*sv)[TILE_S],int tid)
+    T beta,T scale,T (*sv)[TILE_S],int tid)
 {
     constexpr int IT=(TILE_N+NT-1)/NT,BATCH=sizeof(T)==8?1:IT;
 #pragma unroll
@@ -1162,9 +1183,9 @@ template<class T,int NT> __device__ __forceinline__ void stage_vector(const DevS
                     else{a[i]=S.gr[node];b[i]=S.gs[node];}}}}
 #pragma unroll
         for(int i=0;i<BATCH;++i) if(ta[i]!=~0u){
-            sv[0][ta[i]]=from_x?a[i].x:a[i].x+beta*b[i].x;
-            sv[1][ta[i]]=from_x?a[i].y:a[i].y+beta*b[i].y;
-            sv[2][ta[i]]=from_x?a[i].z:a[i].z+beta*b[i].z;}}
+            sv[0][ta[i]]=scale*(from_x?a[i].x:a[i].x+beta*b[i].x);
+            sv[1][ta[i]]=scale*(from_x?a[i].y:a[i].y+beta*b[i].y);
+            sv[2][ta[i]]=scale*(from_x?a[i].z:a[i].z+beta*b[i].z);}}
 }
 // Adds an item's sum at a tile node to the grid.
 template<class T> __device__ __forceinline__ void add_tile_node(const DevState<T>& S,const int* rec,unsigned e,T v0,T v1,T v2)
@@ -1199,6 +1220,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
     auto item=[&](long long w){
         if(FROM_X) return w;
         const int j=list_find(lsm,(int)w);return S.srange[lsm.scene[j]].c0+(w-lsm.pre[j]);};
+    const T scale=ProductScale<T>((T)(*S.dtp)).scale;
     // s^T K s of a loop trip (k_cg_update), per lane until the warp's scene changes
     NodeSum<T> sks;int sks_scene=-1;
     auto add_sks=[&](int next){
@@ -1222,7 +1244,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
             __syncthreads();
             if(w+gridDim.x<nwork) mine=S.items[item(w+gridDim.x)*ITEM_WORDS+lane];
             const int scene=rec[ITEM_SCENE];
-            stage_vector<T,XFER_THREADS>(S,rec+ITEM_NBR,tmap,FROM_X,FROM_X?T(0):(T)S.cg[scene].beta,sv,threadIdx.x);
+            stage_vector<T,XFER_THREADS>(S,rec+ITEM_NBR,tmap,FROM_X,FROM_X?T(0):(T)S.cg[scene].beta,scale,sv,threadIdx.x);
             if constexpr(sizeof(T)==8) if(warp==0) chunk_runs(rec[ITEM_COUNT],(rec[ITEM_COUNT]+31)>>5,run);
             __syncthreads();
             add_sks(scene);
@@ -1250,7 +1272,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
             __syncwarp();
             if(w+dw<nwork) mine=S.items[item(w+dw)*ITEM_WORDS+lane];
             const int scene=rec[ITEM_SCENE];
-            stage_vector<T,32>(S,rec+ITEM_NBR,tmap,FROM_X,FROM_X?T(0):(T)S.cg[scene].beta,sv,lane);
+            stage_vector<T,32>(S,rec+ITEM_NBR,tmap,FROM_X,FROM_X?T(0):(T)S.cg[scene].beta,scale,sv,lane);
             if constexpr(sizeof(T)==8) chunk_runs(rec[ITEM_COUNT],(rec[ITEM_COUNT]+31)>>5,run);
             __syncwarp();
             add_sks(scene);
@@ -1405,7 +1427,7 @@ template<int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) k_p2g_sc
 // r = b - (x + dt^2/m K x) on a node block, two nodes per lane, Project(r) (MPM_CG_System.h:
 // 220-225, intended semantics of Project_Helper.h:30-45; the grid update flagged the nodes),
 // K x cleared; <r,r>_M and max|r|^2.
-template<class T> __device__ __forceinline__ void cg_start_block(const DevState<T>& S,int blk,T dt2,NodeSum<T>& rr,T& amax)
+template<class T> __device__ __forceinline__ void cg_start_block(const DevState<T>& S,int blk,T kdt,NodeSum<T>& rr,T& amax)
 {
     T m[2];V4<T> x[2],b[2],k[2];unsigned char pj[2];
 #pragma unroll
@@ -1414,7 +1436,7 @@ template<class T> __device__ __forceinline__ void cg_start_block(const DevState<
     for(int h=0;h<2;++h){
         const long long n=((long long)blk<<6)+h*32+(threadIdx.x&31);
         if(m[h]>T(0)){
-            const T c=dt2/m[h];
+            const T c=kdt/m[h];
             T r[3]={b[h].x-(c*k[h].x+x[h].x),b[h].y-(c*k[h].y+x[h].y),b[h].z-(c*k[h].z+x[h].z)};
             if(pj[h]) r[0]=r[1]=r[2]=T(0);
             S.gr[n]=V4<T>{r[0],r[1],r[2],T(0)};
@@ -1424,7 +1446,7 @@ template<class T> __device__ __forceinline__ void cg_start_block(const DevState<
         S.gf[n]=V4<T>{T(0),T(0),T(0),T(0)};}
 }
 // The vector update of a loop trip (k_cg_update) on the node block that starts at node n0.
-template<class T> __device__ __forceinline__ void cg_update_block(const DevState<T>& S,long long n0,T alpha,T beta,T dt2,NodeSum<T>& rr,NodeSum<T>& rs,
+template<class T> __device__ __forceinline__ void cg_update_block(const DevState<T>& S,long long n0,T alpha,T beta,T kdt,NodeSum<T>& rr,NodeSum<T>& rs,
     NodeSum<T>& ss,T& amax)
 {
     T m[2];V4<T> s[2],k[2],x[2],r[2];unsigned char pj[2];
@@ -1434,7 +1456,7 @@ template<class T> __device__ __forceinline__ void cg_update_block(const DevState
     for(int h=0;h<2;++h){
         const long long n=n0+h*32+(threadIdx.x&31);
         if(m[h]>T(0)){
-            const T c=dt2/m[h];
+            const T c=kdt/m[h];
             s[h].x=r[h].x+beta*s[h].x;s[h].y=r[h].y+beta*s[h].y;s[h].z=r[h].z+beta*s[h].z;
             T q[3]={c*k[h].x+s[h].x,c*k[h].y+s[h].y,c*k[h].z+s[h].z};
             if(pj[h]) q[0]=q[1]=q[2]=T(0);
@@ -1456,7 +1478,7 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_start(Dev
     using T=typename P::T;
     __shared__ WarpParts W;
     const int na=(int)min(S.ctr->n_active,(unsigned)S.block_cap);
-    const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
+    const T kdt=ProductScale<T>((T)(*S.dtp)).kdt;
     const WarpRange wr(na);
     if(blockIdx.x>=wr.parts) return;
     if((threadIdx.x&31)==0) W.scene[threadIdx.x>>5]=-1;
@@ -1465,7 +1487,7 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_start(Dev
     for(int blk=wr.b;blk<wr.b1;++blk){
         const int sb=S.active_scene[blk];
         if(sb!=scene){if(scene>=0) flush(scene,false);scene=sb;}
-        cg_start_block(S,blk,dt2,rr,amax);}
+        cg_start_block(S,blk,kdt,rr,amax);}
     if(scene>=0) flush(scene,true);
     __shared__ int any;
     if(threadIdx.x==0) any=0;
@@ -1503,7 +1525,7 @@ struct WarpBlocks {
 // The vector update of a loop trip, one pass over the nodes: s = r + beta s_old, q = s +
 // dt^2/m K s, Project(q), x += alpha s, r -= alpha q (Interior only), K s cleared for the next
 // product. alpha = <r,r>_M / <s,q>_M needs no pass of its own over the nodes: <s,q>_M =
-// dt^2 s^T K s + <s,s>_M, of which the Hessian product adds up s^T K s over the particles
+// dt^2 s^T K s + <s,s>_M, of which the Hessian product adds up s^T K s (scaled) over the particles
 // (sum of B:G) and the previous update <s,s>_M = <r,r> + 2 beta <r,s_old> + beta^2
 // <s_old,s_old> (s vanishes at projected nodes). Then the convergence check: stop when
 // max|r| <= tol (and iters >= min, or the norm is below epsilon) or at cg_max_iters; else beta
@@ -1521,7 +1543,7 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
     if((threadIdx.x&31)==0) W.scene[threadIdx.x>>5]=-1;
     load_active_list(S.alist,lsm,true);     // the scenes still iterating
     WarpBlocks wb(wr);
-    const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
+    const ProductScale<T> ps((T)(*S.dtp));
     NodeSum<T> rr,rs,ss;T amax=T(0),alpha=T(0),beta=T(0);
     auto flush=[&](int sc,bool last){
         flush_scene<3,T>(W,S.acc,sc,last,rr,rs,ss,amax);
@@ -1531,9 +1553,9 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
         if(wb.next(lsm,S.srange,bw)){
             if(prev>=0) flush(prev,false);
             const CGState& st=S.cg[wb.scene];
-            const double sq=(double)dt2*S.acc[wb.scene].sks+st.msq;
+            const double sq=(double)ps.sks*S.acc[wb.scene].sks+st.msq;
             alpha=(T)(sq!=0.?st.rho/sq:(double)FLT_MAX);beta=(T)st.beta;}
-        cg_update_block(S,wb.node0(bw),alpha,beta,dt2,rr,rs,ss,amax);}
+        cg_update_block(S,wb.node0(bw),alpha,beta,ps.kdt,rr,rs,ss,amax);}
     if(wb.scene>=0) flush(wb.scene,true);
     __shared__ int any;
     if(threadIdx.x==0) any=0;
@@ -1632,7 +1654,7 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
     const int split=4*nc<=G?4:2*nc<=G?2:1,units=listed?(int)U:nc*split;
     const int per=(na+G*NW-1)/(G*NW),b0=min(na,((int)blockIdx.x*NW+warp)*per),b1=min(na,b0+per);
     const SceneDev<T>& sc=S.scenes[0];
-    const T dtT=(T)(*S.dtp),dt2=dtT*dtT;
+    const ProductScale<T> ps((T)(*S.dtp));
     PairPass pass;                       // the warp's resident pass, when the CTA has one unit
     int held=-1;                         // unit whose item's record is in rec
     unsigned entry=0;                    // its entry
@@ -1648,7 +1670,7 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
                 if(warp==0) rec[lane]=S.items[(long long)(entry>>6)*ITEM_WORDS+lane];
                 held=u;pass.ready=false;
                 __syncthreads();}
-            stage_vector<T,XFER_THREADS>(S,rec+ITEM_NBR,tmap,from_x,beta,sv,threadIdx.x);
+            stage_vector<T,XFER_THREADS>(S,rec+ITEM_NBR,tmap,from_x,beta,ps.scale,sv,threadIdx.x);
             __syncthreads();
             const int M=rec[ITEM_PAIRS],parts=listed?(M+SOLVE_UNIT-1)/SOLVE_UNIT:split;
             hessian_pairs(S,sc,rec[ITEM_START],M,(warp+NW*(int)(entry&63u))*32,NW*parts*32,sv,q,slots,sks,pass);
@@ -1685,7 +1707,7 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
     if(!solve_barrier(ctr,arrived(),[]{},clear_ahead,[]{})) return;
     ++phase;
     {   NodeSum<T> rr;T amax=T(0);
-        for(int blk=b0;blk<b1;++blk) cg_start_block(S,blk,dt2,rr,amax);
+        for(int blk=b0;blk<b1;++blk) cg_start_block(S,blk,ps.kdt,rr,amax);
         const double a=warp_value(rr),m=(double)warp_max<T>(amax);
         if(lane==0){part[warp][0]=a;part[warp][3]=m;}}
     double rho=0.,msq=0.,rmax=0.,beta=0.,rs_sum=0.,ss_sum=0.;        // thread 0 of every CTA: equal values
@@ -1706,12 +1728,12 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
             clear_ahead();
             if(phase>2) msq=rho+beta*(2.*rs_sum+beta*ss_sum);},[&]{
             double s[3],mx;read_slot(s,mx);
-            const double sq=(double)dt2*s[0]+msq;
+            const double sq=(double)ps.sks*s[0]+msq;
             sh_alpha=(T)(sq!=0.?rho/sq:(double)FLT_MAX);})) return;
         ++phase;
         {   const T alpha=sh_alpha;
             NodeSum<T> rr,rs,ss;T amax=T(0);
-            for(int blk=b0;blk<b1;++blk) cg_update_block(S,((long long)blk<<6),alpha,be,dt2,rr,rs,ss,amax);
+            for(int blk=b0;blk<b1;++blk) cg_update_block(S,((long long)blk<<6),alpha,be,ps.kdt,rr,rs,ss,amax);
             const double a=warp_value(rr),b=warp_value(rs),c=warp_value(ss),m=(double)warp_max<T>(amax);
             if(lane==0){part[warp][0]=a;part[warp][1]=b;part[warp][2]=c;part[warp][3]=m;}}
         if(!solve_barrier(ctr,arrived(),[&]{contribute(3,true);},clear_ahead,[&]{

@@ -3,8 +3,9 @@ precision against the oracle of that precision. The clamp brings the negative si
 back to the lower limit, so that det Fe is positive again and Jp is about -1/0.975.
 
 Tolerance of Jp: about 30 FP32 roundings of a quotient of products (64 of 2^-24), mixed one
-rounding of the result (2), FP64 as its Jacobi SVD (1e-12). det Fe after the substep: the limits'
-product 0.975 * 1.0075^2 changed by dt grad v, below 1e-4 * 100 at these speeds."""
+rounding of the result (2), FP64 as its Jacobi SVD (1e-12). Fe moves by dt grad v Fe, and both
+sides stop their CG at the same residual: velocities within 4 of it, gradients 64 (2/dx) times
+that along each axis, and the FP32 rounding of entries near 1."""
 import numpy as np
 import pytest
 
@@ -36,5 +37,6 @@ def test_inverted_particles_match_the_oracle(built_lib, prec, tol):
     flipped = np.linalg.det(fe) < 0
     assert (r["Jp"][flipped] < -1.02).all()
     assert np.abs(g["Jp"] / r["Jp"] - 1).max() <= tol
-    assert np.abs(np.linalg.det(g["Fe"][flipped]) - 0.975 * 1.004 ** 2).max() < 0.02
+    assert (np.linalg.det(g["Fe"][flipped]) > 0).all()
+    assert np.abs(g["Fe"] - r["Fe"]).max() <= 1e-6 * 2 * 64 * 4 * o.stats()["cg_tolerance"] + 64 * 2.0 ** -24
     assert np.array_equal(g["valid"], r["valid"])
