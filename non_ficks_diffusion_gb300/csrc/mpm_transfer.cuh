@@ -1204,6 +1204,7 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
     __shared__ int run_s[sizeof(T)==8?NW:1][129];
     __shared__ unsigned tmap[TILE_N];
     __shared__ ListSmem lsm;
+    __shared__ T scale;                            // a register of it would make the product spill
     const int warp=threadIdx.x>>5,lane=threadIdx.x&31;
     // the first product (FROM_X) covers every work item; a loop trip only the work items of
     // the scenes still iterating (the list the previous convergence check wrote)
@@ -1215,12 +1216,12 @@ template<class P,bool FROM_X,int MINB> __global__ void __launch_bounds__(XFER_TH
     V4<float> (*slots)[32]=reinterpret_cast<V4<float> (*)[32]>(smem_raw+warp*hess_warp_bytes<T>()+6*TILE_S*sizeof(T));
     for(int t=threadIdx.x;t<TILE_N;t+=blockDim.x) tmap[t]=tile_map_entry(t);
     for(int t=lane;t<3*TILE_S;t+=32) (&q[0][0])[t]=T(0);
+    if(threadIdx.x==0) scale=ProductScale<T>((T)(*S.dtp)).scale;
     if(!FROM_X) load_active_list(S.alist,lsm,false);
     __syncthreads();
     auto item=[&](long long w){
         if(FROM_X) return w;
         const int j=list_find(lsm,(int)w);return S.srange[lsm.scene[j]].c0+(w-lsm.pre[j]);};
-    const T scale=ProductScale<T>((T)(*S.dtp)).scale;
     // s^T K s of a loop trip (k_cg_update), per lane until the warp's scene changes
     NodeSum<T> sks;int sks_scene=-1;
     auto add_sks=[&](int next){
