@@ -788,6 +788,15 @@ template<class T> MPM_HD void hessian_stress(const C3<T> (&G)[3],const T* Sm,T c
     for(int j=0;j<3;++j) bg+=cx(B[j])*cx(G[j])+cy(B[j])*cy(G[j])+B[j].z*G[j].z;
 }
 
+// The same of an EOS fluid, a trace: its E holds the pressure, of any size, and snow's 3x3
+// system would take its third power (FP32 overflows above 1e13: 0 * inf in the force).
+template<class T> MPM_HD void fluid_stress(const C3<T> (&G)[3],T c2,C3<T> (&B)[3],T& bg)
+{
+    const T g=cx(G[0])+cy(G[1])+G[2].z,tr=c2*g;
+    B[0]=c3<T>(tr,T(0),T(0));B[1]=c3<T>(T(0),tr,T(0));B[2]=c3<T>(T(0),T(0),tr);
+    bg=tr*g;
+}
+
 // Packed pairs of single-precision operations: one instruction does the work of two, and
 // each half rounds exactly like the scalar fmaf / multiply / sum (their form in host code).
 MPM_HD float2 pdup(float a){return make_float2(a,a);}
@@ -840,6 +849,15 @@ MPM_HD void hessian_stress2(const float2 (&G)[3][3],const float2 (&Sm)[6],float2
             const float2 g=i==j?pfma(n3,G[j][i],tr):pmul(n3,G[j][i]);
             B[i][j]=pfma(M[i][2],cS[ix[2][j]],pfma(M[i][1],cS[ix[1][j]],pfma(M[i][0],cS[ix[0][j]],g)));
             bg=i==0&&j==0?pmul(B[i][j],G[i][j]):pfma(B[i][j],G[i][j],bg);}
+}
+MPM_HD void fluid_stress2(const float2 (&G)[3][3],float2 c2,float2 (&B)[3][3],float2& bg)
+{
+    const float2 g=padd(padd(G[0][0],G[1][1]),G[2][2]),tr=pmul(c2,g);
+#pragma unroll
+    for(int i=0;i<3;++i)
+#pragma unroll
+        for(int j=0;j<3;++j) B[i][j]=i==j?tr:pdup(0.f);
+    bg=pmul(tr,g);
 }
 
 } // namespace mpm

@@ -976,7 +976,9 @@ __device__ __forceinline__ void hessian_pass(const DevState<double>& S,const Sce
         stencil_from_coord(sc,cell,x,st);
         C3<T> G[3];
         gather_grad(st,sv,G);
-        T bg;hessian_stress<T>(G,Sm,q0.w,q2.z,q2.w,Ki,B,bg);
+        T bg;
+        if(sc.eos) fluid_stress<T>(G,q2.z,B,bg);
+        else hessian_stress<T>(G,Sm,q0.w,q2.z,q2.w,Ki,B,bg);
         sks.add(bg);}
     const ScatterRounds R(valid,cell);
     for(int r=0;r<R.rounds;++r){
@@ -1069,14 +1071,17 @@ __device__ __forceinline__ void hessian_pairs(const DevState<float>& S,const Sce
                     G[a][0]=first?pmul(t,dxy):pfma(t,dxy,G[a][0]);
                     G[a][1]=first?pmul(t,xdy):pfma(t,xdy,G[a][1]);
                     G[a][2]=first?pmul(u,wxy):pfma(u,wxy,G[a][2]);}}
-            const V4<float> p1=slots[1][lane],q1=slots[4][lane],p2=slots[2][lane],q2=slots[5][lane];
-            const float2 one=pdup(1.f);
-            const float2 Sm[6]={padd(one,make_float2(p1.x,q1.x)),make_float2(p1.y,q1.y),make_float2(p1.z,q1.z),
-                                padd(one,make_float2(p1.w,q1.w)),make_float2(p2.x,q2.x),padd(one,make_float2(p2.y,q2.y))};
+            const V4<float> p2=slots[2][lane],q2=slots[5][lane];
             const bool two=(entry&PAIR_TWO)!=0u;                    // no second particle: no force
+            const float2 c2=make_float2(p2.z,two?q2.z:0.f);
             float2 bg;
-            hessian_stress2(G,Sm,make_float2(slots[0][lane].w,two?slots[3][lane].w:0.f),make_float2(p2.z,two?q2.z:0.f),
-                            make_float2(p2.w,two?q2.w:0.f),B,bg);
+            if(sc.eos) fluid_stress2(G,c2,B,bg);                    // uniform
+            else{
+                const V4<float> p1=slots[1][lane],q1=slots[4][lane];
+                const float2 one=pdup(1.f);
+                const float2 Sm[6]={padd(one,make_float2(p1.x,q1.x)),make_float2(p1.y,q1.y),make_float2(p1.z,q1.z),
+                                    padd(one,make_float2(p1.w,q1.w)),make_float2(p2.x,q2.x),padd(one,make_float2(p2.y,q2.y))};
+                hessian_stress2(G,Sm,make_float2(slots[0][lane].w,two?slots[3][lane].w:0.f),c2,make_float2(p2.w,two?q2.w:0.f),B,bg);}
             sks.add(bg.x+bg.y);
             weights(w,dw);}
         entry=next;
