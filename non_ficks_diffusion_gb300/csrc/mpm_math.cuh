@@ -397,6 +397,10 @@ MPM_HD F2x ff_prod(F2x a,F2x b){const float p=ff_mul(a.h,b.h);return ff_norm(F2x
 // bounded for the clamp (its first quotient lies in [0, 1]); f = 1 gives the rotation. The
 // neglected terms are of order E^2. Fe, Re = U (f + N - (dU f + f dV)/2) V^T, the leading
 // product to twice FP32 precision.
+//
+// For bands wider than CLAMP_MIN_BAND: only then are no singular values near both limits (below,
+// within 1e-4), and limits that cross (where the lower one wins) are left to the plain form.
+constexpr float CLAMP_MIN_BAND=3e-4f;
 MPM_HD void clamp_refined(float* Fe,float& Jp,const float* U,const float* V,const float cy,const float sy,float* Re,float& Je)
 {
     float dU[9],dV[9];               // symmetric
@@ -597,8 +601,9 @@ template<class T> MPM_HD void harden(const T Jp,const T lambda0,const T mu0,cons
 // only the polar rotation Re is needed, refined in FP64 from the FP32 U V^T by
 // polar_refine3 or polar_refine_mixed. Otherwise the mixed variant corrects the FP32 SVD to
 // FP32 rounding of the exact clamp (clamp_refined); for singular values far from 1, where the
-// correction's quotients are not well conditioned, and in the FP64 variant the FP64 Jacobi
-// SVD runs, warm-started from the FP32 V, and clamp and reconstruction are done in FP64.
+// correction's quotients are not well conditioned, for a yield band that is hardly one
+// (CLAMP_MIN_BAND) and in the FP64 variant the FP64 Jacobi SVD runs, warm-started from the
+// FP32 V, and clamp and reconstruction are done in FP64.
 template<class T,class TS> MPM_HD void precompute(T* Fe,T& Jp,const T lambda0,const T mu0,
     const int plastic,const T hardening,const T cy,const T sy,const T hardening_max,
     T* Re,T& lambda,T& mu,T& Je)
@@ -632,7 +637,7 @@ template<class T,class TS> MPM_HD void precompute(T* Fe,T& Jp,const T lambda0,co
         mat_mul_bt(U32,V32,Re);}
     else if(plastic&&!inside){
         if constexpr(sizeof(T)==8) clamp_fp64<T>(Fe,Jp,V32,plastic,cy,sy,0.,Re,Je);
-        else if(s32[2]>0.25f&&s32[0]<4.f) clamp_refined(Fe,Jp,U32,V32,cy,sy,Re,Je);
+        else if(s32[2]>0.25f&&s32[0]<4.f&&sy-cy>CLAMP_MIN_BAND) clamp_refined(Fe,Jp,U32,V32,cy,sy,Re,Je);
         else{
             ClampArgs a;a.Jp=Jp;a.cy=cy;a.sy=sy;
 #pragma unroll
