@@ -340,10 +340,19 @@ MPM_API mpm_status mpm_autotune(struct mpm_context* ctx, double dt, int substeps
  * caller. Every byte of it is rewritten before it is read, so a call does not depend on
  * what an earlier call left. The first call on a device looks up the area's device address
  * (cudaGetSymbolAddress) with that device current; make that first call before any stream
- * capture. */
+ * capture.
+ * The passes find their offsets by a decoupled look-back with bounded waits. A wait that
+ * gives up (never seen: the CTA waited for is resident) only costs time: the waiting thread
+ * counts the digit in the keys before its tile itself, and the result is the same. */
 #define MPM_NOALLOC_SORT_MAX (1LL<<20)
 MPM_API mpm_status mpm_sort_pairs_noalloc(const uint32_t* keys_in, const int32_t* vals_in, uint32_t* keys_out,
                                           int32_t* vals_out, long long n, int begin_bit, int end_bit, void* stream);
+/* Check of that path: the same sort (arguments, scratch and result as above) in which no tile
+ * publishes its words, so that every wait gives up, after spin_limit polls (1..1000, about
+ * 40 ns each). Some 10 ms at the largest n. */
+MPM_API mpm_status mpm_selftest_sort_wait(const uint32_t* keys_in, const int32_t* vals_in, uint32_t* keys_out,
+                                          int32_t* vals_out, long long n, int begin_bit, int end_bit, int spin_limit,
+                                          void* stream);
 
 #ifdef __cplusplus
 }

@@ -38,7 +38,7 @@ static_assert((NS_SMALL+NS_THREADS*4-1)/(NS_THREADS*4)<=kMaxTiles&&(kMaxPairs+NS
 struct NoallocScratch {
     unsigned keys[kMaxPairs];
     int vals[kMaxPairs];
-    unsigned counter[4],error;
+    unsigned counter[4];
     unsigned hist[4][256];
     unsigned status[4*kMaxTiles*256];
 };
@@ -76,7 +76,7 @@ bool current_context_id(unsigned long long* id)
     return g_ctx_get_id(ctx,id)==CUDA_SUCCESS;
 }
 
-template<int ITEMS> __global__ void k_sort_pass(const unsigned*,const int*,unsigned*,int*,long long,int,const unsigned*,unsigned*,unsigned*,int,unsigned*);
+template<int ITEMS> __global__ void k_sort_pass(const unsigned*,const int*,unsigned*,int*,long long,int,const unsigned*,unsigned*,unsigned*,int,int,bool);
 NoallocScratch* scratch_for(int dev)
 {
     std::lock_guard<std::mutex> lock(g_mutex);
@@ -118,15 +118,18 @@ __global__ void __launch_bounds__(512) k_sort_hist(const unsigned* __restrict__ 
     __syncthreads();
     for(int t=threadIdx.x;t<passes*256;t+=blockDim.x){const unsigned v=(&h[0][0])[t];if(v) atomicAdd(&hist[t],v);}
 }
-// One stable 8-bit pass: the tiles of k_onesweep (ticket order, decoupled look-back with bounded
-// waits) for keys in any order. Peers come from eight ballots instead of match.any, whose cost
+// One stable 8-bit pass: the tiles of k_onesweep (ticket order, decoupled look-back) for keys in
+// any order. A wait for an earlier tile's word gives up after `spin_limit` polls; the thread
+// then counts its digit itself, in the keys of that tile and of all before it, so that the result
+// does not depend on the waits. (`publish` false, for the check of that path: no words are
+// published.) Peers come from eight ballots instead of match.any, whose cost
 // grows with the distinct digits of a warp, and the tile's pairs go through shared memory
 // in digit order, so that each digit's run is stored contiguously. A pass of 10^6 random
 // pairs takes about 17 us, against 44 for five kernels (histogram, three of a scan, scatter).
 // Bound by latency: its 16 MB of traffic take 2.4 us.
 template<int ITEMS> __global__ void __launch_bounds__(NS_THREADS) k_sort_pass(const unsigned* __restrict__ kin,const int* __restrict__ vin,
     unsigned* __restrict__ kout,int* __restrict__ vout,long long n,int shift,const unsigned* __restrict__ hist,unsigned* status,
-    unsigned* tile_counter,int num_tiles,unsigned* error)
+    unsigned* tile_counter,int num_tiles,int spin_limit,bool publish)
 {
     pdl_enter();
     extern __shared__ unsigned smem[];
@@ -174,7 +177,7 @@ template<int ITEMS> __global__ void __launch_bounds__(NS_THREADS) k_sort_pass(co
         if(tid<256){
 #pragma unroll
             for(int q=0;q<NS_WARPS;++q){const unsigned c=wcnt[q][tid];wcnt[q][tid]=count;count+=c;}
-            atomicExch(status+(long long)tile*256+tid,(tile==0?OS_PRE:OS_AGG)|count);}
+            if(publish) atomicExch(status+(long long)tile*256+tid,(tile==0?OS_PRE:OS_AGG)|count);}
         const unsigned f=scan256(count);
         if(tid<256) first[tid]=f;
         __syncthreads();
@@ -188,6 +191,7 @@ template<int ITEMS> __global__ void __launch_bounds__(NS_THREADS) k_sort_pass(co
             unsigned excl=0;
             if(tile>0){
                 bool done=false;
+                long long counted=0;              // keys from the first on that this thread has to count
                 for(int t=tile-1;t>=0&&!done;t-=NS_LOOKBACK){
                     unsigned v[NS_LOOKBACK];
 #pragma unroll
@@ -196,24 +200,24 @@ template<int ITEMS> __global__ void __launch_bounds__(NS_THREADS) k_sort_pass(co
                     for(int u=0;u<NS_LOOKBACK;++u){
                         if(done||t-u<0) continue;
                         unsigned x=v[u];
-                        if((x&~OS_MASK)==0u) x=os_wait(status+(long long)(t-u)*256+tid,error);
+                        for(int spins=0;(x&~OS_MASK)==0u&&spins<spin_limit;++spins){__nanosleep(32);x=os_load(status+(long long)(t-u)*256+tid);}
+                        if((x&~OS_MASK)==0u){counted=(long long)(t-u+1)*NS_THREADS*ITEMS;done=true;break;}
                         excl+=x&OS_MASK;
                         if((x&~OS_MASK)!=OS_AGG) done=true;}}
-                atomicExch(status+(long long)tile*256+tid,OS_PRE|(excl+count));}
+                for(long long i=0;i<counted;++i) excl+=((kin[i]>>shift)&255u)==(unsigned)tid;
+                if(publish) atomicExch(status+(long long)tile*256+tid,OS_PRE|(excl+count));}
             out0[tid]=digit0+excl-f;}
         __syncthreads();
         const int m=(int)(n-t0<NS_THREADS*ITEMS?n-t0:NS_THREADS*ITEMS);
         for(int i=tid;i<m;i+=NS_THREADS){
             const unsigned key=skey[i],pos=out0[(key>>shift)&255u]+i;
-            if(pos<n){kout[pos]=key;vout[pos]=sval[i];}}      // always, unless a wait gave up
+            kout[pos]=key;vout[pos]=sval[i];}
         __syncthreads();
     }
 }
 
-} // namespace
-
-extern "C" mpm_status mpm_sort_pairs_noalloc(const uint32_t* keys_in,const int32_t* vals_in,uint32_t* keys_out,int32_t* vals_out,
-                                             long long n,int begin_bit,int end_bit,void* stream)
+mpm_status sort_pairs(const uint32_t* keys_in,const int32_t* vals_in,uint32_t* keys_out,int32_t* vals_out,
+                      long long n,int begin_bit,int end_bit,void* stream,int spin_limit,bool publish)
 {
     if(n<0||n>kMaxPairs||!keys_out||!vals_out||(n>0&&!keys_in)) return MPM_BAD_ARG;
     if(begin_bit<0||end_bit>32||begin_bit>=end_bit) return MPM_BAD_ARG;
@@ -242,9 +246,27 @@ extern "C" mpm_status mpm_sort_pairs_noalloc(const uint32_t* keys_in,const int32
         unsigned* kout=to_out?keys_out:sc->keys;int* vout=to_out?vals_out:sc->vals;
         const unsigned* h=sc->hist[p];unsigned* status=sc->status+(long long)p*num_tiles*256;
         auto pass=[&](auto kernel){
-            return launch(kernel,g,NS_THREADS,ns_smem(items),st,kin,vin,kout,vout,n,begin_bit+8*p,h,status,sc->counter+p,num_tiles,&sc->error);};
+            return launch(kernel,g,NS_THREADS,ns_smem(items),st,kin,vin,kout,vout,n,begin_bit+8*p,h,status,sc->counter+p,num_tiles,spin_limit,publish);};
         const cudaError_t e=items==4?pass(k_sort_pass<4>):pass(k_sort_pass<8>);
         if(e!=cudaSuccess) return MPM_CUDA_ERROR;
         kin=kout;vin=vout;}
     return MPM_OK;
+}
+
+} // namespace
+
+// Polls of about 40 ns each before a look-back counts for itself: a few milliseconds, against the
+// microseconds in which a resident CTA publishes.
+constexpr int kSortSpinLimit=1<<16;
+
+extern "C" mpm_status mpm_sort_pairs_noalloc(const uint32_t* keys_in,const int32_t* vals_in,uint32_t* keys_out,int32_t* vals_out,
+                                             long long n,int begin_bit,int end_bit,void* stream)
+{
+    return sort_pairs(keys_in,vals_in,keys_out,vals_out,n,begin_bit,end_bit,stream,kSortSpinLimit,true);
+}
+extern "C" mpm_status mpm_selftest_sort_wait(const uint32_t* keys_in,const int32_t* vals_in,uint32_t* keys_out,int32_t* vals_out,
+                                             long long n,int begin_bit,int end_bit,int spin_limit,void* stream)
+{
+    if(spin_limit<1||spin_limit>1000) return MPM_BAD_ARG;
+    return sort_pairs(keys_in,vals_in,keys_out,vals_out,n,begin_bit,end_bit,stream,spin_limit,false);
 }
