@@ -256,6 +256,14 @@ MPM_API mpm_status mpm_get_cg_iterations(struct mpm_context* ctx, int capacity, 
  * flag. Needs mpm_initialize. */
 MPM_API mpm_status mpm_selftest_lookback_wait(struct mpm_context* ctx, int spin_limit);
 
+/* The same for the grid barriers of the one-kernel CG solve: `phases` (1..64) of them by a
+ * cooperative grid of a CTA per SM, counting arrivals from `first` (a 32-bit count that wraps).
+ * With `absent` one CTA never arrives: the others give up after spin_limit polls (1..2^20, up to
+ * 1 us each), and the call reports MPM_CUDA_ERROR ("CG grid barrier wait exceeded its limit"),
+ * as a substep whose wait ran out would. It also reports MPM_CUDA_ERROR if a CTA passes a barrier
+ * before all have arrived. The context stays usable. Needs mpm_initialize. */
+MPM_API mpm_status mpm_selftest_grid_barrier(struct mpm_context* ctx, uint32_t first, int phases, int absent, int spin_limit);
+
 /* Simulation clock: seconds simulated since mpm_initialize (or the last mpm_set_time).
  * Fixed-dt substeps advance it by dt; mpm_advance_to_time by its substeps. */
 MPM_API mpm_status mpm_get_time(struct mpm_context* ctx, double* time);

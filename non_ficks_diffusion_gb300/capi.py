@@ -113,6 +113,7 @@ SIGNATURES = {
     "mpm_preset_particles": (C.c_int, [C.c_int, C.c_int, C.c_ulonglong, C.c_longlong, _dp, _dp, _dp, _dp, _dp]),
     "mpm_get_cg_iterations": (C.c_int, [_vp, C.c_int, _ip, _lp, _ip]),
     "mpm_selftest_lookback_wait": (C.c_int, [_vp, C.c_int]),
+    "mpm_selftest_grid_barrier": (C.c_int, [_vp, C.c_uint32, C.c_int, C.c_int, C.c_int]),
     "mpm_sort_pairs_noalloc": (C.c_int, [_vp, _vp, _vp, _vp, C.c_longlong, C.c_int, C.c_int, _vp]),
     "mpm_selftest_sort_wait": (C.c_int, [_vp, _vp, _vp, _vp, C.c_longlong, C.c_int, C.c_int, C.c_int, _vp]),
 }

@@ -344,6 +344,17 @@ __global__ void __launch_bounds__(32) k_lookback_selftest(unsigned* status,unsig
 {
     chained_prefix(status,1,1u,error,spin_limit);
 }
+// `phases` grid barriers of k_cg_solve by a cooperative grid of which CTA 0 stays away with `absent`.
+// The arrivals start from `first`. Each CTA counts itself in marks[phase] before a barrier and
+// behind it expects all to have; a CTA that a barrier let through early sets marks[phases].
+__global__ void __launch_bounds__(XFER_THREADS) k_barrier_selftest(Counters* ctr,unsigned* marks,unsigned first,int phases,int absent,int spin_limit)
+{
+    if(absent&&blockIdx.x==0) return;
+    for(int p=0;p<phases;++p){
+        if(threadIdx.x==0) atomicAdd(&marks[p],1u);
+        if(!solve_barrier(ctr,first+(unsigned)(p+1)*gridDim.x,[]{},[]{},[&]{
+            if(*(volatile unsigned*)&marks[p]!=gridDim.x-(absent?1u:0u)) atomicOr(&marks[phases],1u);},spin_limit)) return;}
+}
 void set_dt(mpm_context* c,double dt)
 {
     if(dt==c->last_dt) return;
@@ -1425,6 +1436,28 @@ mpm_status mpm_selftest_lookback_wait(mpm_context* c,int spin_limit)
     CUDA_TRY(c,cudaMemsetAsync(&c->ctr->error,0,2*sizeof(unsigned),c->stream));
     k_lookback_selftest<<<1,32,0,c->stream>>>(c->sortws,&c->ctr->error,spin_limit);c->launches++;
     CUDA_TRY(c,cudaGetLastError());
+    return collect_status(c);
+}
+
+mpm_status mpm_selftest_grid_barrier(mpm_context* c,unsigned first,int phases,int absent,int spin_limit)
+{
+    if(!c) return MPM_BAD_ARG;
+    if(phases<1||phases>64||spin_limit<1||spin_limit>SOLVE_SPIN_LIMIT) return fail(c,MPM_BAD_ARG,"phases must be in [1, 64], spin_limit in [1, 2^20]");
+    if(!c->initialized) return fail(c,MPM_NOT_READY,"mpm_initialize has not run");
+    if(!c->coop) return fail(c,MPM_NOT_READY,"no cooperative launches on this device");
+    // marks in the sort scratch, the arrivals in the counters: both rewritten by every substep
+    CUDA_TRY(c,cudaMemsetAsync(c->sortws,0,(size_t)(phases+1)*sizeof(unsigned),c->stream));
+    CUDA_TRY(c,cudaMemcpyAsync(&c->ctr->solve_arrived,&first,sizeof(first),cudaMemcpyHostToDevice,c->stream));
+    CUDA_TRY(c,cudaMemsetAsync(&c->ctr->error,0,2*sizeof(unsigned),c->stream));
+    cudaLaunchAttribute at[1];
+    at[0].id=cudaLaunchAttributeCooperative;at[0].val.cooperative=1;
+    cudaLaunchConfig_t cfg={};
+    cfg.gridDim=dim3((unsigned)c->num_sms);cfg.blockDim=dim3(XFER_THREADS);cfg.stream=c->stream;cfg.attrs=at;cfg.numAttrs=1;
+    CUDA_TRY(c,cudaLaunchKernelEx(&cfg,k_barrier_selftest,c->ctr,c->sortws,first,phases,absent,spin_limit));c->launches++;
+    unsigned early=0;
+    CUDA_TRY(c,cudaMemcpyAsync(&early,c->sortws+phases,sizeof(early),cudaMemcpyDeviceToHost,c->stream));
+    CUDA_TRY(c,cudaStreamSynchronize(c->stream));
+    if(early) return fail(c,MPM_CUDA_ERROR,"a CTA passed the grid barrier before all had arrived");
     return collect_status(c);
 }
 

@@ -1605,9 +1605,11 @@ template<class P> __global__ void __launch_bounds__(NODE_THREADS) k_cg_update(De
 // waits for all (bounded) and runs `post`. False after the limit. A round trip to L2 or a few
 // dependent FP64 operations here are time of every CTA: the poll is the acquire (a fence
 // and a second read after it took 0.7 us), and what the threads do not wait for is in `idle`.
+// The count of arrivals wraps (at 608 CTAs after 3.5 million CG iterations); it is never further than
+// one arrival per CTA from the target, so the sign of their difference decides.
 constexpr int SOLVE_SPIN_LIMIT=1<<20;
 __device__ __forceinline__ unsigned load_acquire(const unsigned* p){unsigned v;asm volatile("ld.acquire.gpu.global.u32 %0,[%1];":"=r"(v):"l"(p):"memory");return v;}
-template<class F0,class F1,class F2> __device__ __forceinline__ bool solve_barrier(Counters* ctr,unsigned target,F0 pre,F1 idle,F2 post)
+template<class F0,class F1,class F2> __device__ __forceinline__ bool solve_barrier(Counters* ctr,unsigned target,F0 pre,F1 idle,F2 post,int spin_limit=SOLVE_SPIN_LIMIT)
 {
     __shared__ bool ok;
     __syncthreads();
@@ -1620,8 +1622,8 @@ template<class F0,class F1,class F2> __device__ __forceinline__ bool solve_barri
             idle();
             int spins=0;
             unsigned seen;
-            while((seen=load_acquire(&ctr->solve_arrived))<target&&++spins<SOLVE_SPIN_LIMIT) if(spins>64) __nanosleep(32);
-            ok=seen>=target;
+            while((int)((seen=load_acquire(&ctr->solve_arrived))-target)<0&&++spins<spin_limit) if(spins>64) __nanosleep(32);
+            ok=(int)(seen-target)>=0;
             if(!ok) atomicOr(&ctr->error,ERR_GRID_WAIT);
             post();}}
     __syncthreads();
@@ -1664,8 +1666,8 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
     PairPass pass;                       // the warp's resident pass, when the CTA has one unit
     int held=-1;                         // unit whose item's record is in rec
     unsigned entry=0;                    // its entry
-    int phase=0;
-    auto arrived=[&]{return (unsigned)(phase+1)*(unsigned)G;};
+    unsigned phase=0;                    // wraps as the count does
+    auto arrived=[&]{return (phase+1u)*(unsigned)G;};
     // K v for v = x, or s = r + beta s_old with s^T K s into part[][0]
     auto product=[&](bool from_x,T beta){
         NodeSum<T> sks;
@@ -1732,7 +1734,7 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
         product(false,be);
         if(!solve_barrier(ctr,arrived(),[&]{contribute(1,false);},[&]{
             clear_ahead();
-            if(phase>2) msq=rho+beta*(2.*rs_sum+beta*ss_sum);},[&]{
+            if(iters>0) msq=rho+beta*(2.*rs_sum+beta*ss_sum);},[&]{
             double s[3],mx;read_slot(s,mx);
             const double sq=(double)ps.sks*s[0]+msq;
             sh_alpha=(T)(sq!=0.?rho/sq:(double)FLT_MAX);})) return;
