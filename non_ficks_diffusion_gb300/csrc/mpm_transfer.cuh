@@ -1722,7 +1722,7 @@ template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_cg_solve(D
     int iters=0,converged=0;
     const double tol=S.cg[0].tol,tol2=tol*tol;
     // sqrt(mx) <= tol; the root (on the barriers' critical path) only where rounding could decide
-    auto small=[&](double mx){return mx<tol2*(1.-1e-14)?true:mx>tol2*(1.+1e-14)?false:sqrt(mx)<=tol;};
+    auto small=[&](double mx){return tol<0.?false:mx<tol2*(1.-1e-14)?true:mx>tol2*(1.+1e-14)?false:sqrt(mx)<=tol;};
     if(!solve_barrier(ctr,arrived(),[&]{contribute(1,true);},clear_ahead,[&]{
         double s[3],mx;read_slot(s,mx);
         rmax=mx;rho=msq=s[0];
