@@ -6,6 +6,7 @@
 #include "mpm_transfer.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -266,7 +267,8 @@ template<class P> void enqueue_binning(mpm_context* c,cudaStream_t st,const DevS
         launch_dep(c,k_items<TT<P>>,grid_for(c,16),XFER_THREADS,order?order_bytes(c->cfg.chunk):0,st,S,order?1:0,order&&solve_units<P>(c)?1:0);counted(c,PH_BIN);}
 }
 
-int max_cg_iters(mpm_context* c){int m=0;for(auto& s:c->scenes) m=std::max(m,s.desc.cg_max_iters);return m;}
+// Bound on the CG loop's trips over all scenes: one above the largest cg_max_iters, in an int.
+int max_cg_trips(mpm_context* c){int m=0;for(auto& s:c->scenes) m=std::max(m,s.desc.cg_max_iters);return m<INT_MAX?m+1:m;}
 
 // One Hessian product in the context's form: work items per CTA, per warp, or chosen per launch.
 template<class P,bool FROM_X> void launch_hessian(mpm_context* c,cudaStream_t st,const DevState<TT<P>>& S2)
@@ -282,7 +284,7 @@ template<class P> void enqueue_cg_body(mpm_context* c,cudaStream_t st,const DevS
     {PhaseScope ps(c,PH_HESS,st);
         launch_hessian<P,false>(c,st,S2);counted(c,PH_HESS);}
     {PhaseScope ps(c,PH_CGNODE,st);
-        launch_dep(c,k_cg_update<P>,grid_for(c,c->node_grid),NODE_THREADS,0,st,S2,cond,use_cond,max_cg_iters(c)+1);counted(c,PH_CGNODE);}
+        launch_dep(c,k_cg_update<P>,grid_for(c,c->node_grid),NODE_THREADS,0,st,S2,cond,use_cond,max_cg_trips(c));counted(c,PH_CGNODE);}
 }
 
 // CTAs of k_cg_solve: at most those that fit the GPU at once (the launch is cooperative); fewer
@@ -300,7 +302,7 @@ template<class P> cudaError_t launch_solve(mpm_context* c,cudaStream_t st,const 
         cudaLaunchConfig_t cfg={};
         cfg.gridDim=dim3((unsigned)std::min<long long>((long long)c->num_sms*std::max(per_sm,1),std::max<long long>(c->num_sms,c->n_total/(solve_units<P>(c)?64:128))));
         cfg.blockDim=dim3(XFER_THREADS);cfg.dynamicSmemBytes=smem;cfg.stream=st;cfg.attrs=at;cfg.numAttrs=1;
-        return cudaLaunchKernelEx(&cfg,k_cg_solve<P>,S2,max_cg_iters(c)+1);}
+        return cudaLaunchKernelEx(&cfg,k_cg_solve<P>,S2,max_cg_trips(c));}
     else return cudaErrorNotSupported;
 }
 
@@ -370,7 +372,7 @@ template<class P> mpm_status substep_eager(mpm_context* c,double dt,int stop_aft
     if(!dt_on_device) set_dt(c,dt);
     DevState<TT<P>> S2=enqueue_pre<P>(c,st,c->cur,dt,0,0,stop_after);
     if(stop_after==1||stop_after==2){return MPM_OK;}
-    const int cap=max_cg_iters(c)+1;
+    const int cap=max_cg_trips(c);
     for(int it=0;it<cap;++it){
         CUDA_TRY(c,cudaMemcpyAsync(&c->h_ctr->any_active,&c->ctr->any_active,sizeof(int),cudaMemcpyDeviceToHost,st));
         CUDA_TRY(c,cudaStreamSynchronize(st));
