@@ -296,7 +296,9 @@ typedef struct mpm_launch_config {
                                scene or batch), else a CTA per item (small scenes, and the last
                                trips when few scenes still iterate). With 2, the graphs of a
                                single FP32 or mixed scene of at most 2^20 particles run the
-                               whole CG as one cooperative kernel.
+                               whole CG as one cooperative kernel (where the device refuses
+                               that launch, or with MPM_COOP=0 in the environment, the loop
+                               of kernels).
                                Default 2 */
     int incremental_sort; /* binning of a substep: 0 a full stable radix sort of the cell keys;
                              1 the same order obtained by sorting only the particles whose

@@ -90,7 +90,8 @@ struct mpm_context {
     int xfer_grid=12;                        // transfer-kernel CTAs per SM (grid-stride over work items)
     int node_grid=4;                         // node-kernel (grid update, CG vectors) CTAs per SM
     int hess_warp=HESS_AUTO;                 // Hessian work items per CTA (0), per warp (1), or chosen per launch (2)
-    bool coop=false;                          // the device takes cooperative launches
+    bool coop=false;                          // the device takes cooperative launches (until one is refused, see build_graphs)
+    bool coop_refuse=false;                   // stand-in for a refusal (MPM_COOP=refuse)
     bool use_pdl=true;                       // substep kernels as programmatic dependents
     // timing
     bool timing=false;
@@ -297,10 +298,11 @@ template<class P> cudaError_t launch_solve(mpm_context* c,cudaStream_t st,const 
         int per_sm=0;
         cudaError_t e=cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,k_cg_solve<P>,XFER_THREADS,smem);
         if(e!=cudaSuccess) return e;
+        if(per_sm<1||c->coop_refuse) return cudaErrorCooperativeLaunchTooLarge;
         cudaLaunchAttribute at[1];
         at[0].id=cudaLaunchAttributeCooperative;at[0].val.cooperative=1;
         cudaLaunchConfig_t cfg={};
-        cfg.gridDim=dim3((unsigned)std::min<long long>((long long)c->num_sms*std::max(per_sm,1),std::max<long long>(c->num_sms,c->n_total/(solve_units<P>(c)?64:128))));
+        cfg.gridDim=dim3((unsigned)std::min<long long>((long long)c->num_sms*per_sm,std::max<long long>(c->num_sms,c->n_total/(solve_units<P>(c)?64:128))));
         cfg.blockDim=dim3(XFER_THREADS);cfg.dynamicSmemBytes=smem;cfg.stream=st;cfg.attrs=at;cfg.numAttrs=1;
         return cudaLaunchKernelEx(&cfg,k_cg_solve<P>,S2,max_cg_trips(c));}
     else return cudaErrorNotSupported;
@@ -441,7 +443,7 @@ template<class P> mpm_status capture_substep(mpm_context* c,cudaStream_t st,cuda
     return s;
 }
 
-template<class P> mpm_status build_graphs(mpm_context* c,double dt)
+template<class P> mpm_status build_substep_graphs(mpm_context* c,double dt)
 {
     for(int parity=0;parity<2;++parity){
         if(c->gexec[parity]){cudaGraphExecDestroy(c->gexec[parity]);c->gexec[parity]=nullptr;}
@@ -465,7 +467,7 @@ template<class P> mpm_status build_graphs(mpm_context* c,double dt)
 // two substeps (parities p and p^1, so the buffers alternate), each preceded by k_cfl; the
 // second one sits in an IF node that k_cfl of the first opens only when the advance goes
 // on, and k_frame_cond closes the loop once a substep has ended the advance.
-template<class P> mpm_status build_frame_graphs(mpm_context* c)
+template<class P> mpm_status build_advance_graphs(mpm_context* c)
 {
     if(!c->stream3&&cudaStreamCreateWithFlags(&c->stream3,cudaStreamNonBlocking)!=cudaSuccess) return fail(c,MPM_CUDA_ERROR,"stream");
     if(!c->stream4&&cudaStreamCreateWithFlags(&c->stream4,cudaStreamNonBlocking)!=cudaSuccess) return fail(c,MPM_CUDA_ERROR,"stream");
@@ -510,6 +512,21 @@ template<class P> mpm_status build_frame_graphs(mpm_context* c)
     c->frame_graph_valid=true;c->graph_ntotal=c->n_total;
     return MPM_OK;
 }
+
+// Runs `build`. Where the solve's cooperative launch is refused (at capture, or when the graph is
+// instantiated: CUDA takes none in a conditional body under MPS), the context goes over to the
+// loop of kernels and builds once more.
+template<class P,class F> mpm_status build_or_loop(mpm_context* c,F build)
+{
+    mpm_status s=build();
+    if(s!=MPM_OK&&solve_in_one<P>(c)){
+        cudaGetLastError();
+        c->coop=false;
+        s=build();}
+    return s;
+}
+template<class P> mpm_status build_graphs(mpm_context* c,double dt){return build_or_loop<P>(c,[&]{return build_substep_graphs<P>(c,dt);});}
+template<class P> mpm_status build_frame_graphs(mpm_context* c){return build_or_loop<P>(c,[&]{return build_advance_graphs<P>(c);});}
 
 template<class P> mpm_status substep_graph(mpm_context* c,double dt)
 {
@@ -899,6 +916,9 @@ mpm_status mpm_create(const mpm_config* cfg,mpm_context** out)
     {int v=0;if(cudaDeviceGetAttribute(&v,cudaDevAttrCooperativeLaunch,c0.device)==cudaSuccess) c->coop=v!=0;}
     {int v=0;if(cudaDeviceGetAttribute(&v,cudaDevAttrPageableMemoryAccess,c0.device)==cudaSuccess) c->pageable_access=v!=0;}
     if(const char* v=std::getenv("MPM_HOST_DIRECT")) c->host_direct=std::strcmp(v,"0")!=0;   // "0": always stage host arrays
+    if(const char* v=std::getenv("MPM_COOP")){                                               // "0": the CG always as a loop of kernels
+        if(!std::strcmp(v,"0")) c->coop=false;
+        c->coop_refuse=!std::strcmp(v,"refuse");}                                            // "refuse": its cooperative launch is refused (for tests)
     if(const char* v=std::getenv("MPM_PDL")) c->use_pdl=std::strcmp(v,"0")!=0;               // "0": plain stream order
     if(const char* v=std::getenv("MPM_HESSIAN_WARP")) c->hess_warp=std::min(2,std::max(0,std::atoi(v)));  // form of the Hessian product
     if(c0.precision==MPM_PRECISION_FP64){c->minb_hess=c->minb_p2g=c->minb_g2p=3;}
