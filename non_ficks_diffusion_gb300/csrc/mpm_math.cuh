@@ -12,13 +12,9 @@ namespace mpm {
 
 // T: particle/grid storage and transfer arithmetic. TS: SVD/polar arithmetic. (CG dot products
 // and norms are formed per node in T and added up to FP64 or twice FP32 precision.)
-// xfer_blocks: resident CTAs per SM the transfer kernels are compiled for (register cap).
-struct PrecFP32  { using T=float;  using TS=float;  static constexpr int id=0; static constexpr int xfer_blocks=4; };
-struct PrecMixed { using T=float;  using TS=double; static constexpr int id=1; static constexpr int xfer_blocks=4; };
-struct PrecFP64  { using T=double; using TS=double; static constexpr int id=2; static constexpr int xfer_blocks=2; };
-
-template<class T> struct Vec4 { T x,y,z,w; };
-template<> struct Vec4<float> { float x,y,z,w; };
+struct PrecFP32  { using T=float;  using TS=float;  static constexpr int id=0; };
+struct PrecMixed { using T=float;  using TS=double; static constexpr int id=1; };
+struct PrecFP64  { using T=double; using TS=double; static constexpr int id=2; };
 
 template<class T> MPM_HD T mpm_sqrt(T x);
 template<> MPM_HD float mpm_sqrt<float>(float x){return sqrtf(x);}
@@ -208,8 +204,6 @@ template<class T,int max_sweeps=6> MPM_HD void svd3(const T* F,T* U,T* s,T* V,co
 }
 
 // ---- constitutive model (reference MPM_Constitutive_Model.cpp:32-76) ----
-struct Plasticity { int plastic; double hardening,compression_yield,stretching_yield,hardening_max; };
-
 // 1/sqrt(x) for x within 1e-4 of 1: 1 - e/2 + 3e^2/8 - 5e^3/16 with e = x - 1 (next term
 // 35e^4/128, below 3e-17); otherwise the root and the division.
 template<class T> MPM_HD T rsqrt_near1(T x)
@@ -667,6 +661,8 @@ template<class T,class TS> MPM_HD void precompute(T* Fe,T& Jp,const T lambda0,co
     harden(Jp,lambda0,mu0,plastic,hardening,hardening_max,lambda,mu);
 }
 
+// The stress and its differential as the reference writes them: for the host checks, which hold
+// them to the oracle; the kernels use the form of HessianData below.
 // First Piola-Kirchhoff stress P = 2 mu (Fe - Re) + lambda (Je-1) cof(Fe), reference :63-67.
 template<class T> MPM_HD void stress_P(const T* Fe,const T* Re,const T lambda,const T mu,const T Je,T* P)
 {
