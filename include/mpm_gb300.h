@@ -45,7 +45,8 @@ typedef enum mpm_status {
 
 typedef enum mpm_precision {
     MPM_PRECISION_FP32 = 0,  /* everything FP32 (the reference's shipped T=float) */
-    MPM_PRECISION_MIXED = 1, /* FP32 state, transfers and CG vectors; SVD/polar to FP64-class accuracy, FP64 CG norms */
+    MPM_PRECISION_MIXED = 1, /* FP32 state, transfers and CG vectors; SVD/polar to FP64-class accuracy,
+                                  CG sums to 48 bits (FP32 pairs) inside a warp and FP64 across warps */
     MPM_PRECISION_FP64 = 2   /* everything FP64 (the reference built with T=double) */
 } mpm_precision;
 
@@ -229,7 +230,8 @@ MPM_API mpm_status mpm_synchronize(struct mpm_context* ctx);
 MPM_API void* mpm_stream(struct mpm_context* ctx);
 
 /* Per-phase device timing (CUDA events on the context stream). While enabled, substeps
- * run eagerly with events around each phase. */
+ * run eagerly with events around each phase: as a loop of kernels, also where the graphs
+ * of a small scene run the CG as one kernel. */
 MPM_API mpm_status mpm_set_timing(struct mpm_context* ctx, int enabled);
 /* Phase names and accumulated milliseconds and launch counts since timing was enabled;
  * returns the number of phases. */
@@ -325,7 +327,9 @@ MPM_API mpm_status mpm_set_launch_config(struct mpm_context* ctx, const mpm_laun
  * (256..2048 particles), the occupancy variant of each transfer kernel, the transfer grid
  * size, the node-kernel grid size and the binning (full or incremental sort), one
  * coordinate at a time, in two sweeps (the second from the first one's best, timing only
- * configurations not yet timed). Each trial starts
+ * configurations not yet timed). Where the graphs run the CG as one kernel (see
+ * hessian_warp_items) ctas_hessian does nothing and node_grid_per_sm sizes the grid update
+ * alone, so that what is chosen there is noise. Each trial starts
  * from the same saved particle state, runs one untimed substep of size dt (graph build)
  * and then `substeps` timed substeps; the median per-substep time ranks the candidates.
  * The particle state, the buffer parity and the substep counters are restored afterwards,

@@ -126,6 +126,8 @@ template<class T> __global__ void __launch_bounds__(256) k_keys(DevState<T> S,un
 }
 
 // ---- one-sweep radix pass (decoupled look-back) ----
+// After Adinets & Merrill, "Onesweep: A Faster Least Significant Digit Radix Sort for GPUs" (2022),
+// and Merrill & Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back" (2016).
 // One kernel per 8-bit pass. Tiles are taken in the order of an atomic counter, so every
 // tile before the one a CTA holds is held by a CTA that has already started. A tile ranks
 // its keys stably (peers with the same digit by lane order, on top of the warp's running

@@ -380,7 +380,7 @@ MPM_HD F2x ff_prod(F2x a,F2x b){const float p=ff_mul(a.h,b.h);return ff_norm(F2x
 // The clamped plasticity update of the mixed variant from the FP32 SVD F ~ U diag(s) V^T
 // (s2 well above 0), to FP32 rounding of the exact result, without FP64 operations: the FP64
 // pipe runs at 1/64 of the FP32 rate, and the FP64 Jacobi this replaces took four fifths
-// of P2G once most particles yield (1.94M particles, nearly all clamped: P2G 1.79 -> 0.65 ms).
+// of P2G once most particles yield (1.94M particles, 81 % clamped: P2G 1.79 -> 0.65 ms).
 // One step of first-order correction, its inputs evaluated to twice FP32 precision:
 //   dU = U^T U - I, dV = V^T V - I   (the orthonormal factors are U (I - dU/2), V (I - dV/2)),
 //   M = U^T F V - (dU D + D dV)/2 = D + E with D diagonal and E ~ 1e-7.

@@ -716,7 +716,7 @@ template<int MINB> __global__ void __launch_bounds__(XFER_THREADS,MINB) k_p2g(De
 // over all SMs and keeps the plasticity's code out of the scatter's loop, where the two
 // together overran the instruction cache (38 % of the stall cycles on yielding particles).
 // Ordering, particles and scatter against the one kernel before: 0.71 -> 0.50 ms (1.94M particles,
-// nearly all yielding), 2.15 -> 1.75 ms (64-scene batch), 82 -> 62 us (60K), 2.78 -> 2.74 ms
+// 81 % yielding), 2.15 -> 1.75 ms (64-scene batch), 82 -> 62 us (60K), 2.78 -> 2.74 ms
 // (21.5M unstrained particles). Bound by instruction issue where particles yield, else by HBM.
 template<class P> __global__ void __launch_bounds__(XFER_THREADS,4) k_particles(DevState<typename P::T> S)
 {
