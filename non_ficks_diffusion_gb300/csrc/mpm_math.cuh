@@ -609,7 +609,8 @@ template<class T,class TS> MPM_HD void precompute(T* Fe,T& Jp,const T lambda0,co
     if constexpr(sizeof(T)==4){
         // no clamp for certain, all singular values inside the yield band: only the rotation is
         // needed (unstrained and lightly strained bodies; the SVD below took half of P2G there)
-        const float lim=plastic?fminf(fminf((sy-margin)*(sy-margin)-1.f,1.f-(cy+margin)*(cy+margin)),POLAR_SERIES_MAX):POLAR_SERIES_MAX;
+        const float top=fmaxf(sy-margin,0.f);       // a limit below -1 has a square above 1, too
+        const float lim=plastic?fminf(fminf(top*top-1.f,1.f-(cy+margin)*(cy+margin)),POLAR_SERIES_MAX):POLAR_SERIES_MAX;
         if(lim>0.f&&polar_near(F32,lim*lim,Re)){
             Je=det3_dot2(F32);
             harden(Jp,lambda0,mu0,plastic,hardening,hardening_max,lambda,mu);
