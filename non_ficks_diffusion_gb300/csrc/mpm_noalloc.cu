@@ -211,7 +211,8 @@ template<int ITEMS> __global__ void __launch_bounds__(NS_THREADS) k_sort_pass(co
         const int m=(int)(n-t0<NS_THREADS*ITEMS?n-t0:NS_THREADS*ITEMS);
         for(int i=tid;i<m;i+=NS_THREADS){
             const unsigned key=skey[i],pos=out0[(key>>shift)&255u]+i;
-            kout[pos]=key;vout[pos]=sval[i];}
+            // always, unless calls overlap and mix their counts: that spoils their results, not other memory
+            if(pos<n){kout[pos]=key;vout[pos]=sval[i];}}
         __syncthreads();
     }
 }
